@@ -734,7 +734,7 @@ class Engine : public EngineBase {
     const int nb = (int)jobs.size();
     std::vector<RkLeafDesc> desc(nb);
     long long ws = 0, fl = 0;
-    int max_m = 1, max_n = 1, max_cap = 1;
+    int max_cap = 1;
     for (int b = 0; b < nb; ++b) {
       const LeafInfo& l = L[jobs[b].leaf];
       RkLeafDesc& d = desc[b];
@@ -748,8 +748,6 @@ class Engine : public EngineBase {
       d.pad = 0;
       ws += pad32(rk_slot_elems(l.m, l.n, d.kcap));
       fl += l.m + l.n;
-      max_m = std::max(max_m, l.m);
-      max_n = std::max(max_n, l.n);
       max_cap = std::max(max_cap, d.kcap);
     }
     // ACA shape of each leaf: the autotuner's choice for its size bucket; capacity retries run
@@ -974,8 +972,13 @@ class Engine : public EngineBase {
     times_ms[1] += ms;
     if (stratum >= 0) join_stratum(stratum, jobs, desc, d_desc, d_ws, d_ranks, h_status, h_ranks, src);
 
+    // ---- the dense-SVD jobs: SVD of the dense blocks at the compression epsilon (a stratum's
+    // dense sum: at the low-rank epsilon, truncatedSvd in formattedAddParts); the regular
+    // truncation below then takes them like every other leaf, at the ranks they come back with ----
+    compress_dense(jobs, desc, h_status, h_ranks, add_stratum ? eps_trunc : eps_aca, d_desc.p, d_ws.p, d_ranks.p,
+                   d_status.p, d_counter.p);
+
     std::vector<int> good;
-    int max_k = 1;
     for (int b = 0; b < nb; ++b) {
       if (h_status[b] == kLeafAcaCapacity) {
         const LeafInfo& l = L[jobs[b].leaf];
@@ -989,18 +992,14 @@ class Engine : public EngineBase {
       if (h_status[b] != kLeafOk)
         throw Error("device compression failed on a leaf (status " + std::to_string(h_status[b]) + ")");
       if (h_ranks[b] > 0 && !jobs[b].pass) good.push_back(b);
-      max_k = std::max(max_k, h_ranks[b]);
     }
     auto tcost = [&](int b) { return (double)(desc[b].m + desc[b].n) * h_ranks[b] * h_ranks[b]; };
     std::stable_sort(good.begin(), good.end(), [&](int x, int y) { return tcost(x) > tcost(y); });
 
     typedef typename Traits<T>::wide W;
-    DevArray<W> d_scratch, d_tri, d_maps;
-    DevArray<int> d_good, d_svd_good;
+    DevArray<W> d_tri, d_maps;
     DevArray<TsItem> d_ts_seg[4], d_ts_stack[4];
     DevArray<TsCore> d_ts_core[4];
-    long long slab = 0, grid = 0;
-    std::vector<int> svd_good, large;
     std::vector<TsItem> ts_seg[4], ts_stack[4];
     std::vector<TsCore> ts_core[4];
     bool any_ts = false;
@@ -1015,20 +1014,11 @@ class Engine : public EngineBase {
     if (!good.empty()) {
       // Leaves up to rank ts_kmax go to the tall-skinny phases (row segments of A and B
       // reduced to triangles, stacks of triangles reduced again, core, apply), higher ranks
-      // to the same phases with a CTA per item; the dense-SVD jobs, whose rank is only known
-      // on the device, to the CTA-per-leaf kernel.
-      int big_m = 1, big_n = 1, big_k = 1;
+      // to the same phases with a CTA per item.
       long long tri_n = 0, map_n = 0, tb_tri = 0, tb_map = 0;
       int tb_rows = 1, tb_k = 1;
       const int kmax = ts_kmax<T>();
       for (int b : good) {
-        if (jobs[b].svd) {
-          large.push_back(b);
-          big_m = std::max(big_m, desc[b].m);
-          big_n = std::max(big_n, desc[b].n);
-          big_k = std::max(big_k, h_ranks[b]);
-          continue;
-        }
         const int K = ts_bucket(h_ranks[b], kmax);
         if (!K) {
           // segments of at least k rows (the last one takes the remainder)
@@ -1130,24 +1120,6 @@ class Engine : public EngineBase {
         ts_core[q].push_back(c);
         any_ts = true;
       }
-      for (int b : good)
-        if (jobs[b].svd) svd_good.push_back(b);
-      if (!svd_good.empty()) {
-        big_m = max_m;
-        big_n = max_n;
-        big_k = max_k;
-      }
-      if (!large.empty() || !svd_good.empty()) {
-        slab = truncate_slab_elems<T>(big_m, big_n, big_k);
-        // the slabs are sized for the largest leaf: let them use a third of the free memory
-        // when that is more than the ACA budget, so long high-rank leaves still fill the grid
-        size_t budget = workspace_budget();
-        size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) budget = std::max(budget, free_b / 3);
-        grid = std::min<long long>((long long)std::max(large.size(), svd_good.size()), persistent_grid(2));
-        grid = std::max(1LL, std::min<long long>(grid, (long long)(budget / (slab * sizeof(W)))));
-        d_scratch.alloc((size_t)(grid * slab));
-      }
       if (any_ts) {
         d_tri.alloc((size_t)tri_n);
         d_maps.alloc((size_t)map_n);
@@ -1181,23 +1153,12 @@ class Engine : public EngineBase {
         d_tb_stack.upload(tb_stack, stream_);
         d_tb_core.upload(tb_core, stream_);
       }
-      d_svd_good.upload(svd_good, stream_);
-      d_good.upload(large, stream_);
       HB_CUDA(cudaStreamSynchronize(stream_));
     }
     HB_CUDA(cudaEventRecord(ev_[4], stream_));
     if (!good.empty()) {
-      if (!svd_good.empty()) {
-        // SVD of the dense blocks at the compression epsilon (a stratum's dense sum: at the
-        // low-rank epsilon, truncatedSvd in formattedAddParts), then the regular truncation
-        HB_CUDA(cudaMemsetAsync(d_counter.p, 0, sizeof(int), stream_));
-        launch_truncate<T>(d_desc.p, d_svd_good.p, (int)svd_good.size(), add_stratum ? eps_trunc : eps_aca, d_ws.p,
-                           d_ranks.p, d_status.p,
-                           d_counter.p, d_scratch.p, slab, (int)grid, stream_);
-        HB_CUDA(cudaGetLastError());
-      }
-      // the tall-skinny phases hold leaves disjoint from the CTA kernel's: they run on a
-      // second stream beside it
+      // the warp-level phases hold leaves disjoint from the CTA-per-item ones: they run on a
+      // second stream beside them
       if (any_ts) {
         HB_CUDA(cudaEventRecord(fork_[0], stream_));
         HB_CUDA(cudaStreamWaitEvent(stream2_, fork_[0], 0));
@@ -1211,12 +1172,6 @@ class Engine : public EngineBase {
           HB_CUDA(cudaGetLastError());
         }
         HB_CUDA(cudaEventRecord(fork_[1], stream2_));
-      }
-      if (!large.empty()) {
-        HB_CUDA(cudaMemsetAsync(d_counter.p, 0, sizeof(int), stream_));
-        launch_truncate<T>(d_desc.p, d_good.p, (int)large.size(), eps_trunc, d_ws.p, d_ranks.p, d_status.p,
-                           d_counter.p, d_scratch.p, slab, (int)grid, stream_);
-        HB_CUDA(cudaGetLastError());
       }
       if (!tb_core.empty()) {
         launch_tsqr_cta<T>(d_tb_seg.p, (int)tb_seg.size(), d_ws.p, d_tb_tri.p, false, d_tb_scratch.p, tb_slab,
@@ -1290,6 +1245,69 @@ class Engine : public EngineBase {
       piece_loff_[leaf] = loff[b];
     }
     pieces_.push_back(std::move(piece));
+  }
+
+  // The first truncation of the dense-SVD jobs of a batch (rank min(m, n) on entry): h_ranks and
+  // the device's ranks become those of their SVDs at `eps`.  A block whose wide copy fits shared
+  // memory goes to the shared-memory kernel, a larger one to the CTA-per-leaf kernel on slabs.
+  void compress_dense(const std::vector<RkJob>& jobs, const std::vector<RkLeafDesc>& desc,
+                      const std::vector<int>& h_status, std::vector<int>& h_ranks, double eps,
+                      const RkLeafDesc* d_desc, T* d_ws, int* d_ranks, int* d_status, int* d_counter) {
+    typedef typename Traits<T>::wide W;
+    std::vector<int> small, large;
+    int sm = 1, sn = 1, lm = 1, ln = 1, lk = 1;
+    for (int b = 0; b < (int)jobs.size(); ++b) {
+      if (!jobs[b].svd || jobs[b].pass || h_status[b] != kLeafOk || h_ranks[b] <= 0) continue;
+      const int m = desc[b].m, n = desc[b].n;
+      if (dense_svd_fits<T>(m, n)) {
+        small.push_back(b);
+        sm = std::max(sm, std::min(m, n));
+        sn = std::max(sn, std::max(m, n));
+      } else {
+        large.push_back(b);
+        lm = std::max(lm, m);
+        ln = std::max(ln, n);
+        lk = std::max(lk, h_ranks[b]);
+      }
+    }
+    if (small.empty() && large.empty()) return;
+    auto cost = [&](int b) { return (double)(desc[b].m + desc[b].n) * h_ranks[b] * h_ranks[b]; };
+    auto by_cost = [&](int x, int y) { return cost(x) > cost(y); };
+    std::stable_sort(small.begin(), small.end(), by_cost);
+    std::stable_sort(large.begin(), large.end(), by_cost);
+    DevArray<int> d_small, d_large;
+    DevArray<W> d_scratch;
+    d_small.upload(small, stream_);
+    d_large.upload(large, stream_);
+    long long slab = 0, grid = 0;
+    if (!large.empty()) {
+      slab = truncate_slab_elems<T>(lm, ln, lk);
+      // the slabs are sized for the largest leaf: let them use a third of the free memory
+      // when that is more than the ACA budget, so long leaves still fill the grid
+      size_t budget = workspace_budget();
+      size_t free_b = 0, total_b = 0;
+      if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) budget = std::max(budget, free_b / 3);
+      grid = std::min<long long>((long long)large.size(), persistent_grid(2));
+      grid = std::max(1LL, std::min<long long>(grid, (long long)(budget / (slab * sizeof(W)))));
+      d_scratch.alloc((size_t)(grid * slab));
+    }
+    HB_CUDA(cudaStreamSynchronize(stream_));
+    HB_CUDA(cudaEventRecord(ev_[4], stream_));
+    if (!small.empty())
+      HB_CUDA(launch_dense_svd<T>(d_desc, d_small.p, (int)small.size(), sm, sn, eps, d_ws, d_ranks, d_status, d_counter,
+                                  stream_));
+    if (!large.empty()) {
+      HB_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(int), stream_));
+      launch_truncate<T>(d_desc, d_large.p, (int)large.size(), eps, d_ws, d_ranks, d_status, d_counter, d_scratch.p,
+                         slab, (int)grid, stream_);
+      HB_CUDA(cudaGetLastError());
+    }
+    HB_CUDA(cudaEventRecord(ev_[5], stream_));
+    HB_CUDA(cudaMemcpyAsync(h_ranks.data(), d_ranks, h_ranks.size() * sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    HB_CUDA(cudaStreamSynchronize(stream_));
+    float ms = 0;
+    HB_CUDA(cudaEventElapsedTime(&ms, ev_[4], ev_[5]));
+    times_ms[2] += ms;
   }
 
   void assemble_rk(int method, double eps_aca, double eps_trunc, int svd_below, int stratum) {

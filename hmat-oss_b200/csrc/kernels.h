@@ -117,6 +117,15 @@ void launch_truncate(const RkLeafDesc* d_leaves, const int* d_order, int nleaves
 template <typename T>
 long long truncate_slab_elems(int max_m, int max_n, int max_k);
 
+// SVD compression at `epsilon` of dense blocks held as an exact factorisation with an identity
+// factor (dense_to_rk, exact_factors), a CTA per leaf with the block in shared memory; the leaves
+// must fit (dense_svd_fits), max_m x max_n bound them.  Resets `counter`.
+template <typename T>
+bool dense_svd_fits(int m, int n);
+template <typename T>
+cudaError_t launch_dense_svd(const RkLeafDesc* d_leaves, const int* d_order, int nleaves, int max_m, int max_n,
+                             double epsilon, T* ws, int* ranks, int* status, int* counter, cudaStream_t s);
+
 // Arena panels of assembled Rk leaves back into workspace slots (inverse of launch_compact).
 template <typename T>
 void launch_unpack(const RkLeafDesc* d_leaves, int nleaves, const int* ranks, const RkStoreDesc* store,

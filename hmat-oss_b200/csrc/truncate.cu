@@ -724,6 +724,291 @@ __global__ void __launch_bounds__(kTsWarps * 32) tsapply_kernel(const TsItem* __
 }
 
 // ---------------------------------------------------------------------------------
+// SVD compression of a dense block that is held as an exact factorisation with an identity
+// factor (A = M, B = I for m >= n, A = I, B = M^T otherwise): the tall factor X (len x k,
+// k = min(m, n)) is X = U S V^H, and M's truncated factors are U S^1/2 on X's side and
+// conj(V) S^1/2 on the identity's.
+//
+// A CTA per leaf, X widened into shared memory (leading dimension odd: no bank conflicts along
+// rows).  A column-pivoted Householder QR X P = Q R stops once the columns left hold at most
+// 8 u (or eps / 64) of the block's Frobenius norm, the rounding level of the SVD itself: blocks
+// of smooth kernels reach it at 20 to 30 columns out of 64.  One-sided Jacobi then runs on the
+// r rows of R in place, Y = R^H, Y J = V' S with V = P V' (the rows of a pivoted R are graded,
+// which Jacobi converges on in a few sweeps), so neither Q nor J is formed: U S^1/2 =
+// X V S^-1/2, read from the block that still stands in the slot.
+//
+// Bound by the latency of the Jacobi rounds.  The slab kernel above, which these blocks took
+// before, rotates all k columns in global memory, the noise columns (norms near u sigma_0) in
+// every sweep: with the default compressionMinLeafSize the truncation of the 8,000-point
+// cylinder (leaf 64, epsilon 1e-4, FP64; 1,716 blocks of up to 63 x 63) took 37.8 ms, and 3.9 ms
+// with this kernel followed by the tall-skinny phases.
+constexpr int kDenseSvdThreads = 256;
+constexpr int kDenseSvdCols = 128;  // columns of X at most: four per lane of a Jacobi row
+// Columns a warp updates together in a QR step (their shuffle sums overlap).
+constexpr int kDenseSvdBatch = 4;
+constexpr size_t kDenseSvdSmem = 200 * 1024;  // bytes of X at most
+
+__host__ __device__ constexpr int dense_svd_ld(int len) { return len | 1; }
+
+template <typename T>
+__global__ void __launch_bounds__(kDenseSvdThreads) dense_svd_kernel(const RkLeafDesc* __restrict__ leaves,
+                                                                     const int* __restrict__ order, int nleaves,
+                                                                     double eps, T* ws, int* ranks, int* status,
+                                                                     int* counter) {
+  typedef typename Traits<T>::wide W;
+  extern __shared__ __align__(16) unsigned char dsvd_smem[];
+  __shared__ double s_nrm[kDenseSvdCols];  // squared norms of the columns left, then sigma
+  __shared__ int s_perm[kDenseSvdCols];
+  __shared__ int s_ord[kDenseSvdCols];
+  __shared__ double s_total;
+  __shared__ int s_item, s_piv, s_rot, s_newk;
+  W* X = reinterpret_cast<W*>(dsvd_smem);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const double u = 1.1102230246251565e-16;
+  const double tol = fmin(8.0 * u, eps / 64.0);
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) s_item = atomicAdd(counter, 1);
+    __syncthreads();
+    if (s_item >= nleaves) break;
+    const int leaf = order[s_item];
+    const RkLeafDesc d = leaves[leaf];
+    if (ranks[leaf] <= 0) continue;
+    const bool tall = d.m >= d.n;
+    const int len = tall ? d.m : d.n, k = tall ? d.n : d.m;
+    const int ld = dense_svd_ld(len);
+    T* A = ws + d.ws_off;
+    T* B = A + (size_t)d.m * d.kcap;
+    T* src = tall ? A : B;    // X, and U S^1/2 in the end
+    T* other = tall ? B : A;  // conj(V) S^1/2
+    for (int c = warp; c < k; c += nw) {
+      double n2 = 0.0;
+      for (int i = lane; i < len; i += 32) {
+        const W v = widen(src[(size_t)c * len + i]);
+        X[(size_t)c * ld + i] = v;
+        n2 += abs2(v);
+      }
+      n2 = warp_sum(n2);
+      if (lane == 0) {
+        s_nrm[c] = n2;
+        s_perm[c] = c;
+      }
+    }
+    __syncthreads();
+    // ---- column-pivoted QR: R in the upper trapezoid of X, columns in pivot order ----
+    int r = 0;
+    for (; r < k; ++r) {
+      if (warp == 0) {
+        KeyIdx best{-1.0, -1};
+        double left = 0.0;
+        for (int c = r + lane; c < k; c += 32) {
+          const double v = s_nrm[c];
+          left += v;
+          if (best.idx < 0 || v > best.key) best = KeyIdx{v, c};
+        }
+        left = warp_sum(left);
+        best = warp_arg<true>(best);
+        if (lane == 0) {
+          if (r == 0) s_total = left;
+          // NaN, Inf or an overflow in the block: no early stop, and the Jacobi below reports it
+          s_piv = (left <= tol * tol * s_total && isfinite(s_total)) ? -1 : best.idx;
+        }
+      }
+      __syncthreads();
+      const int piv = s_piv;
+      if (piv < 0) break;
+      if (piv != r) {
+        for (int i = tid; i < len; i += blockDim.x) {
+          const W a = X[(size_t)r * ld + i], b = X[(size_t)piv * ld + i];
+          X[(size_t)r * ld + i] = b;
+          X[(size_t)piv * ld + i] = a;
+        }
+        if (tid == 0) {
+          const int a = s_perm[r];
+          s_perm[r] = s_perm[piv];
+          s_perm[piv] = a;
+          s_nrm[piv] = s_nrm[r];
+        }
+        __syncthreads();
+      }
+      // Householder vector of column r, formed by every warp alike
+      W* x = X + (size_t)r * ld;
+      double n2 = 0.0;
+      for (int i = r + lane; i < len; i += 32) n2 += abs2(x[i]);
+      n2 = warp_bcast(warp_sum(n2));
+      const double nrm = sqrt(n2);
+      const W alpha = x[r];
+      const double aa = sqrt_abs2(alpha);
+      const W beta = scal(-nrm, phase_of(alpha, aa));
+      const W v0 = alpha - beta;
+      const double vn2 = n2 - aa * aa + abs2(v0);
+      const double t = vn2 > 0.0 ? 2.0 / vn2 : 0.0;
+      // H = I - t v v^H on the columns after r, kDenseSvdBatch of them a warp at a time, with
+      // the norms they keep below row r
+      for (int c0 = r + 1 + warp; c0 < k; c0 += nw * kDenseSvdBatch) {
+        W s[kDenseSvdBatch];
+        double q[kDenseSvdBatch];
+#pragma unroll
+        for (int b = 0; b < kDenseSvdBatch; ++b) {
+          s[b] = zero<W>();
+          q[b] = 0.0;
+        }
+        for (int i = r + lane; i < len; i += 32) {
+          const W v = conjg(i == r ? v0 : x[i]);
+#pragma unroll
+          for (int b = 0; b < kDenseSvdBatch; ++b)
+            if (c0 + b * nw < k) s[b] = s[b] + v * X[(size_t)(c0 + b * nw) * ld + i];
+        }
+#pragma unroll
+        for (int b = 0; b < kDenseSvdBatch; ++b) s[b] = warp_bcast(warp_sum(s[b]));
+        for (int i = r + lane; i < len; i += 32) {
+          const W v = i == r ? v0 : x[i];
+#pragma unroll
+          for (int b = 0; b < kDenseSvdBatch; ++b)
+            if (c0 + b * nw < k) {
+              W* y = X + (size_t)(c0 + b * nw) * ld + i;
+              const W w = *y - scal(t, s[b]) * v;
+              *y = w;
+              if (i > r) q[b] += abs2(w);
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < kDenseSvdBatch; ++b) {
+          q[b] = warp_sum(q[b]);
+          if (lane == 0 && c0 + b * nw < k) s_nrm[c0 + b * nw] = q[b];
+        }
+      }
+      __syncthreads();
+      if (tid == 0) x[r] = beta;  // read again only after the next barrier
+    }
+    __syncthreads();
+    // ---- one-sided Jacobi on Y = R^H: row p of R (conjugated) is column p of Y ----
+    for (int e = tid; e < r * k; e += blockDim.x) {
+      const int p = e % r, j = e / r;
+      W* z = X + (size_t)j * ld + p;
+      *z = j < p ? zero<W>() : conjg(*z);
+    }
+    __syncthreads();
+    const int kk = (r + 1) & ~1;
+    const int max_sweeps = g_jacobi_max_sweeps;
+    bool conv = r <= 1;
+    for (int sweep = 0; sweep < max_sweeps && !conv; ++sweep) {
+      if (tid == 0) s_rot = 0;
+      __syncthreads();
+      for (int round = 0; round < kk - 1; ++round) {
+        for (int pr = warp; pr < kk / 2; pr += nw) {
+          const int a = pr == 0 ? 0 : 1 + (pr - 1 + round) % (kk - 1);
+          const int b = 1 + (kk - 2 - pr + round) % (kk - 1);
+          const int p = min(a, b), q = max(a, b);
+          if (q >= r) continue;
+          W wp[kDenseSvdCols / 32], wq[kDenseSvdCols / 32];
+          double al = 0.0, be = 0.0;
+          W g = zero<W>();
+#pragma unroll
+          for (int h = 0; h < kDenseSvdCols / 32; ++h) {
+            const int j = lane + 32 * h;
+            wp[h] = wq[h] = zero<W>();
+            if (j < k) {
+              wp[h] = X[(size_t)j * ld + p];
+              wq[h] = X[(size_t)j * ld + q];
+              al += abs2(wp[h]);
+              be += abs2(wq[h]);
+              g = g + conjg(wp[h]) * wq[h];
+            }
+          }
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1) {
+            al += __shfl_xor_sync(0xffffffffu, al, off);
+            be += __shfl_xor_sync(0xffffffffu, be, off);
+            g = g + ts_xor(g, off);
+          }
+          const double ag = sqrt(abs2(g));
+          if (ag == 0.0 || ag <= 1e-15 * sqrt(al * be)) continue;
+          if (lane == 0) s_rot = 1;
+          const W phc = conjg(scal(1.0 / ag, g));
+          const double zeta = (be - al) / (2.0 * ag);
+          const double tt = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+          const double cs = 1.0 / sqrt(1.0 + tt * tt), sn = cs * tt;
+#pragma unroll
+          for (int h = 0; h < kDenseSvdCols / 32; ++h) {
+            const int j = lane + 32 * h;
+            if (j < k) {
+              const W x = wp[h], y = wq[h] * phc;
+              X[(size_t)j * ld + p] = scal(cs, x) - scal(sn, y);
+              X[(size_t)j * ld + q] = scal(sn, x) + scal(cs, y);
+            }
+          }
+        }
+        __syncthreads();
+      }
+      conv = !s_rot;
+      __syncthreads();
+    }
+    // ---- singular values in descending order (ties by index), k' ----
+    for (int p = warp; p < r; p += nw) {
+      double s2 = 0.0;
+      for (int j = lane; j < k; j += 32) s2 += abs2(X[(size_t)j * ld + p]);
+      s2 = warp_sum(s2);
+      if (lane == 0) s_nrm[p] = sqrt(s2);
+    }
+    __syncthreads();
+    for (int p = tid; p < r; p += blockDim.x) {
+      int at = 0;
+      for (int i = 0; i < r; ++i) at += (s_nrm[i] > s_nrm[p]) || (s_nrm[i] == s_nrm[p] && i < p);
+      s_ord[at] = p;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      int nk = 0;
+      if (r > 0) {
+        const double thr = s_nrm[s_ord[0]] * eps;
+        while (nk < r && !(s_nrm[s_ord[nk]] <= thr)) nk++;
+      }
+      s_newk = nk;
+    }
+    __syncthreads();
+    const int nk = s_newk;
+    // ---- the factors: conj(V) S^1/2, and U S^1/2 = X V S^-1/2 row by row (a row's outputs are
+    // kept until its inputs are all read: they replace its first k' entries) ----
+    for (int c = warp; c < nk; c += nw) {
+      const int p = s_ord[c];
+      const double f = 1.0 / sqrt(s_nrm[p]);
+      for (int j = lane; j < k; j += 32)
+        other[(size_t)c * k + s_perm[j]] = narrow<T>(scal(f, conjg(X[(size_t)j * ld + p])));
+    }
+    for (int i = tid; i < len; i += blockDim.x) {
+      T keep[kDenseSvdCols];
+      for (int c0 = 0; c0 < nk; c0 += 8) {
+        W acc[8];
+        int row[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          acc[q] = zero<W>();
+          row[q] = c0 + q < nk ? s_ord[c0 + q] : 0;
+        }
+        for (int j = 0; j < k; ++j) {
+          const W xv = widen(src[(size_t)s_perm[j] * len + i]);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) acc[q] = acc[q] + xv * X[(size_t)j * ld + row[q]];
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (c0 + q < nk) {
+            const double sg = s_nrm[row[q]];
+            keep[c0 + q] = narrow<T>(scal(1.0 / (sg * sqrt(sg)), acc[q]));
+          }
+      }
+      for (int c = 0; c < nk; ++c) src[(size_t)c * len + i] = keep[c];
+    }
+    __syncthreads();
+    if (tid == 0) {
+      ranks[leaf] = nk;
+      if (!conv && status[leaf] == kLeafOk) status[leaf] = kLeafSvdNoConverge;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------
 // Tall-skinny truncation of the leaves above the register buckets (rank > 32 real / 16
 // complex, not dense-SVD jobs): the same algorithm as tsqr / tscore / tsapply (triangles of
 // row segments, stacks of triangles, core, factors times maps), each item taken by a CTA of
@@ -899,6 +1184,36 @@ void launch_truncate(const RkLeafDesc* d_leaves, const int* d_order, int nleaves
   int g = grid < nleaves ? grid : nleaves;
   truncate_kernel<T><<<g, kTruncThreads, 0, s>>>(d_leaves, d_order, nleaves, epsilon, ws, ranks, status, counter,
                                                 scratch, slab_elems);
+}
+
+template <typename T>
+bool dense_svd_fits(int m, int n) {
+  const int k = m < n ? m : n, len = m < n ? n : m;
+  return k <= kDenseSvdCols && (size_t)dense_svd_ld(len) * k * sizeof(typename Traits<T>::wide) <= kDenseSvdSmem;
+}
+
+template <typename T>
+cudaError_t launch_dense_svd(const RkLeafDesc* d_leaves, const int* d_order, int nleaves, int max_m, int max_n,
+                             double epsilon, T* ws, int* ranks, int* status, int* counter, cudaStream_t s) {
+  auto kern = dense_svd_kernel<T>;
+  if (nleaves <= 0) {
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, kern);
+  }
+  const int k = max_m < max_n ? max_m : max_n, len = max_m < max_n ? max_n : max_m;
+  size_t smem = (size_t)dense_svd_ld(len) * k * sizeof(typename Traits<T>::wide);
+  if (smem > kDenseSvdSmem) smem = kDenseSvdSmem;  // a tall leaf beside a wide one: each fits by itself
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSvdSmem);
+  if (e != cudaSuccess) return e;
+  e = cudaMemsetAsync(counter, 0, sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kDenseSvdThreads, smem) != cudaSuccess || per_sm < 1)
+    per_sm = 1;
+  const int g = persistent_grid(per_sm);
+  kern<<<g < nleaves ? g : nleaves, kDenseSvdThreads, smem, s>>>(d_leaves, d_order, nleaves, epsilon, ws, ranks, status,
+                                                                 counter);
+  return cudaGetLastError();
 }
 
 template <typename T>
@@ -1115,6 +1430,7 @@ void preload_truncate_kernels() {
   typedef typename Traits<T>::wide W;
   cudaFuncAttributes a;
   cudaFuncGetAttributes(&a, truncate_kernel<T>);
+  launch_dense_svd<T>(nullptr, nullptr, 0, 0, 0, 0.0, nullptr, nullptr, nullptr, nullptr, 0);
   cudaFuncGetAttributes(&a, compact_kernel<T>);
   cudaFuncGetAttributes(&a, unpack_kernel<T>);
   const int kmax = ts_kmax<T>();
@@ -1134,6 +1450,9 @@ void preload_truncate_kernels() {
   template long long truncate_slab_elems<T>(int, int, int);                                               \
   template void launch_truncate<T>(const RkLeafDesc*, const int*, int, double, T*, int*, int*, int*,     \
                                    typename Traits<T>::wide*, long long, int, cudaStream_t);               \
+  template bool dense_svd_fits<T>(int, int);                                                               \
+  template cudaError_t launch_dense_svd<T>(const RkLeafDesc*, const int*, int, int, int, double, T*, int*, int*, \
+                                           int*, cudaStream_t);                                            \
   template void launch_compact<T>(const RkLeafDesc*, int, const T*, const int*, const RkStoreDesc*,        \
                                   const PanelDesc*, T*, cudaStream_t);                                    \
   template void launch_unpack<T>(const RkLeafDesc*, int, const int*, const RkStoreDesc*, const PanelDesc*,  \
