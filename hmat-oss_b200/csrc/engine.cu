@@ -974,7 +974,7 @@ class Engine : public EngineBase {
 
     // ---- the dense-SVD jobs: SVD of the dense blocks at the compression epsilon (a stratum's
     // dense sum: at the low-rank epsilon, truncatedSvd in formattedAddParts); the regular
-    // truncation below then takes them like every other leaf, at the ranks they come back with ----
+    // truncation below follows, at the ranks they come back with ----
     compress_dense(jobs, desc, h_status, h_ranks, add_stratum ? eps_trunc : eps_aca, d_desc.p, d_ws.p, d_ranks.p,
                    d_status.p, d_counter.p);
 
@@ -997,9 +997,12 @@ class Engine : public EngineBase {
     std::stable_sort(good.begin(), good.end(), [&](int x, int y) { return tcost(x) > tcost(y); });
 
     typedef typename Traits<T>::wide W;
-    DevArray<W> d_tri, d_maps;
+    DevArray<W> d_scratch, d_tri, d_maps;
+    DevArray<int> d_large;
     DevArray<TsItem> d_ts_seg[4], d_ts_stack[4];
     DevArray<TsCore> d_ts_core[4];
+    long long slab = 0, grid = 0;
+    std::vector<int> large;
     std::vector<TsItem> ts_seg[4], ts_stack[4];
     std::vector<TsCore> ts_core[4];
     bool any_ts = false;
@@ -1014,11 +1017,21 @@ class Engine : public EngineBase {
     if (!good.empty()) {
       // Leaves up to rank ts_kmax go to the tall-skinny phases (row segments of A and B
       // reduced to triangles, stacks of triangles reduced again, core, apply), higher ranks
-      // to the same phases with a CTA per item.
+      // to the same phases with a CTA per item.  The dense-SVD jobs go to the CTA-per-leaf kernel:
+      // the signs (phases) of its factor columns come from B's entries alone, not from the signs
+      // their SVD happened to give them.
+      int big_m = 1, big_n = 1, big_k = 1;
       long long tri_n = 0, map_n = 0, tb_tri = 0, tb_map = 0;
       int tb_rows = 1, tb_k = 1;
       const int kmax = ts_kmax<T>();
       for (int b : good) {
+        if (jobs[b].svd) {
+          large.push_back(b);
+          big_m = std::max(big_m, desc[b].m);
+          big_n = std::max(big_n, desc[b].n);
+          big_k = std::max(big_k, h_ranks[b]);
+          continue;
+        }
         const int K = ts_bucket(h_ranks[b], kmax);
         if (!K) {
           // segments of at least k rows (the last one takes the remainder)
@@ -1120,6 +1133,7 @@ class Engine : public EngineBase {
         ts_core[q].push_back(c);
         any_ts = true;
       }
+      if (!large.empty()) grid = alloc_slabs(d_scratch, big_m, big_n, big_k, large.size(), &slab);
       if (any_ts) {
         d_tri.alloc((size_t)tri_n);
         d_maps.alloc((size_t)map_n);
@@ -1153,12 +1167,13 @@ class Engine : public EngineBase {
         d_tb_stack.upload(tb_stack, stream_);
         d_tb_core.upload(tb_core, stream_);
       }
+      d_large.upload(large, stream_);
       HB_CUDA(cudaStreamSynchronize(stream_));
     }
     HB_CUDA(cudaEventRecord(ev_[4], stream_));
     if (!good.empty()) {
-      // the warp-level phases hold leaves disjoint from the CTA-per-item ones: they run on a
-      // second stream beside them
+      // the warp-level phases hold leaves disjoint from the CTA kernels': they run on a second
+      // stream beside them
       if (any_ts) {
         HB_CUDA(cudaEventRecord(fork_[0], stream_));
         HB_CUDA(cudaStreamWaitEvent(stream2_, fork_[0], 0));
@@ -1172,6 +1187,12 @@ class Engine : public EngineBase {
           HB_CUDA(cudaGetLastError());
         }
         HB_CUDA(cudaEventRecord(fork_[1], stream2_));
+      }
+      if (!large.empty()) {
+        HB_CUDA(cudaMemsetAsync(d_counter.p, 0, sizeof(int), stream_));
+        launch_truncate<T>(d_desc.p, d_large.p, (int)large.size(), eps_trunc, d_ws.p, d_ranks.p, d_status.p,
+                           d_counter.p, d_scratch.p, slab, (int)grid, stream_);
+        HB_CUDA(cudaGetLastError());
       }
       if (!tb_core.empty()) {
         launch_tsqr_cta<T>(d_tb_seg.p, (int)tb_seg.size(), d_ws.p, d_tb_tri.p, false, d_tb_scratch.p, tb_slab,
@@ -1247,6 +1268,23 @@ class Engine : public EngineBase {
     pieces_.push_back(std::move(piece));
   }
 
+  // Slabs of the CTA-per-leaf truncation of `count` leaves of at most m x n at rank k; returns the
+  // grid.
+  long long alloc_slabs(DevArray<typename Traits<T>::wide>& scratch, int m, int n, int k, size_t count,
+                        long long* slab) {
+    typedef typename Traits<T>::wide W;
+    *slab = truncate_slab_elems<T>(m, n, k);
+    // the slabs are sized for the largest leaf: let them use a third of the free memory
+    // when that is more than the ACA budget, so long leaves still fill the grid
+    size_t budget = workspace_budget();
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) budget = std::max(budget, free_b / 3);
+    long long grid = std::min<long long>((long long)count, persistent_grid(2));
+    grid = std::max(1LL, std::min<long long>(grid, (long long)(budget / (*slab * sizeof(W)))));
+    scratch.alloc((size_t)(grid * *slab));
+    return grid;
+  }
+
   // The first truncation of the dense-SVD jobs of a batch (rank min(m, n) on entry): h_ranks and
   // the device's ranks become those of their SVDs at `eps`.  A block whose wide copy fits shared
   // memory goes to the shared-memory kernel, a larger one to the CTA-per-leaf kernel on slabs.
@@ -1280,17 +1318,7 @@ class Engine : public EngineBase {
     d_small.upload(small, stream_);
     d_large.upload(large, stream_);
     long long slab = 0, grid = 0;
-    if (!large.empty()) {
-      slab = truncate_slab_elems<T>(lm, ln, lk);
-      // the slabs are sized for the largest leaf: let them use a third of the free memory
-      // when that is more than the ACA budget, so long leaves still fill the grid
-      size_t budget = workspace_budget();
-      size_t free_b = 0, total_b = 0;
-      if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) budget = std::max(budget, free_b / 3);
-      grid = std::min<long long>((long long)large.size(), persistent_grid(2));
-      grid = std::max(1LL, std::min<long long>(grid, (long long)(budget / (slab * sizeof(W)))));
-      d_scratch.alloc((size_t)(grid * slab));
-    }
+    if (!large.empty()) grid = alloc_slabs(d_scratch, lm, ln, lk, large.size(), &slab);
     HB_CUDA(cudaStreamSynchronize(stream_));
     HB_CUDA(cudaEventRecord(ev_[4], stream_));
     if (!small.empty())

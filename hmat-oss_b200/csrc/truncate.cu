@@ -737,11 +737,9 @@ __global__ void __launch_bounds__(kTsWarps * 32) tsapply_kernel(const TsItem* __
 // which Jacobi converges on in a few sweeps), so neither Q nor J is formed: U S^1/2 =
 // X V S^-1/2, read from the block that still stands in the slot.
 //
-// Bound by the latency of the Jacobi rounds.  The slab kernel above, which these blocks took
-// before, rotates all k columns in global memory, the noise columns (norms near u sigma_0) in
-// every sweep: with the default compressionMinLeafSize the truncation of the 8,000-point
-// cylinder (leaf 64, epsilon 1e-4, FP64; 1,716 blocks of up to 63 x 63) took 37.8 ms, and 3.9 ms
-// with this kernel followed by the tall-skinny phases.
+// For the complex types; a complex factor's columns carry arbitrary phases.  Real blocks keep the
+// rotations of the slab kernel (dense_jacobi_kernel), whose rounding decides the signs of the
+// factors that gradients are taken by.
 constexpr int kDenseSvdThreads = 256;
 constexpr int kDenseSvdCols = 128;  // columns of X at most: four per lane of a Jacobi row
 // Columns a warp updates together in a QR step (their shuffle sums overlap).
@@ -1008,6 +1006,209 @@ __global__ void __launch_bounds__(kDenseSvdThreads) dense_svd_kernel(const RkLea
   }
 }
 
+// The same compression for real blocks, on truncate_kernel's own arithmetic: every sum, rotation
+// and reflection has its operands and its order, so the factors are bit for bit those of the slab
+// kernel (their signs come out of the rounding of nearly converged rotations).
+//
+// The block, the rotated matrix and V sit in shared memory, and what the identity factor adds is
+// known: its QR is R = -I and its Q negates.  A Jacobi pair takes 16 lanes, two pairs a warp, all
+// pairs of 64 columns in one pass of 512 threads: the scalar chain of a rotation (square roots and
+// divides, about 170 dependent FP64 operations) bounds a round, a warp runs it for two pairs at
+// once, and the other warps' loads and sums hide behind it.  The lanes add their elements in the
+// order of a warp's sum over lanes 0 .. 31: chains over v, v + 32, ... for the virtual lanes
+// v = l + 16 c, then (v, v + 16), (v, v + 8), ... .
+//
+// 8,000-point cylinder (leaf 64, epsilon 1e-4, FP64), default compressionMinLeafSize, 1,048 blocks
+// of up to 63 x 63: truncation 37.8 ms with every block on the slab kernel, 15.7 ms here (4 lanes
+// a pair 22.1 ms, 8 lanes 17.6 ms).
+constexpr int kDenseJacobiLanes = 16;                        // lanes a pair
+constexpr int kDenseJacobiThreads = 32 * kDenseJacobiLanes;  // all pairs of 64 columns at once
+constexpr int kDenseJacobiChain = 3;  // elements of a chain: columns of at most 96
+constexpr size_t kDenseJacobiSmem = 216 * 1024;
+
+__host__ __device__ constexpr size_t dense_jacobi_smem(int len, int k) {
+  return (size_t)3 * len * k * sizeof(double) + 2 * (size_t)k * sizeof(double) + (size_t)k * sizeof(int);
+}
+
+// Sum over the virtual lanes of a pair's lanes (v[c]: virtual lane l + L c), as warp_sum adds 32
+// lanes.
+template <int L>
+__device__ __forceinline__ double lanes_sum(const double (&v)[32 / L]) {
+  double t[32 / L];
+#pragma unroll
+  for (int c = 0; c < 32 / L; ++c) t[c] = v[c];
+#pragma unroll
+  for (int n = 16 / L; n > 0; n >>= 1)
+#pragma unroll
+    for (int c = 0; c < n; ++c) t[c] = __dadd_rn(t[c], t[c + n]);
+  double s = t[0];
+#pragma unroll
+  for (int off = L / 2; off > 0; off >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, off));
+  return s;
+}
+
+// jacobi_svd with L lanes a pair; Wm and V in shared memory.
+template <int L>
+__device__ bool jacobi_svd_lanes(double* Wm, double* V, int k, int* s_rot) {
+  constexpr int C = 32 / L, H = kDenseJacobiChain;
+  const int l = threadIdx.x % L, grp = threadIdx.x / L, ngrp = blockDim.x / L;
+  const int kk = (k + 1) & ~1;
+  const int max_sweeps = g_jacobi_max_sweeps;
+  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    if (threadIdx.x == 0) *s_rot = 0;
+    __syncthreads();
+    for (int round = 0; round < kk - 1; ++round) {
+      for (int pr0 = 0; pr0 < kk / 2; pr0 += ngrp) {  // block-uniform: every lane joins the shuffles
+        const int pr = pr0 + grp;
+        const int a = pr == 0 ? 0 : 1 + (pr - 1 + round) % (kk - 1);
+        const int b = 1 + (kk - 2 - pr + round) % (kk - 1);
+        const int p = min(a, b), q = max(a, b);
+        const bool live = pr < kk / 2 && q < k;
+        double* wp = Wm + (size_t)(live ? p : 0) * k;
+        double* wq = Wm + (size_t)(live ? q : 0) * k;
+        double x[C][H], y[C][H], alc[C], bec[C], gc[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          double al = 0.0, be = 0.0, g = 0.0;
+#pragma unroll
+          for (int h = 0; h < H; ++h) {
+            const int i = l + L * c + 32 * h;
+            const bool in = live && i < k;
+            x[c][h] = in ? wp[i] : 0.0;
+            y[c][h] = in ? wq[i] : 0.0;
+            al = fma(x[c][h], x[c][h], al);
+            be = fma(y[c][h], y[c][h], be);
+            g = fma(x[c][h], y[c][h], g);
+          }
+          alc[c] = al;
+          bec[c] = be;
+          gc[c] = g;
+        }
+        const double al = lanes_sum<L>(alc), be = lanes_sum<L>(bec), g = lanes_sum<L>(gc);
+        const double ag = sqrt(abs2(g));
+        if (!live || ag == 0.0 || ag <= 1e-15 * sqrt(al * be)) continue;
+        if (l == 0) *s_rot = 1;
+        const double phc = __dmul_rn(1.0 / ag, g);
+        const double zeta = __dsub_rn(be, al) / __dmul_rn(2.0, ag);
+        const double t = (zeta >= 0.0 ? 1.0 : -1.0) / __dadd_rn(fabs(zeta), sqrt(fma(zeta, zeta, 1.0)));
+        const double cs = 1.0 / sqrt(fma(t, t, 1.0)), sn = __dmul_rn(cs, t);
+        double* vp = V + (size_t)p * k;
+        double* vq = V + (size_t)q * k;
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+          for (int h = 0; h < H; ++h) {
+            const int i = l + L * c + 32 * h;
+            if (i < k) {
+              // the roundings of the slab kernel's rotation, pinned
+              const double wx = x[c][h], wy = __dmul_rn(y[c][h], phc);
+              wp[i] = fma(cs, wx, -__dmul_rn(sn, wy));
+              wq[i] = fma(sn, wx, __dmul_rn(cs, wy));
+              const double vx = vp[i], vy = __dmul_rn(vq[i], phc);
+              vp[i] = fma(cs, vx, -__dmul_rn(sn, vy));
+              vq[i] = fma(sn, vx, __dmul_rn(cs, vy));
+            }
+          }
+      }
+      __syncthreads();
+    }
+    if (!*s_rot) return true;
+    __syncthreads();
+  }
+  return false;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kDenseJacobiThreads, 2) dense_jacobi_kernel(const RkLeafDesc* __restrict__ leaves,
+                                                                            const int* __restrict__ order,
+                                                                            int nleaves, double eps, T* ws,
+                                                                            int* ranks, int* status, int* counter) {
+  extern __shared__ __align__(16) unsigned char dj_smem[];
+  __shared__ RedScratch rs;
+  __shared__ int s_item, s_rot, s_newk;
+  const int tid = threadIdx.x;
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) s_item = atomicAdd(counter, 1);
+    __syncthreads();
+    if (s_item >= nleaves) break;
+    const int leaf = order[s_item];
+    const RkLeafDesc d = leaves[leaf];
+    if (ranks[leaf] <= 0) continue;
+    const bool tall = d.m >= d.n;
+    const int len = tall ? d.m : d.n, k = tall ? d.n : d.m;
+    T* A = ws + d.ws_off;
+    T* B = A + (size_t)d.m * d.kcap;
+    T* src = tall ? A : B;    // the block (or its transpose), len x k
+    T* other = tall ? B : A;  // the identity, k x k
+    double* X = reinterpret_cast<double*>(dj_smem);
+    double* Rm = X + (size_t)len * k;
+    double* Vm = Rm + (size_t)len * k;
+    double* tau = Vm + (size_t)len * k;
+    double* sig = tau + k;
+    int* ord = reinterpret_cast<int*>(sig + k);
+    for (int e = tid; e < len * k; e += blockDim.x) X[e] = widen(src[e]);
+    __syncthreads();
+    householder_qr(X, len, k, tau, Vm, rs);
+    __syncthreads();
+    // Ra Rb^T with the identity's R = -I: -R when the block is A, -R^T when it is B
+    for (int e = tid; e < k * k; e += blockDim.x) {
+      const int i = e % k, j = e / k;
+      Rm[e] = tall ? (i <= j ? -Vm[e] : 0.0) : (i >= j ? -Vm[j + (size_t)i * k] : 0.0);
+    }
+    __syncthreads();
+    for (int e = tid; e < k * k; e += blockDim.x) Vm[e] = e % (k + 1) == 0 ? 1.0 : 0.0;
+    __syncthreads();
+    const bool conv = jacobi_svd_lanes<kDenseJacobiLanes>(Rm, Vm, k, &s_rot);
+    for (int j = tid; j < k; j += blockDim.x) {
+      double s2 = 0.0;
+      for (int i = 0; i < k; ++i) s2 += abs2(Rm[i + (size_t)j * k]);
+      sig[j] = sqrt(s2);
+    }
+    __syncthreads();
+    // descending order, ties by index (stable)
+    for (int j = tid; j < k; j += blockDim.x) {
+      int r = 0;
+      for (int i = 0; i < k; ++i) r += (sig[i] > sig[j]) || (sig[i] == sig[j] && i < j);
+      ord[r] = j;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      const double thr = sig[ord[0]] * eps;
+      int nk = 0;
+      while (nk < k && !(sig[ord[nk]] <= thr)) nk++;
+      s_newk = nk;
+    }
+    __syncthreads();
+    const int nk = s_newk;
+    // U sqrt(S) from the rotated matrix, V sqrt(S); the identity's side is done once negated, the
+    // block's is set up where the other side's matrix was and taken through Q
+    auto left = [&](int i, int c) {
+      const double sc = sig[ord[c]];
+      return sc > 0.0 ? scal(1.0 / sqrt(sc), Rm[i + (size_t)ord[c] * k]) : 0.0;
+    };
+    auto right = [&](int i, int c) { return scal(sqrt(sig[ord[c]]), Vm[i + (size_t)ord[c] * k]); };
+    for (int e = tid; e < k * nk; e += blockDim.x) {
+      const int i = e % k, c = e / k;
+      other[e] = narrow<T>(-(tall ? right(i, c) : left(i, c)));
+    }
+    __syncthreads();
+    double* C = tall ? Vm : Rm;
+    for (int e = tid; e < len * nk; e += blockDim.x) {
+      const int i = e % len, c = e / len;
+      C[e] = i < k ? (tall ? left(i, c) : right(i, c)) : 0.0;
+    }
+    __syncthreads();
+    apply_q(X, len, k, tau, C, nk);
+    for (int e = tid; e < len * nk; e += blockDim.x) src[e] = narrow<T>(C[e]);
+    __syncthreads();
+    if (tid == 0) {
+      ranks[leaf] = nk;
+      if (!conv && status[leaf] == kLeafOk) status[leaf] = kLeafSvdNoConverge;
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------------
 // Tall-skinny truncation of the leaves above the register buckets (rank > 32 real / 16
 // complex, not dense-SVD jobs): the same algorithm as tsqr / tscore / tsapply (triangles of
@@ -1189,31 +1390,38 @@ void launch_truncate(const RkLeafDesc* d_leaves, const int* d_order, int nleaves
 template <typename T>
 bool dense_svd_fits(int m, int n) {
   const int k = m < n ? m : n, len = m < n ? n : m;
+  // real: the QR's norms must be one element a thread, as in the slab kernel's 256
+  if constexpr (!Traits<T>::is_complex)
+    return k <= 32 * kDenseJacobiChain && len <= kTruncThreads && dense_jacobi_smem(len, k) <= kDenseJacobiSmem;
   return k <= kDenseSvdCols && (size_t)dense_svd_ld(len) * k * sizeof(typename Traits<T>::wide) <= kDenseSvdSmem;
 }
 
 template <typename T>
 cudaError_t launch_dense_svd(const RkLeafDesc* d_leaves, const int* d_order, int nleaves, int max_m, int max_n,
                              double epsilon, T* ws, int* ranks, int* status, int* counter, cudaStream_t s) {
-  auto kern = dense_svd_kernel<T>;
-  if (nleaves <= 0) {
-    cudaFuncAttributes a;
-    return cudaFuncGetAttributes(&a, kern);
-  }
   const int k = max_m < max_n ? max_m : max_n, len = max_m < max_n ? max_n : max_m;
-  size_t smem = (size_t)dense_svd_ld(len) * k * sizeof(typename Traits<T>::wide);
-  if (smem > kDenseSvdSmem) smem = kDenseSvdSmem;  // a tall leaf beside a wide one: each fits by itself
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSvdSmem);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(counter, 0, sizeof(int), s);
-  if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kDenseSvdThreads, smem) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  const int g = persistent_grid(per_sm);
-  kern<<<g < nleaves ? g : nleaves, kDenseSvdThreads, smem, s>>>(d_leaves, d_order, nleaves, epsilon, ws, ranks, status,
-                                                                 counter);
-  return cudaGetLastError();
+  auto run = [&](auto kern, int threads, size_t smem, size_t most) {
+    if (nleaves <= 0) {
+      cudaFuncAttributes a;
+      return cudaFuncGetAttributes(&a, kern);
+    }
+    if (smem > most) smem = most;  // a tall leaf beside a wide one: each fits by itself
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e != cudaSuccess) return e;
+    e = cudaMemsetAsync(counter, 0, sizeof(int), s);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess || per_sm < 1)
+      per_sm = 1;
+    const int g = persistent_grid(per_sm);
+    kern<<<g < nleaves ? g : nleaves, threads, smem, s>>>(d_leaves, d_order, nleaves, epsilon, ws, ranks, status,
+                                                          counter);
+    return cudaGetLastError();
+  };
+  if constexpr (Traits<T>::is_complex)
+    return run(dense_svd_kernel<T>, kDenseSvdThreads, (size_t)dense_svd_ld(len) * k * sizeof(cdouble), kDenseSvdSmem);
+  else
+    return run(dense_jacobi_kernel<T>, kDenseJacobiThreads, dense_jacobi_smem(len, k), kDenseJacobiSmem);
 }
 
 template <typename T>
