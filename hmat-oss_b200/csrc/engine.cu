@@ -301,7 +301,8 @@ class Engine : public EngineBase {
     check_gemv_args(trans, nrhs);
     if (nrhs == 0) return;
     const T a = *(const T*)alpha, b = *(const T*)beta;
-    xz_.ensure(xz_elems());
+    DevArray<T>& scratch = trans == 'N' ? xz_ : rz_;
+    scratch.ensure(xz_elems(trans == 'N' ? 0 : 1));
     GraphKey key(trans, nrhs, x, y);
     memcpy(key.ab, &a, sizeof(T));
     memcpy(key.ab + sizeof(T), &b, sizeof(T));
@@ -312,7 +313,7 @@ class Engine : public EngineBase {
       }
       cudaGraph_t g;
       HB_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-      launch_gemv<T>(plan_, trans, nrhs, a, b, (const T*)x, (T*)y, xz_.p, err_.p, stream_);
+      launch_gemv<T>(plan_, trans, nrhs, a, b, (const T*)x, (T*)y, scratch.p, err_.p, stream_);
       cudaError_t launch_err = cudaGetLastError();
       HB_CUDA(cudaStreamEndCapture(stream_, &g));
       HB_CUDA(launch_err);
@@ -396,8 +397,8 @@ class Engine : public EngineBase {
     if (Traits<T>::is_complex) throw Error("leaf gradients are implemented for real value types");
     if (nrhs < 1 || nrhs > 16) throw Error("leaf gradients take 1 to 16 right-hand sides");
     check_device();
-    xz_.ensure(xz_elems());
-    rz_.ensure(xz_elems());
+    xz_.ensure(xz_elems(0));
+    rz_.ensure(xz_elems(1));
     cudaStream_t s = user_stream ? user_stream : stream_;
     launch_leaf_gradients<T>(plan_, nrhs, (const T*)x, (const T*)r, xz_.p, rz_.p, (T*)grad, (T*)grad, accumulate,
                              err_.p, s);
@@ -410,8 +411,8 @@ class Engine : public EngineBase {
     if (Traits<T>::is_complex) throw Error("the adjoint is implemented for real value types");
     if (nrhs < 1 || nrhs > 16) throw Error("the adjoint takes 1 to 16 right-hand sides");
     check_device();
-    xz_.ensure(xz_elems());
-    rz_.ensure(xz_elems());
+    xz_.ensure(xz_elems(0));
+    rz_.ensure(xz_elems(1));
     cudaStream_t s = user_stream ? user_stream : stream_;
     launch_gemv_adjoint<T>(plan_, nrhs, (const T*)x, (const T*)r, (T*)dx, xz_.p, rz_.p, (T*)grad, (T*)grad, accumulate,
                            err_.p, s);
@@ -547,10 +548,11 @@ class Engine : public EngineBase {
   void profile_gemv(char trans, const void* x, void* y, int nrhs, double* ms3, double* bytes3) override {
     check_gemv_args(trans, nrhs);
     if (nrhs < 1 || nrhs > 16) throw Error("profile_gemv takes 1 to 16 right-hand sides");
-    xz_.ensure(xz_elems());
+    DevArray<T>& scratch = trans == 'N' ? xz_ : rz_;
+    scratch.ensure(xz_elems(trans == 'N' ? 0 : 1));
     GemvTiming tm;
     for (int i = 0; i < 4; ++i) HB_CUDA(cudaEventCreate(&tm.ev[i]));
-    launch_gemv<T>(plan_, trans, nrhs, one<T>(), zero<T>(), (const T*)x, (T*)y, xz_.p, err_.p, stream_, &tm);
+    launch_gemv<T>(plan_, trans, nrhs, one<T>(), zero<T>(), (const T*)x, (T*)y, scratch.p, err_.p, stream_, &tm);
     cudaError_t le = cudaGetLastError();
     cudaError_t se = cudaStreamSynchronize(stream_);
     float a = 0, b = 0, c = 0;
@@ -578,11 +580,14 @@ class Engine : public EngineBase {
     }
     const double n_in = trans == 'N' ? C_->n : R_->n, n_out = trans == 'N' ? R_->n : C_->n;
     bytes3[0] = 2.0 * n_in * nrhs * s;
-    bytes3[1] = (trans == 'N' ? fb : fa) * s;
-    bytes3[2] = (full + (trans == 'N' ? fa : fb)) * s + n_out * nrhs * s;
+    // 'T': the column pass reads the full leaves with the A panels
+    bytes3[1] = (trans == 'N' ? fb : full + fa) * s;
+    bytes3[2] = (trans == 'N' ? full + fa : fb) * s + n_out * nrhs * s;
   }
 
-  size_t gemv_scratch_bytes() const override { return xz_elems() * sizeof(T); }
+  size_t gemv_scratch_bytes() const override {
+    return (size_t)std::max(noalloc_rows_, 1LL) * gemv_rhs_stride((int)sizeof(T), 16) * sizeof(T);
+  }
   int gemv_launches(char trans, int nrhs) const override {
     if (!assembled) throw Error("matrix not assembled");
     return gemv_launch_count(plan_, trans, nrhs, (int)sizeof(T));
@@ -592,11 +597,18 @@ class Engine : public EngineBase {
                                 cudaStream_t stream, void* scratch, size_t scratch_bytes) override {
     check_gemv_args(trans, nrhs);
     if (nrhs == 0) return;
-    if (gemv_scratch_bytes() > scratch_bytes) throw Error("scratch buffer too small for this matrix");
+    // the widest tile of right-hand sides whose rows fit (the partial rows of a transposed product
+    // of a large matrix may not fit at 16)
+    int tile = 16;
+    auto need = [&]() {
+      return (size_t)plan_.xz_rows[trans == 'N' ? 0 : 1] * gemv_rhs_stride((int)sizeof(T), tile) * sizeof(T);
+    };
+    while (tile > 1 && need() > scratch_bytes) tile = tile > 4 ? tile / 2 : 1;
+    if (need() > scratch_bytes) throw Error("scratch buffer too small for this matrix");
     cudaStream_t s = stream ? stream : stream_;
     // the status flag is the matrix's own (allocated with the engine), read by gemv_status
     launch_gemv<T>(plan_, trans, nrhs, *(const T*)alpha, *(const T*)beta, (const T*)x, (T*)y, (T*)scratch, err_.p,
-                   s);
+                   s, nullptr, tile);
     HB_CUDA(cudaGetLastError());
   }
 
@@ -629,8 +641,10 @@ class Engine : public EngineBase {
     }
   };
 
-  size_t xz_elems() const {
-    return (size_t)std::max(plan_.xz_rows, 1LL) * gemv_rhs_stride((int)sizeof(T), 16);
+  // Elements of the scratch of an 'N' (side 0) or 'T' / 'C' product in its widest tiles of
+  // right-hand sides (16; complex double 4).  Products in the two directions use a buffer each (xz_, rz_).
+  size_t xz_elems(int side) const {
+    return (size_t)std::max(plan_.xz_rows[side], 1LL) * gemv_rhs_stride((int)sizeof(T), sizeof(T) >= 16 ? 4 : 16);
   }
 
   static constexpr const char* kWaitGaveUp =
@@ -1753,10 +1767,12 @@ class Engine : public EngineBase {
   // gemv schedule
   struct SideBuf {
     DevArray<GemvUnit> units;
-    DevArray<GemvTask> tasks[GemvSide::kMaxLaunch + 1];
-    DevArray<int> begin[GemvSide::kMaxLaunch + 1];
+    DevArray<GemvTransUnit> tunits;
+    DevArray<GemvTask> tasks[GemvSide::kMaxLaunch + 2];
+    DevArray<int> begin[GemvSide::kMaxLaunch + 2];
     DevArray<GemvZred> zred;
     DevArray<int> zcnt;
+    DevArray<int> colmap;
     DevArray<int2> yrows;
   };
 
@@ -1765,14 +1781,9 @@ class Engine : public EngineBase {
   // (cylinder 100,000, 16 RHS, FP64: z-phase 0.385 -> 0.352 ms).  Not the FP32 tensor-core
   // z-phase, whose short kernel ends later by the chunks' fences and the last warps' sums than
   // the separate pass takes (0.134 -> 0.141 ms).
-  static bool zsum_in_kernel(bool trans) { return !trans && !kTensorN; }
+  static constexpr bool kZsumInKernel = !std::is_same<T, float>::value;
 
   static int rank_class(int k) { return k <= 16 ? 0 : (k <= 32 ? 1 : (k <= 64 ? 2 : 3)); }
-  static void class_shape(int c, int& ol, int& rpt) {
-    ol = c == 0 ? 16 : 32;
-    rpt = c <= 1 ? 1 : (c == 2 ? 2 : 4);
-  }
-
   // Columns per unit of a warp-level launch: the piece (O x cols) and its X rows fit one
   // pipeline stage at the widest right-hand-side tile.
   static int warp_unit_cols(int O) {
@@ -1852,48 +1863,34 @@ class Engine : public EngineBase {
       u.push_back(g);
     }
   }
-  // Units of out[o_base + w] += sum_i P[i, w] X[i] for a column-major C x W block at `poff`.
-  void ptx_units(std::vector<GemvUnit>& u, long long poff, int C, int W, int o_base, int xrow) {
-    if (C > 128) throw Error("gemv plan: transposed inner extent above 128 (rank or block too large)");
-    for (int w0 = 0; w0 < W; w0 += 32) {
-      GemvUnit g{};  // nruns = 0: contiguous X rows
-      g.poff = poff + (long long)w0 * C;
-      g.xrow = xrow;
-      g.c = C;
-      g.o0 = o_base + w0;
-      g.ow = std::min(32, W - w0);
-      g.pel = C * g.ow;
-      g.shift = (int)(g.poff % kPad);
-      u.push_back(g);
-    }
-  }
-
-  // Contiguous ranges of tasks of about equal bytes for a persistent grid: one range per
-  // CTA, or per warp for warp-level launches.  Returns the range starts; *ncta is the grid.
-  // CTAs of the persistent grid of a launch: as many as fit the SMs at once.
-  static int launch_ctas(int omax, bool transposed, bool warp_level, int map) {
-    const int Rmax = sizeof(T) >= 16 ? 4 : 16;
-    const int RS16 = gemv_rhs_stride((int)sizeof(T), Rmax);
-    const size_t smem = map == 4      ? umma_smem_bytes()
-                        : warp_level ? warp_stream_smem_bytes((int)sizeof(T))
-                                     : stream_smem_bytes((int)sizeof(T), Rmax, RS16, omax, transposed);
-    // warp-level kernels: 228 KB of shared memory an SM, 1 KB reserved a CTA (their launch
-    // bounds guarantee the registers for that many CTAs)
-    // (shared memory is allocated in 128-byte granules)
+  // CTAs of the persistent grid of an 'N' launch: as many as fit the SMs at once.
+  static int launch_ctas(int omax, int map) {
+    const size_t smem = map == 4 ? umma_smem_bytes() : warp_stream_smem_bytes((int)sizeof(T));
+    // 228 KB of shared memory an SM, 1 KB reserved a CTA, allocated in 128-byte granules (the
+    // kernels' launch bounds guarantee the registers for that many CTAs)
     const size_t alloc = (smem + 127) / 128 * 128;
-    int per_sm = (int)std::min<size_t>(8, ((warp_level ? 228 : 226) * 1024) / (alloc + 1024));
+    int per_sm = (int)std::min<size_t>(8, (228 * 1024) / (alloc + 1024));
     if (map == 3) per_sm = std::min(per_sm, mma_stream_blocks_per_sm(omax / 8, (int)sizeof(T)));  // registers
     per_sm = std::max(per_sm, 1);
     return persistent_grid(per_sm);
   }
+  // CTAs of a transposed launch of `smem` bytes a CTA.
+  static int trans_ctas(size_t smem) {
+    if (smem > (size_t)kMaxCtaSmem) throw Error("gemv plan: transposed launch above the shared memory of a CTA");
+    const size_t alloc = (smem + 127) / 128 * 128;
+    const size_t most = (size_t)trans_ctas_per_sm((int)sizeof(T));
+    return persistent_grid((int)std::max<size_t>(1, std::min(most, (228 * 1024) / (alloc + 1024))));
+  }
 
-  std::vector<int> partition(const std::vector<GemvTask>& tasks, const std::vector<GemvUnit>& units, int omax,
-                             bool transposed, bool warp_level, int map, int* ncta) {
+  // Contiguous ranges of tasks of about equal bytes, one per warp of the grid.  Returns the
+  // range starts; *ncta is the grid.
+  std::vector<int> partition(const std::vector<GemvTask>& tasks, const std::vector<GemvUnit>& units, int omax, int map,
+                             int* ncta) {
     const int Rmax = sizeof(T) >= 16 ? 4 : 16;
     const int RS16 = gemv_rhs_stride((int)sizeof(T), Rmax);
-    const int wpc = warp_level ? warp_stream_warps_per_cta() : 1;
+    const int wpc = warp_stream_warps_per_cta();
     const int nt = (int)tasks.size();
-    const int cta = std::max(1, std::min((nt + wpc - 1) / wpc, launch_ctas(omax, transposed, warp_level, map)));
+    const int cta = std::max(1, std::min((nt + wpc - 1) / wpc, launch_ctas(omax, map)));
     *ncta = cta;
     const int G = cta * wpc;
     std::vector<double> cost(tasks.size());
@@ -1922,8 +1919,6 @@ class Engine : public EngineBase {
   // window (2 rows per lane) up to 32 rows, half-warp row groups up to 64, lanes over rows
   // up to 128 (4 rows per lane).
   static void warp_shape(GemvLaunch& L, int omax) {
-    L.warp_level = true;
-    L.ol = 32;
     if (std::is_same<T, float>::value) {
       // FP32: tensor-core tiles of 8 output rows (map 3, rpt = row tiles held per warp: exactly
       // those of the tallest task up to 8, else 16)
@@ -1939,18 +1934,11 @@ class Engine : public EngineBase {
     L.rpt = omax <= 32 ? 2 : 4;
   }
 
-  // With `begin` given (one range of tasks per warp, or per CTA, of the full persistent grid),
-  // the ranges are taken as they are instead of being cut by cost here.
+  // With `begin` given (one range of tasks per warp, or per CTA for map 4, of the full persistent
+  // grid), the ranges are taken as they are instead of being cut by cost here.
   void finish_launch(GemvLaunch& L, SideBuf& sb, int slot, std::vector<GemvTask>& tasks,
-                     const std::vector<GemvUnit>& units, int ol, int rpt, bool transposed, bool out_is_y,
-                     const std::vector<int>* begin_given = nullptr) {
+                     const std::vector<GemvUnit>& units, const std::vector<int>* begin_given = nullptr) {
     L.ntasks = (int)tasks.size();
-    if (!L.warp_level) {
-      L.ol = ol;
-      L.rpt = rpt;
-    }
-    L.transposed = transposed;
-    L.out_is_y = out_is_y;
     if (tasks.empty()) return;
     // X rows of every unit: contiguous, or at most kUnitRuns runs covering exactly c rows
     for (auto& t : tasks)
@@ -1961,19 +1949,16 @@ class Engine : public EngineBase {
           long long rows = 0;
           for (int r = 0; r < g.nruns; ++r) rows += g.run_len[r];
           if (rows != g.c) throw Error("gemv plan: unit runs do not cover its columns");
-          if (transposed) throw Error("gemv plan: runs of X rows in a transposed unit");  // read as one block
         }
       }
     // the kernel walks units sequentially across the tasks of a CTA
     for (size_t t = 1; t < tasks.size(); ++t)
       if (tasks[t].first_unit != tasks[t - 1].first_unit + tasks[t - 1].nunits)
         throw Error("gemv plan: units of a launch are not contiguous");
-    const int omax = L.map == 4       ? 128
-                     : L.warp_level ? (L.map == 3 ? 8 * L.rpt : (L.map == 2 ? 32 : (L.map == 1 || L.map == 5 ? 64 : 128)))
-                                    : ol * rpt;
+    const int omax = L.map == 4 ? 128 : (L.map == 3 ? 8 * L.rpt : (L.map == 2 ? 32 : (L.map == 1 || L.map == 5 ? 64 : 128)));
     for (auto& t : tasks)
       if (t.O > omax) throw Error("gemv plan: task taller than its launch shape");
-    if (L.warp_level) {
+    if (L.map != 4) {
       // every unit of the launch must fit one stage of the per-warp pipeline
       const int Rmax = sizeof(T) >= 16 ? 4 : 16;
       const long long xrow_bytes = (long long)gemv_rhs_stride((int)sizeof(T), Rmax) * sizeof(T);
@@ -1999,13 +1984,13 @@ class Engine : public EngineBase {
     }
     std::vector<int> begin;
     if (begin_given) {
-      const int wpc = L.warp_level ? warp_stream_warps_per_cta() : 1;
-      L.ncta = launch_ctas(omax, transposed, L.warp_level, L.map);
+      const int wpc = L.map != 4 ? warp_stream_warps_per_cta() : 1;
+      L.ncta = launch_ctas(omax, L.map);
       begin = *begin_given;
       if ((int)begin.size() != L.ncta * wpc + 1 || begin.front() != 0 || begin.back() != (int)tasks.size())
         throw Error("gemv plan: task ranges do not match the launch grid");
     } else {
-      begin = partition(tasks, units, omax, transposed, L.warp_level, L.map, &L.ncta);
+      begin = partition(tasks, units, omax, L.map, &L.ncta);
     }
     sb.tasks[slot].upload(tasks, stream_);
     sb.begin[slot].upload(begin, stream_);
@@ -2013,54 +1998,39 @@ class Engine : public EngineBase {
     L.cta_begin = sb.begin[slot].p;
   }
 
-  // Builds one side: 'N' (trans = false) or 'T' / 'C'.
-  void build_side(bool trans, const std::vector<GemvRkLeaf>& K, const std::vector<int>& rk_leaf,
-                  long long& next_row, GemvSide& side, SideBuf& sb) {
+  // The 'N' side.
+  void build_side(const std::vector<GemvRkLeaf>& K, const std::vector<int>& rk_leaf, long long& next_row,
+                  GemvSide& side, SideBuf& sb) {
     const auto& L = bt_->leaves;
-    const std::vector<Block>& oblocks = trans ? cblocks_ : rblocks_;
-    const std::vector<int>& ostarts = trans ? cstarts_ : rstarts_;
+    const std::vector<Block>& oblocks = rblocks_;
+    const std::vector<int>& ostarts = rstarts_;
     std::vector<GemvUnit> units;
-    // a longer z task is cut into chunks summed afterwards (spreads long leaves over warps): the
-    // 'N' chunk size is the gemv tuner's choice
-    const int kMaxUnits = trans ? 16 : tune_zparts_;
-    // FP32 'N' y-phase on the tensor-memory kernel when HMAT_B200_TC_Y=1
-    const bool tc_y = !trans && std::is_same<T, float>::value && tc_y_enabled();
+    // a longer z task is cut into chunks summed afterwards (spreads long groups over warps): the
+    // chunk size is the gemv tuner's choice
+    const int kMaxUnits = tune_zparts_;
+    // FP32 y-phase on the tensor-memory kernel when HMAT_B200_TC_Y=1
+    const bool tc_y = std::is_same<T, float>::value && tc_y_enabled();
 
-    // ---- z-phase: 'N' one task per B^T group (z = B^T x_J of its leaves at once, the x rows
-    // read once), 'T' one per Rk leaf (z' = A^T x_I over its A panels); long ones cut into
-    // chunks; one launch per height class ----
+    // ---- z-phase: one task per B^T group (z = B^T x_J of its leaves at once, the x rows read
+    // once); long ones cut into chunks; one launch per height class ----
     std::vector<GemvTask> zt[4];
     std::vector<GemvUnit> zunits[4];
     std::vector<GemvZred> zred;
     std::vector<GemvUnit> lu;
     const auto& G = layout_.zgroups;
-    const size_t nz = trans ? K.size() : G.size();
+    const size_t nz = G.size();
     for (size_t t = 0; t < nz; ++t) {
       lu.clear();
-      int O, zrow;
-      if (!trans) {
-        // the group's stacked B^T: h x n column-major
-        const ZGroup& g = G[t];
-        int xoff = 0;
-        const int zc = kTensorN ? mma_unit_cols(g.h, &xoff) : warp_unit_cols_wide(g.h, &xoff);
-        px_units(lu, g.base, g.h, g.n, g.col_off, zc, xoff);
-        O = g.h;
-        zrow = zgroup_row_[0][t];
-      } else {
-        const GemvRkLeaf& k = K[t];
-        const int leaf = rk_leaf[t];
-        // z' = A^T x_I: each A panel (len x k) is a transposed piece
-        auto br = block_range(rblocks_, rstarts_, k.row_off, k.m);
-        for (int b = br.first; b < br.second; ++b)
-          ptx_units(lu, layout_.panel[layout_.first[leaf] + (b - br.first)], rblocks_[b].len, k.k, 0,
-                    rblocks_[b].off);
-        O = k.k;
-        zrow = k.zrow_t;
-      }
+      // the group's stacked B^T: h x n column-major
+      const ZGroup& g = G[t];
+      int xoff = 0;
+      const int zc = kTensorN ? mma_unit_cols(g.h, &xoff) : warp_unit_cols_wide(g.h, &xoff);
+      px_units(lu, g.base, g.h, g.n, g.col_off, zc, xoff);
+      const int O = g.h, zrow = zgroup_row_[0][t];
       if (O > 128) throw Error("gemv plan: ranks above 128 are not supported by the streamed kernels");
-      // 'N' launches take every height up to 32 in one launch; the tensor-core kernel takes every
-      // height up to 64 in one (its tile count is a per-task constant), so one wave covers them
-      const int cls = trans ? rank_class(O) : (kTensorN && O <= 64 ? 2 : std::max(1, rank_class(O)));
+      // one launch takes every height up to 32; the tensor-core kernel takes every height up to 64
+      // in one (its tile count is a per-task constant), so one wave covers them
+      const int cls = kTensorN && O <= 64 ? 2 : std::max(1, rank_class(O));
       // units of one launch must be contiguous in task order: collect them per class
       std::vector<GemvUnit>& cu = zunits[cls];
       if ((int)lu.size() <= kMaxUnits) {
@@ -2073,7 +2043,7 @@ class Engine : public EngineBase {
         for (int pidx = 0; pidx < nparts; ++pidx) {
           const int u0 = pidx * kMaxUnits, u1 = std::min((int)lu.size(), u0 + kMaxUnits);
           GemvTask task{O, (int)cu.size(), u1 - u0, part_row + pidx * O};
-          if (zsum_in_kernel(trans)) task.red = (int)zred.size();
+          if (kZsumInKernel) task.red = (int)zred.size();
           zt[cls].push_back(task);
           cu.insert(cu.end(), lu.begin() + u0, lu.begin() + u1);
         }
@@ -2089,19 +2059,17 @@ class Engine : public EngineBase {
     std::vector<std::vector<int>> per_block(oblocks.size());  // leaves with storage covering each block
     for (int i = 0; i < (int)L.size(); ++i) {
       if (layout_.first[i] < 0) continue;
-      auto br = trans ? block_range(oblocks, ostarts, L[i].col_off, L[i].n)
-                      : block_range(oblocks, ostarts, L[i].row_off, L[i].m);
+      auto br = block_range(oblocks, ostarts, L[i].row_off, L[i].m);
       for (int b = br.first; b < br.second; ++b) per_block[b].push_back(i);
     }
     std::vector<int> rk_index(L.size(), -1);
     for (size_t t = 0; t < rk_leaf.size(); ++t) rk_index[rk_leaf[t]] = (int)t;
     std::vector<GemvTask> yt;
-    std::vector<int> ybegin;  // 'N': the warps' task ranges, cut here by cost
+    std::vector<int> ybegin;  // the warps' task ranges, cut here by cost
     int maxlen = 1;
     for (const Block& ob : oblocks) maxlen = std::max(maxlen, ob.len);
-    const ClusterTree* otree = trans ? C_ : R_;
-    std::vector<int2> yrows(otree->n, int2{0, 0});
-    if (!trans) {
+    std::vector<int2> yrows(R_->n, int2{0, 0});
+    {
       // Each output block's matrix (the y region of the arena) in units of whole columns; the X
       // rows of its columns are the leaves' x rows (full) and z rows (Rk), merged into runs where
       // adjacent, and the zero rows for the padding columns.
@@ -2177,7 +2145,7 @@ class Engine : public EngineBase {
       if (tc_y) probe.map = 4;
       else warp_shape(probe, maxlen);
       const int wpc = probe.map == 4 ? 1 : warp_stream_warps_per_cta();
-      const int G = launch_ctas(probe.map == 3 ? 8 * probe.rpt : maxlen, false, probe.map != 4, probe.map) * wpc;
+      const int G = launch_ctas(probe.map == 3 ? 8 * probe.rpt : maxlen, probe.map) * wpc;
       const int nyu = (int)units.size() - first_y;
       std::vector<double> cum(nyu + 1, 0.0);
       for (int v = 0; v < nyu; ++v) {
@@ -2216,46 +2184,7 @@ class Engine : public EngineBase {
       for (size_t b = 0; b < oblocks.size(); ++b) {
         const Block& ob = oblocks[b];
         for (int l = 0; l < ob.len; ++l)
-          yrows[otree->perm[ob.off + l]] = int2{part_row[b] + l, (nparts[b] << 8) | ob.len};
-      }
-    } else {
-      // each output block is cut into chunks of at most kYChunkUnits units whose partial rows go
-      // to xz; a final pass sums them into y (client order).  The chunks spread the blocks with
-      // many leaves over the grid.  The Rk terms come per B^T group: the block's columns of the
-      // group's matrix times the group's z' rows.
-      const int kYChunkUnits = 16;
-      std::vector<std::vector<int>> groups_of(oblocks.size());
-      for (size_t gi = 0; gi < G.size(); ++gi) {
-        auto br = block_range(oblocks, ostarts, G[gi].col_off, G[gi].n);
-        for (int b = br.first; b < br.second; ++b) groups_of[b].push_back((int)gi);
-      }
-      for (size_t b = 0; b < oblocks.size(); ++b) {
-        const Block& ob = oblocks[b];
-        const int first = (int)units.size();
-        for (int i : per_block[b]) {
-          const LeafInfo& l = L[i];
-          if (l.type != 0) continue;
-          // columns of block b in every row panel of full leaf i
-          auto br = block_range(rblocks_, rstarts_, l.row_off, l.m);
-          for (int q = br.first; q < br.second; ++q) {
-            const int len = rblocks_[q].len;
-            ptx_units(units, layout_.panel[layout_.first[i] + (q - br.first)] + (long long)(ob.off - l.col_off) * len,
-                      len, ob.len, 0, rblocks_[q].off);
-          }
-        }
-        for (int gi : groups_of[b]) {
-          const ZGroup& g = G[gi];
-          ptx_units(units, g.base + (long long)(ob.off - g.col_off) * g.h, g.h, ob.len, 0, zgroup_row_[1][gi]);
-        }
-        const int nu = (int)units.size() - first;
-        const int nparts = (nu + kYChunkUnits - 1) / kYChunkUnits;
-        const int part_row = (int)next_row;
-        next_row += (long long)nparts * ob.len;
-        for (int pidx = 0; pidx < nparts; ++pidx) {
-          const int u0 = pidx * kYChunkUnits, u1 = std::min(nu, u0 + kYChunkUnits);
-          yt.push_back(GemvTask{ob.len, first + u0, u1 - u0, part_row + pidx * ob.len});
-        }
-        for (int l = 0; l < ob.len; ++l) yrows[otree->perm[ob.off + l]] = int2{part_row + l, (nparts << 8) | ob.len};
+          yrows[R_->perm[ob.off + l]] = int2{part_row[b] + l, (nparts[b] << 8) | ob.len};
       }
     }
     // launches
@@ -2263,31 +2192,26 @@ class Engine : public EngineBase {
     static const int kClassMax[4] = {16, 32, 64, 128};
     for (int c = 0; c < 4; ++c) {
       if (zt[c].empty()) continue;
-      int ol, rpt;
-      class_shape(c, ol, rpt);
       GemvLaunch& L = side.z[side.nz];
       L = GemvLaunch();
-      if (!trans) {
-        int om = 1;  // the class's tallest task (FP32 launches hold exactly its tiles)
-        for (const GemvTask& t : zt[c]) om = std::max(om, t.O);
-        warp_shape(L, kTensorN ? om : kClassMax[c]);
-      }
-      finish_launch(L, sb, side.nz, zt[c], units, ol, rpt, trans, false);
+      int om = 1;  // the class's tallest task (FP32 launches hold exactly its tiles)
+      for (const GemvTask& t : zt[c]) om = std::max(om, t.O);
+      warp_shape(L, kTensorN ? om : kClassMax[c]);
+      finish_launch(L, sb, side.nz, zt[c], units);
       side.nz++;
     }
-    const int rpt = maxlen <= 32 ? 1 : (maxlen <= 64 ? 2 : 4);
     side.y = GemvLaunch();
     if (tc_y)
       side.y.map = 4;
-    else if (!trans)
+    else
       warp_shape(side.y, maxlen);
-    finish_launch(side.y, sb, GemvSide::kMaxLaunch, yt, units, 32, rpt, trans, false, trans ? nullptr : &ybegin);
+    finish_launch(side.y, sb, GemvSide::kMaxLaunch, yt, units, &ybegin);
     sb.units.upload(units, stream_);
     side.units = sb.units.p;
     sb.zred.upload(zred, stream_);
     side.nzred = (int)zred.size();
     side.zred = sb.zred.p;
-    side.zfused = zsum_in_kernel(trans);
+    side.zfused = kZsumInKernel;
     sb.zcnt.alloc((size_t)std::max<size_t>(zred.size(), 1));
     HB_CUDA(cudaMemsetAsync(sb.zcnt.p, 0, sb.zcnt.n * sizeof(int), stream_));
     side.zcnt = sb.zcnt.p;
@@ -2295,6 +2219,241 @@ class Engine : public EngineBase {
     side.nyrows = (int)yrows.size();
     side.yrows = sb.yrows.p;
   }
+
+  // Cuts the units [first, first + owner.size()) (owner: the output each belongs to, equal ones
+  // adjacent) into tasks: one range of about equal cost per member of a grid of G, split where
+  // the owner changes.  begin[g] is the first task of member g; task_owner the owner of each.
+  static void cut_tasks(const std::vector<GemvTransUnit>& units, int first, const std::vector<int>& owner, int G,
+                        std::vector<GemvTask>& tasks, std::vector<int>& task_owner, std::vector<int>& begin) {
+    const int n = (int)owner.size();
+    std::vector<double> cum(n + 1, 0.0);
+    for (int v = 0; v < n; ++v) cum[v + 1] = cum[v] + (double)units[first + v].rows * units[first + v].cols + 256;
+    const double tot = std::max(cum[n], 1.0);
+    begin.assign(G + 1, 0);
+    int w = 0;
+    for (int v = 0; v < n;) {
+      while (w + 1 < G && cum[v] >= tot * (w + 1) / G) begin[++w] = (int)tasks.size();
+      const double wend = w + 1 < G ? tot * (w + 1) / G : 1e300;
+      int v1 = v + 1;
+      while (v1 < n && owner[v1] == owner[v] && cum[v1] < wend) ++v1;
+      tasks.push_back(GemvTask{0, first + v, v1 - v, 0});
+      task_owner.push_back(owner[v]);
+      v = v1;
+    }
+    for (++w; w <= G; ++w) begin[w] = (int)tasks.size();
+  }
+
+  void upload_launch(GemvLaunch& L, SideBuf& sb, int slot, const std::vector<GemvTask>& tasks,
+                     const std::vector<int>& begin) {
+    L.ntasks = (int)tasks.size();
+    sb.tasks[slot].upload(tasks, stream_);
+    sb.begin[slot].upload(begin, stream_);
+    L.tasks = sb.tasks[slot].p;
+    L.cta_begin = sb.begin[slot].p;
+  }
+
+  // The 'T' / 'C' side: the column pass over the output blocks' matrices, the sums of the z' parts
+  // of leaves over several blocks, the group pass over the B^T groups, the final sum.
+  void build_trans_side(const std::vector<GemvRkLeaf>& K, const std::vector<int>& rk_leaf, long long& next_row,
+                        GemvSide& side, SideBuf& sb) {
+    const auto& L = bt_->leaves;
+    const auto& G = layout_.zgroups;
+    const int s = (int)sizeof(T);
+    const int CL = trans_lanes(s), CW = trans_cols(s);
+    const int RS16 = gemv_rhs_stride(s, s >= 16 ? 4 : 16);
+    std::vector<GemvTransUnit> units;
+
+    // the rows of y: the column blocks cut into strips of at most CW columns, CL-wide but the last
+    std::vector<Block> strips;
+    std::vector<int> strip_of(C_->n);
+    for (const Block& cb : cblocks_) {
+      const int groups = (cb.len + CL - 1) / CL, n = (groups + CW / CL - 1) / (CW / CL);
+      for (int i = 0, g0 = 0; i < n; ++i) {
+        const int g1 = (int)((long long)groups * (i + 1) / n);
+        const int o = cb.off + g0 * CL, len = std::min(cb.len, g1 * CL) - g0 * CL;
+        for (int j = 0; j < len; ++j) strip_of[o + j] = (int)strips.size();
+        strips.push_back(Block{o, len});
+        g0 = g1;
+      }
+    }
+
+    // ---- group pass: the strips' columns of every B^T group, groups of up to CW rows in one
+    // launch (small stages, more CTAs), taller ones (one leaf of higher rank) in another ----
+    std::vector<std::vector<int>> groups_of(cblocks_.size());
+    for (size_t gi = 0; gi < G.size(); ++gi) {
+      auto br = block_range(cblocks_, cstarts_, G[gi].col_off, G[gi].n);
+      for (int b = br.first; b < br.second; ++b) groups_of[b].push_back((int)gi);
+    }
+    std::vector<int> nparts(strips.size(), 0);
+    std::vector<GemvTask> gt[2];
+    std::vector<int> gstrip[2], gbegin[2];
+    side.ng = 0;
+    for (int cls = 0; cls < 2; ++cls) {
+      const int first = (int)units.size();
+      std::vector<int> owner;
+      int piece = 16, hmax = 1;
+      for (size_t b = 0, st = 0; b < cblocks_.size(); ++b) {
+        const int cend = cblocks_[b].off + cblocks_[b].len;
+        for (; st < strips.size() && strips[st].off < cend; ++st)
+          for (int gi : groups_of[b]) {
+            const ZGroup& g = G[gi];
+            if ((g.h > 32) != (cls == 1)) continue;
+            if (g.h > 128) throw Error("gemv plan: ranks above 128 are not supported by the streamed kernels");
+            // columns of a unit: the strip's, or as many CL-wide groups as keep the piece small
+            const int most = std::max(1, kTransPieceBytes / (g.h * s * CL)) * CL;
+            for (int j0 = 0; j0 < strips[st].len; j0 += most) {
+              GemvTransUnit u{};
+              u.poff = g.base + (long long)(strips[st].off - g.col_off + j0) * g.h;
+              u.x = zgroup_row_[1][gi];
+              u.rows = (unsigned char)g.h;
+              u.o0 = (unsigned char)j0;
+              u.cols = (unsigned char)std::min(most, strips[st].len - j0);
+              units.push_back(u);
+              owner.push_back((int)st);
+              piece = std::max(piece, (int)((u.rows * u.cols + u.poff % kPad) * s + 15) / 16 * 16);
+              hmax = std::max(hmax, g.h);
+            }
+          }
+      }
+      if (owner.empty()) continue;
+      GemvLaunch& l = side.g[side.ng];
+      l = GemvLaunch();
+      l.piece_bytes = piece;
+      l.xrows = hmax;
+      l.ncta = trans_ctas(trans_groups_smem(piece, hmax, RS16 * s));
+      const int wpc = trans_warps_per_cta();
+      l.ncta = std::max(1, std::min(l.ncta, ((int)owner.size() + wpc - 1) / wpc));
+      cut_tasks(units, first, owner, l.ncta * wpc, gt[side.ng], gstrip[side.ng], gbegin[side.ng]);
+      for (int st : gstrip[side.ng]) nparts[st]++;
+      side.ng++;
+    }
+
+    // ---- the parts of y: a full leaf gives a strip one part per row block it covers ----
+    std::vector<int> fullparts(strips.size(), 0);
+    for (int i = 0; i < (int)L.size(); ++i) {
+      if (layout_.first[i] < 0 || L[i].type != 0) continue;
+      auto br = block_range(rblocks_, rstarts_, L[i].row_off, L[i].m);
+      const int last = strip_of[L[i].col_off + L[i].n - 1];
+      for (int st = strip_of[L[i].col_off]; st <= last; ++st) fullparts[st] += br.second - br.first;
+    }
+    std::vector<int> part_row(strips.size(), 0), taken(strips.size(), 0);
+    std::vector<int2> yrows(C_->n, int2{0, 0});
+    for (size_t st = 0; st < strips.size(); ++st) {
+      const int np = fullparts[st] + nparts[st];
+      part_row[st] = (int)next_row;
+      next_row += (long long)np * strips[st].len;
+      for (int l = 0; l < strips[st].len; ++l)
+        yrows[C_->perm[strips[st].off + l]] = int2{part_row[st] + l, (np << 8) | strips[st].len};
+    }
+    for (int c = 0; c < side.ng; ++c)
+      for (size_t t = 0; t < gt[c].size(); ++t) {
+        const int st = gstrip[c][t];
+        gt[c][t].O = strips[st].len;
+        gt[c][t].out_row = part_row[st] + (fullparts[st] + taken[st]++) * strips[st].len;
+      }
+    std::fill(taken.begin(), taken.end(), 0);
+
+    // ---- column pass: the destination row of every column of every output block's matrix (the
+    // block's columns at colbase, a multiple of 8), then its units of whole columns ----
+    std::vector<long long> colbase(rblocks_.size() + 1, 0);
+    for (size_t b = 0; b < rblocks_.size(); ++b) colbase[b + 1] = colbase[b] + layout_.ywidth[b];
+    if (colbase.back() >= (1LL << 31)) throw Error("gemv plan: too many columns");
+    std::vector<int> colmap((size_t)colbase.back() + 4, 0), used(rblocks_.size(), 0);
+    std::vector<GemvZred> zred;
+    std::vector<int> rk_index(L.size(), -1);
+    for (size_t t = 0; t < rk_leaf.size(); ++t) rk_index[rk_leaf[t]] = (int)t;
+    for (int i = 0; i < (int)L.size(); ++i) {
+      if (layout_.first[i] < 0) continue;
+      auto br = block_range(rblocks_, rstarts_, L[i].row_off, L[i].m);
+      const int nb = br.second - br.first, w = L[i].type == 0 ? L[i].n : ranks[i];
+      int zrow = 0;
+      if (L[i].type != 0) {
+        const GemvRkLeaf& k = K[rk_index[i]];
+        zrow = k.zrow_t;
+        if (nb > 1) {  // parts, one per row block, summed into the leaf's z' rows
+          zred.push_back(GemvZred{zrow, w, (int)next_row, nb});
+          zrow = (int)next_row;
+          next_row += (long long)nb * w;
+        }
+      }
+      for (int b = br.first; b < br.second; ++b) {
+        int* m = &colmap[(size_t)colbase[b] + layout_.pcol[layout_.first[i] + (b - br.first)]];
+        used[b] += w;
+        if (L[i].type != 0) {
+          for (int j = 0; j < w; ++j) m[j] = zrow + (b - br.first) * w + j;
+          continue;
+        }
+        for (int j = 0; j < w;) {
+          const int c = L[i].col_off + j, st = strip_of[c], e = std::min(w - j, strips[st].off + strips[st].len - c);
+          const int row = part_row[st] + taken[st]++ * strips[st].len + (c - strips[st].off);
+          for (int q = 0; q < e; ++q) m[j + q] = row + q;
+          j += e;
+        }
+      }
+    }
+    // the longest sums first: they take a CTA each
+    std::stable_sort(zred.begin(), zred.end(), [](const GemvZred& x, const GemvZred& y) { return x.nparts > y.nparts; });
+    side.nzwide = 0;
+    while (side.nzwide < (int)zred.size() && zred[side.nzwide].nparts > kZredWideParts) side.nzwide++;
+    const int first = (int)units.size();
+    std::vector<int> owner;
+    int stage = 32, omax = 1;
+    for (size_t b = 0; b < rblocks_.size(); ++b) {
+      const int O = rblocks_[b].len;
+      // CW columns where the piece stays small, twice that for short blocks, else as many CL-wide
+      // groups as fit
+      int cols = std::max(1, kTransPieceBytes / (O * s * CL)) * CL;
+      cols = cols >= 2 * CW && O * s * 2 * CW <= kTransPieceBytes / 2 ? 2 * CW : std::min(cols, CW);
+      for (int j0 = 0; j0 < used[b]; j0 += cols) {
+        GemvTransUnit u{};
+        u.poff = layout_.yblock[b] + (long long)j0 * O;
+        u.x = (int)(colbase[b] + j0);
+        u.rows = (unsigned char)O;
+        u.cols = (unsigned char)std::min(cols, used[b] - j0);
+        if (u.poff % kPad) throw Error("gemv plan: misaligned block piece");
+        units.push_back(u);
+        owner.push_back((int)b);
+        stage = std::max(stage, (O * u.cols * s + 15) / 16 * 16 + (u.cols * 4 + 15) / 16 * 16);
+        omax = std::max(omax, O);
+      }
+    }
+    side.nz = 0;
+    if (!owner.empty()) {
+      GemvLaunch& l = side.z[0];
+      l = GemvLaunch();
+      l.piece_bytes = stage;
+      l.xrows = omax;
+      // x rows padded by 16 bytes where the kernel pads them
+      l.ncta = trans_ctas(trans_columns_smem(stage, omax, RS16 * s + 16));
+      const int wpc = trans_warps_per_cta();
+      l.ncta = std::max(1, std::min(l.ncta, ((int)owner.size() + wpc - 1) / wpc));
+      std::vector<GemvTask> ct;
+      std::vector<int> cblock, cbegin;
+      cut_tasks(units, first, owner, l.ncta, ct, cblock, cbegin);
+      for (size_t t = 0; t < ct.size(); ++t) {
+        ct[t].O = rblocks_[cblock[t]].len;
+        ct[t].out_row = rblocks_[cblock[t]].off;  // the block's x rows
+      }
+      upload_launch(l, sb, 0, ct, cbegin);
+      side.nz = 1;
+    }
+    for (int c = 0; c < side.ng; ++c) upload_launch(side.g[c], sb, GemvSide::kMaxLaunch + c, gt[c], gbegin[c]);
+    for (int m : colmap)
+      if (m < 0 || m >= next_row) throw Error("gemv plan: column map out of range");
+    sb.tunits.upload(units, stream_);
+    side.tunits = sb.tunits.p;
+    sb.colmap.upload(colmap, stream_);
+    side.colmap = sb.colmap.p;
+    sb.zred.upload(zred, stream_);
+    side.nzred = (int)zred.size();
+    side.zred = sb.zred.p;
+    side.zfused = false;
+    sb.yrows.upload(yrows, stream_);
+    side.nyrows = (int)yrows.size();
+    side.yrows = sb.yrows.p;
+  }
+  // Sums of z' parts above this many take a CTA of eight warps instead of one warp.
+  static constexpr int kZredWideParts = 16;
 
   void build_plan() {
     const auto& L = bt_->leaves;
@@ -2306,7 +2465,6 @@ class Engine : public EngineBase {
     plan_.n_rows = R_->n;
     plan_.n_cols = C_->n;
     plan_.n_in_max = std::max(R_->n, C_->n);
-    long long next_row = plan_.n_in_max + kZeroRows;
     for (size_t i = 0; i < L.size(); ++i) {
       if (L[i].type == 0 && layout_.first[i] >= 0) {
         F.push_back(GemvFullLeaf{L[i].row_off, L[i].m, L[i].col_off, L[i].n, goff});
@@ -2318,21 +2476,24 @@ class Engine : public EngineBase {
         rk_leaf.push_back((int)i);
       }
     }
-    // z slots ('N', then 'T') in the order of the B^T groups: a group's z rows are contiguous
+    // z slots in the order of the B^T groups: a group's z rows are contiguous ('N' and 'T' each
+    // in their own numbering)
     std::vector<int> kidx(L.size(), -1);
     for (size_t t = 0; t < rk_leaf.size(); ++t) kidx[rk_leaf[t]] = (int)t;
     const auto& G = layout_.zgroups;
-    zgroup_row_[0].assign(G.size(), 0);
-    zgroup_row_[1].assign(G.size(), 0);
-    for (int side = 0; side < 2; ++side)
+    long long next_row[2];
+    for (int side = 0; side < 2; ++side) {
+      next_row[side] = plan_.n_in_max + kZeroRows;
+      zgroup_row_[side].assign(G.size(), 0);
       for (size_t gi = 0; gi < G.size(); ++gi) {
-        zgroup_row_[side][gi] = (int)next_row;
+        zgroup_row_[side][gi] = (int)next_row[side];
         for (int i : G[gi].leaves) {
           GemvRkLeaf& k = K[kidx[i]];
-          (side == 0 ? k.zrow_n : k.zrow_t) = (int)next_row;
-          next_row += k.k;
+          (side == 0 ? k.zrow_n : k.zrow_t) = (int)next_row[side];
+          next_row[side] += k.k;
         }
       }
+    }
     if (!d_perm_rows_.p || !d_perm_cols_.p) throw Error("gemv plan: cluster permutations are not on the device");
     plan_.perm_rows = d_perm_rows_.p;
     plan_.perm_cols = d_perm_cols_.p;
@@ -2352,10 +2513,43 @@ class Engine : public EngineBase {
     plan_.rk = g_rk_.p;
     plan_.nfull = (int)F.size();
     plan_.nrk = (int)K.size();
-    build_side(false, K, rk_leaf, next_row, plan_.side[0], side_buf_[0]);
-    build_side(true, K, rk_leaf, next_row, plan_.side[1], side_buf_[1]);
-    plan_.xz_rows = next_row;
-    if (next_row >= (1LL << 31)) throw Error("gemv plan: z buffer too large");
+    build_side(K, rk_leaf, next_row[0], plan_.side[0], side_buf_[0]);
+    build_trans_side(K, rk_leaf, next_row[1], plan_.side[1], side_buf_[1]);
+    for (int side = 0; side < 2; ++side) {
+      plan_.xz_rows[side] = next_row[side];
+      if (next_row[side] >= (1LL << 31)) throw Error("gemv plan: z buffer too large");
+    }
+    noalloc_rows_ = next_row[0] + noalloc_trans_rows(K);
+  }
+
+  // The bound of the allocation-free products is stated in rows of one buffer for both
+  // directions, with the partial rows of transposed products that took a slot per 16 units of 32
+  // columns: callers know which matrices it takes, so it stays, although a transposed product now
+  // uses its scratch differently (gemv_device_with_scratch).
+  long long noalloc_trans_rows(const std::vector<GemvRkLeaf>& K) const {
+    const auto& L = bt_->leaves;
+    const long long kUnits = 16;
+    auto strips32 = [](long long w) { return (w + 31) / 32; };
+    long long rows = 0;
+    for (const GemvRkLeaf& k : K) {
+      rows += k.k;
+      auto br = block_range(rblocks_, rstarts_, k.row_off, k.m);
+      const long long nu = (br.second - br.first) * strips32(k.k);
+      if (nu > kUnits) rows += (nu + kUnits - 1) / kUnits * k.k;
+    }
+    std::vector<long long> nu(cblocks_.size(), 0);
+    for (int i = 0; i < (int)L.size(); ++i) {
+      if (L[i].type != 0 || layout_.first[i] < 0) continue;
+      auto rb = block_range(rblocks_, rstarts_, L[i].row_off, L[i].m);
+      auto cb = block_range(cblocks_, cstarts_, L[i].col_off, L[i].n);
+      for (int b = cb.first; b < cb.second; ++b) nu[b] += (rb.second - rb.first) * strips32(cblocks_[b].len);
+    }
+    for (const ZGroup& g : layout_.zgroups) {
+      auto cb = block_range(cblocks_, cstarts_, g.col_off, g.n);
+      for (int b = cb.first; b < cb.second; ++b) nu[b] += strips32(cblocks_[b].len);
+    }
+    for (size_t b = 0; b < cblocks_.size(); ++b) rows += (nu[b] + kUnits - 1) / kUnits * cblocks_[b].len;
+    return rows;
   }
 
   // Gemv tuner.  Two knobs of the 'N' schedule: the size of the chunks long z tasks are cut into
@@ -2382,7 +2576,7 @@ class Engine : public EngineBase {
     xb.alloc((size_t)C_->n * nr);
     yb.alloc((size_t)R_->n * nr);
     HB_CUDA(cudaMemsetAsync(xb.p, 0, xb.n * sizeof(T), stream_));
-    xz_.ensure(xz_elems());
+    xz_.ensure(xz_elems(0));
     GemvTiming tm;
     for (int i = 0; i < 4; ++i) HB_CUDA(cudaEventCreate(&tm.ev[i]));
     for (int rep = 0; rep < 2; ++rep)
@@ -2492,7 +2686,8 @@ class Engine : public EngineBase {
   SideBuf side_buf_[2];
   std::vector<int> zgroup_row_[2];  // first z row of each B^T group, 'N' and 'T' 
   GemvPlan plan_;
-  DevArray<T> xz_, rz_, stage_x_, stage_y_;
+  long long noalloc_rows_ = 0;
+  DevArray<T> xz_, rz_, stage_x_, stage_y_;  // scratch of 'N' and of 'T' products, host staging
   DevArray<GemvStatus> err_;       // status block of this matrix's products (flag, wait bound)
   GemvStatus* h_err_ = nullptr;    // pinned host copy
   cudaGraphExec_t gexec_ = nullptr;

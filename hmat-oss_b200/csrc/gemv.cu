@@ -6,17 +6,20 @@
 // c_wrapping.hpp:233-252), as a few launches over device-resident schedules (gemv_plan.h):
 //
 //   gather   xz[i][q] = x[perm[i] + q ld]           client -> cluster order, row-major
-//   z-phase  z_L = B_L^T x_J ('N') / A_L^T x_I ('T')  one task per Rk leaf (chunks for long ones)
-//   z-reduce sums the chunk partials of long leaves
-//   y-phase  y_I = beta y_I + alpha sum (F x | A z)   one task per output block; the result is
-//                                                     scattered straight to client order
+//   'N': z-phase  z = B^T x_J, one task per group of Rk leaves with one column range (chunks for
+//                 long ones, summed afterwards)
+//        y-phase  partial rows of sum (F x | A z), the output blocks' matrices streamed
+//   'T': column pass  every column of every output block's matrix times the block's x rows: the
+//                 full leaves' share of y and the z' = A^T x parts of the Rk leaves
+//        z'-sum   the parts of leaves over several blocks
+//        group pass  partial rows of sum B z' per output block, over the B^T groups
+//   final    y = beta y + alpha sum of a row's parts, in client order
 //
 // Every task streams its units (contiguous pieces of the leaf arena and of the xz buffer)
-// through a shared-memory pipeline filled by TMA bulk copies (cp.async.bulk, completion on
-// an mbarrier), on a persistent grid where each CTA owns a contiguous range of tasks of
-// about equal bytes.  Each thread accumulates up to 4 output rows x R right-hand sides in
-// registers; inner-dimension slices (warps, and lanes when the output is narrow) are summed
-// at the end of each task in a fixed order, so repeated products are bitwise identical.
+// through per-warp shared-memory pipelines filled by TMA bulk copies (cp.async.bulk, completion
+// on an mbarrier), on a persistent grid cut into ranges of about equal bytes.  Sums run in a
+// fixed order, so repeated products are bitwise identical.
+#include <cstring>
 #include <type_traits>
 
 #include "gemv_plan.h"
@@ -25,12 +28,6 @@
 namespace hmatb200 {
 size_t warp_stream_smem_bytes(int elem_bytes);
 namespace {
-
-constexpr int kThreads = 128;
-constexpr int kWarps = kThreads / 32;
-constexpr int kPieceCols = 32;         // inner extent of a non-transposed unit
-constexpr int kPieceElems = 128 * 32;  // P capacity of a stage (elements)
-constexpr int kMaxInner = 128;         // inner extent of a transposed unit
 
 // ---------------------------------------------------------------------------------
 // TMA bulk copy + mbarrier helpers
@@ -153,10 +150,6 @@ template <typename T>
 constexpr int rs_of(int R) {
   return R * (int)sizeof(T) >= 16 ? R : (16 / (int)sizeof(T));
 }
-template <typename T>
-constexpr int nstage_of() {
-  return sizeof(T) >= 16 ? 2 : 3;
-}
 
 // ---------------------------------------------------------------------------------
 // x (client order, column-major with leading dimension ldx; right-hand sides q0 .. q0 + R - 1
@@ -270,158 +263,6 @@ __device__ inline void issue_x(unsigned char* dst, const T* xz, const GemvUnit& 
       bulk_xrows(dst + off, xz + (size_t)U.run_row[r] * RS, b, bar);
       off += b;
     }
-  }
-}
-
-// ---------------------------------------------------------------------------------
-// The streamed task kernel.  OL output lanes x (32 / OL) inner slices per warp, RPT rows per
-// lane (output rows <= OL * RPT), R right-hand sides (xz row stride RS).
-template <typename T, int R, int RS, int OL, int RPT, bool TRANSP, int NSTAGE>
-__global__ void __launch_bounds__(kThreads) stream_kernel(const GemvTask* __restrict__ tasks,
-                                                          const int* __restrict__ cta_begin,
-                                                          const GemvUnit* __restrict__ units,
-                                                          const T* __restrict__ arena, T* xz, int conj,
-                                                          int out_is_y, const int* __restrict__ perm_out,
-                                                          T* __restrict__ y, int ldy, int q0, int r, T alpha,
-                                                          T beta, GemvStatus* err) {
-  constexpr int LS = 32 / OL;
-  constexpr int OMAX = OL * RPT;
-  constexpr int XCAP = (TRANSP ? kMaxInner : kPieceCols) * RS;
-  constexpr int PCAP = kPieceElems + 2 * OMAX + 16;  // slack: alignment shift, masked lanes reading past a piece
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  T* Ps = reinterpret_cast<T*>(smem_raw);
-  T* Xs = Ps + (size_t)NSTAGE * PCAP;
-  T* red = Xs + (size_t)NSTAGE * XCAP;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(red + (size_t)kWarps * OMAX * R);
-
-  const int t0 = cta_begin[blockIdx.x], t1 = cta_begin[blockIdx.x + 1];
-  if (t0 >= t1) return;
-  const int u_begin = tasks[t0].first_unit;
-  const int u_end = tasks[t1 - 1].first_unit + tasks[t1 - 1].nunits;
-  const long long wlim = err->wait_limit;
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ol = lane % OL, ls = lane / OL;
-
-  if (tid == 0) {
-    for (int s = 0; s < NSTAGE; ++s) mbar_init(&bars[s], 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-  // producer: thread 0 arms a stage's barrier and issues the unit's two bulk copies
-  auto issue = [&](int u) {
-    const int s = (u - u_begin) % NSTAGE;
-    const GemvUnit U = units[u];
-    // the copy starts at the 16-byte boundary at or below the piece (TMA alignment rule)
-    const uint32_t pbytes = round16((uint64_t)(U.pel + U.shift) * sizeof(T));
-    const uint32_t xbytes = (uint32_t)U.c * RS * (uint32_t)sizeof(T);
-    mbar_expect_tx(&bars[s], pbytes + xbytes);
-    bulk_piece(Ps + (size_t)s * PCAP, arena + (U.poff - U.shift), pbytes, &bars[s]);
-    bulk_xrows(Xs + (size_t)s * XCAP, xz + (size_t)U.xrow * RS, xbytes, &bars[s]);
-  };
-  if (tid == 0)
-    for (int u = u_begin; u < u_end && u < u_begin + NSTAGE; ++u) issue(u);
-
-  int u = u_begin;
-  for (int t = t0; t < t1; ++t) {
-    const GemvTask task = tasks[t];
-    T acc[RPT][R];
-#pragma unroll
-    for (int a = 0; a < RPT; ++a)
-#pragma unroll
-      for (int q = 0; q < R; ++q) acc[a][q] = zero<T>();
-
-    for (int k = 0; k < task.nunits; ++k, ++u) {
-      const int s = (u - u_begin) % NSTAGE;
-      const uint32_t parity = (uint32_t)(((u - u_begin) / NSTAGE) & 1);
-      const bool ok = mbar_wait_bounded(&bars[s], parity, wlim);
-      const GemvUnit U = units[u];
-      const T* P = Ps + (size_t)s * PCAP + U.shift;
-      const T* X = Xs + (size_t)s * XCAP;
-      const int c = U.c;
-      if constexpr (!TRANSP) {
-        // P is O x c column-major: out[o] += sum_j P[o, j] X[j]
-        const int O = task.O;
-#pragma unroll 2
-        for (int j = warp * LS + ls; j < c; j += kWarps * LS) {
-          T xv[R];
-          lds_vec<T, R>(X + (size_t)j * RS, xv);
-#pragma unroll
-          for (int a = 0; a < RPT; ++a) {
-            const T p = P[ol + a * OL + (size_t)j * O];
-#pragma unroll
-            for (int q = 0; q < R; ++q) acc[a][q] = fmadd(p, xv[q], acc[a][q]);
-          }
-        }
-      } else {
-        // P is c x ow column-major, covering outputs [o0, o0 + ow):
-        // out[o] += sum_j op(P[j, o - o0]) X[j]
-        const int o0 = U.o0, ow = U.ow;
-        for (int j = warp * LS + ls; j < c; j += kWarps * LS) {
-          T xv[R];
-          lds_vec<T, R>(X + (size_t)j * RS, xv);
-#pragma unroll
-          for (int a = 0; a < RPT; ++a) {
-            const int oo = ol + a * OL - o0;
-            if (oo >= 0 && oo < ow) {
-              T p = P[j + (size_t)oo * c];
-              if (conj) p = conjg(p);
-#pragma unroll
-              for (int q = 0; q < R; ++q) acc[a][q] = fmadd(p, xv[q], acc[a][q]);
-            }
-          }
-        }
-      }
-      // stage s is free again; a copy that did not land in time stops the whole CTA, after
-      // the copies it has in flight (units u .. u + NSTAGE - 1) have landed
-      if (__syncthreads_or(!ok)) {
-        if (tid == 0) {
-          atomicCAS(&err->failed, 0, 1);
-          for (int v = u; v < u_end && v < u + NSTAGE; ++v)
-            mbar_wait_bounded(&bars[(v - u_begin) % NSTAGE], (uint32_t)(((v - u_begin) / NSTAGE) & 1),
-                              drain_limit(err));
-        }
-        return;
-      }
-      if (tid == 0 && u + NSTAGE < u_end) issue(u + NSTAGE);
-    }
-
-    // ---- epilogue: lane slices, then warps, in a fixed order ----
-#pragma unroll
-    for (int m = OL; m < 32; m <<= 1)
-#pragma unroll
-      for (int a = 0; a < RPT; ++a)
-#pragma unroll
-        for (int q = 0; q < R; ++q) acc[a][q] = acc[a][q] + shfl_xor(acc[a][q], m);
-    if (ls == 0) {
-#pragma unroll
-      for (int a = 0; a < RPT; ++a)
-#pragma unroll
-        for (int q = 0; q < R; ++q) red[((size_t)warp * OMAX + ol + a * OL) * R + q] = acc[a][q];
-    }
-    __syncthreads();
-    for (int e = tid; e < task.O * R; e += kThreads) {
-      const int o = e / R, q = e % R;
-      T v = red[(size_t)o * R + q];
-#pragma unroll
-      for (int w = 1; w < kWarps; ++w) v = v + red[((size_t)w * OMAX + o) * R + q];
-      if (out_is_y) {
-        if (q0 + q < r) {
-          T* yp = y + (size_t)perm_out[task.out_row + o] + (size_t)(q0 + q) * ldy;
-          T outv = alpha * v;
-          if (!is_zero_val(beta)) outv = fmadd(beta, *yp, outv);
-          *yp = outv;
-        }
-      } else {
-        xz[(size_t)(task.out_row + o) * RS + q] = v;
-      }
-    }
-    if constexpr (RS > R) {
-      if (!out_is_y)
-        for (int e = tid; e < task.O * (RS - R); e += kThreads)
-          xz[(size_t)(task.out_row + e / (RS - R)) * RS + R + e % (RS - R)] = zero<T>();
-    }
-    __syncthreads();
   }
 }
 
@@ -960,6 +801,329 @@ __global__ void __launch_bounds__(kWarpCTA * 32, mma_min_blocks(NTILE, sizeof(T)
 }
 
 // ---------------------------------------------------------------------------------
+// Transposed products ('T' / 'C'), every type: out[col] += sum_i op(P[i, col]) X[i] for
+// column-major pieces P.  A warp holds CL x CP columns, lane = slice * CL + cl: column cl + CL a
+// (a < CP) in its registers for all R right-hand sides, rows slice, slice + SL, ... of the piece.
+// Each X row it loads serves CP columns, and each P scalar R multiply-adds, so at 16 right-hand
+// sides the FMAs bound it (FP32: 32 paired FMAs per 4 scalars of P and 4 loads of X a lane); the
+// slices are joined by a shuffle exchange that leaves each lane a share of the sums.
+//
+// Products that ran a CTA per task, with a block barrier per unit and one column a lane, took
+// (device time, before -> now): cylinder of 50,001 points, FP32, 16 right-hand sides 753 -> 192 us
+// (1.9 TB/s); of 60,000 points, FP64, 11 right-hand sides 1,948 -> 384 us (2.4 TB/s); 12 covariance
+// matrices, FP32, one right-hand side 906 -> 159 us (3.9 TB/s); Helmholtz cylinder of 50,000
+// points, complex FP32, four 1,794 -> 300 us (3.6 TB/s).  FP32 stays on CUDA cores: its sums are
+// chains of a few FMAs a slice, more accurate than the split TF32 products of the 'N' kernels.
+
+// acc[a] += sum over this lane's rows of P[i, cols[a]] X[i], a in [A0, A0 + NA).
+template <typename T, int R, int CP, int A0, int NA, int SL>
+__device__ __forceinline__ void trans_rows(const T* P, int O, int c, int cl, int CL, const T* X, int xs, int sl,
+                                           bool conj, typename RowOps<T, R>::AV (&acc)[CP]) {
+  using Ops = RowOps<T, R>;
+  const T* p[NA];
+#pragma unroll
+  for (int a = 0; a < NA; ++a) p[a] = P + (size_t)min(cl + CL * a, c - 1) * O;  // past the piece: not written
+#pragma unroll 2
+  for (int i = sl; i < O; i += SL) {
+    typename Ops::XV xv;
+    Ops::load(X + (size_t)i * xs, xv);
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+      T v = p[a][i];
+      if constexpr (Traits<T>::is_complex) {
+        if (conj) v = conjg(v);
+      }
+      Ops::fma(v, xv, acc[A0 + a]);
+    }
+  }
+}
+// The number of columns groups (na of CP from group a0) as a compile-time constant.
+template <typename T, int R, int CP, int SL, int A0 = 0, int NA = 1>
+__device__ __forceinline__ void trans_dispatch(int a0, int na, const T* P, int O, int c, int cl, int CL, const T* X,
+                                               int xs, int sl, bool conj, typename RowOps<T, R>::AV (&acc)[CP]) {
+  if (a0 == A0 && na == NA) {
+    trans_rows<T, R, CP, A0, NA, SL>(P, O, c, cl, CL, X, xs, sl, conj, acc);
+    return;
+  }
+  if constexpr (A0 + NA < CP) {
+    trans_dispatch<T, R, CP, SL, A0, NA + 1>(a0, na, P, O, c, cl, CL, X, xs, sl, conj, acc);
+  } else if constexpr (A0 + 1 < CP) {
+    trans_dispatch<T, R, CP, SL, A0 + 1, 1>(a0, na, P, O, c, cl, CL, X, xs, sl, conj, acc);
+  }
+}
+
+// Sums v over the lanes that differ in the slice bits (M = 16 down to CL), in exchanges that
+// halve what each lane keeps: afterwards the lane holds the sums of values off .. off + (what is
+// left) - 1; `mine` is false on lanes holding a copy of another lane's.
+__host__ __device__ constexpr int trans_left(int V, int CL) {
+  for (int m = 16; m >= CL; m >>= 1)
+    if (V % 2 == 0) V /= 2;
+  return V;
+}
+template <typename T, int CL, int N, int V, int M>
+__device__ __forceinline__ void slice_sum(T (&v)[N], int lane, int& off, bool& mine) {
+  if constexpr (M >= CL) {
+    if constexpr (V % 2 == 0) {
+      constexpr int H = V / 2;
+      const bool hi = (lane & M) != 0;
+#pragma unroll
+      for (int i = 0; i < H; ++i) {
+        const T send = hi ? v[i] : v[i + H];
+        const T keep = hi ? v[i + H] : v[i];
+        v[i] = keep + shfl_xor(send, M);
+      }
+      off += hi ? H : 0;
+      slice_sum<T, CL, N, H, M / 2>(v, lane, off, mine);
+    } else {
+#pragma unroll
+      for (int i = 0; i < V; ++i) v[i] = v[i] + shfl_xor(v[i], M);
+      mine = mine && (lane & M) == 0;
+      slice_sum<T, CL, N, V, M / 2>(v, lane, off, mine);
+    }
+  }
+}
+template <typename T, int Q>
+__device__ inline void stg_vec(T* p, const T* v) {
+  constexpr int bytes = Q * (int)sizeof(T);
+  if constexpr (bytes % 16 == 0) {
+#pragma unroll
+    for (int c = 0; c < bytes / 16; ++c) reinterpret_cast<uint4*>(p)[c] = reinterpret_cast<const uint4*>(v)[c];
+  } else {
+#pragma unroll
+    for (int c = 0; c < Q; ++c) p[c] = v[c];
+  }
+}
+
+constexpr int kTransWarps = 4;
+constexpr int kTransStages = 2;
+__device__ inline GemvTransUnit load_unit(const GemvTransUnit* p) {
+  const int4 w = __ldg(reinterpret_cast<const int4*>(p));
+  GemvTransUnit u;
+  memcpy(&u, &w, sizeof(u));
+  return u;
+}
+
+// Row stride (scalars) of the x rows the column pass keeps in shared memory: padded by 16 bytes
+// where the slices' rows would otherwise share banks.
+template <typename T, int RS>
+__host__ __device__ constexpr int trans_xstride() {
+  return (RS * (int)sizeof(T)) % 64 == 0 ? RS + 16 / (int)sizeof(T) : RS;
+}
+
+// Column pass: a task is a part of an output block's matrix (O rows, the block's x rows at
+// out_row), a unit up to 64 whole columns of it; column j of a unit is written to the xz row
+// colmap[unit.xrow + j].  The four warps of a CTA share the block's x rows (staged once a task)
+// and take its units in turn, each through its own two-stage ring.
+template <typename T, int R, int RS>
+__global__ void __launch_bounds__(kTransWarps * 32, (trans_ctas_per_sm((int)sizeof(T))))
+    trans_columns_kernel(const GemvTask* __restrict__ tasks, const int* __restrict__ cta_begin,
+                         const GemvTransUnit* __restrict__ units, const int* __restrict__ colmap,
+                         const T* __restrict__ arena, T* xz, int conj, int stage_bytes, int xrows, GemvStatus* err) {
+  using Ops = RowOps<T, R>;
+  constexpr int CL = trans_column_lanes((int)sizeof(T), R), CW = trans_cols((int)sizeof(T)), CP = CW / CL, SL = 32 / CL;
+  constexpr int XS = trans_xstride<T, RS>();
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  pdl_wait();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int cl = lane % CL, sl = lane / CL;
+  T* X = reinterpret_cast<T*>(smem_raw);
+  unsigned char* wbase = smem_raw + (size_t)xrows * XS * sizeof(T) + (size_t)warp * kTransStages * stage_bytes;
+  unsigned char* tail = smem_raw + (size_t)xrows * XS * sizeof(T) + (size_t)kTransWarps * kTransStages * stage_bytes;
+  int2* uslot = reinterpret_cast<int2*>(tail) + warp * kTransStages;  // a unit's columns, offset of its map
+  uint64_t* bars = reinterpret_cast<uint64_t*>(tail + kTransWarps * kTransStages * sizeof(int2)) + warp * kTransStages;
+  const int t0 = cta_begin[blockIdx.x], t1 = cta_begin[blockIdx.x + 1];
+  if (t0 >= t1) return;
+  const int u_begin = tasks[t0].first_unit + warp;
+  const int u_end = tasks[t1 - 1].first_unit + tasks[t1 - 1].nunits;
+  const long long wlim = err->wait_limit;
+  if (lane == 0) {
+    for (int s = 0; s < kTransStages; ++s) mbar_init(&bars[s], 1);
+    mbar_fence_init();
+  }
+  __syncwarp();
+  GemvTransUnit nxt{};  // lane 0: the next unit to issue, loaded one issue ahead
+  int issued = 0;       // lane 0: units issued so far (unit i of the warp is u_begin + i kTransWarps)
+  auto issue = [&](const GemvTransUnit& U, int v) {
+    const int s = issued % kTransStages;
+    ++issued;
+    const uint32_t pbytes = round16((uint64_t)U.rows * U.cols * sizeof(T)), mbytes = round16((uint64_t)U.cols * sizeof(int));
+    unsigned char* st = wbase + (size_t)s * stage_bytes;
+    if (U.cols == 0 || U.rows == 0 || pbytes + mbytes > (uint32_t)stage_bytes ||
+        (reinterpret_cast<uintptr_t>(arena + U.poff) & 15) != 0 || (U.x & 3) != 0) {
+      record_bad_unit(err, v);
+      uslot[s] = make_int2(0, 0);
+      mbar_arrive(&bars[s]);
+      return;
+    }
+    uslot[s] = make_int2(U.cols, (int)pbytes);
+    mbar_expect_tx(&bars[s], pbytes + mbytes);
+    bulk_piece(st, arena + U.poff, pbytes, &bars[s]);
+    bulk_piece(st + pbytes, colmap + U.x, mbytes, &bars[s]);
+  };
+  if (lane == 0)
+    for (int k = 0, v = u_begin; k < kTransStages && v < u_end; ++k, v += kTransWarps) issue(load_unit(units + v), v);
+  int vnext = u_begin + kTransStages * kTransWarps;  // the next unit to issue
+  if (lane == 0 && vnext < u_end) nxt = load_unit(units + vnext);
+
+  bool dead = false;  // a wait gave up: the warp only keeps the CTA's barriers company
+  int u = u_begin, done = 0;
+  for (int t = t0; t < t1; ++t) {
+    const GemvTask task = tasks[t];
+    const int O = task.O;
+    __syncthreads();  // the previous task's x rows are read
+    {
+      constexpr int V = 16 / (int)sizeof(T);  // scalars a 16-byte chunk
+      constexpr int RC = RS / V;              // chunks a row
+      const uint4* src = reinterpret_cast<const uint4*>(xz + (size_t)task.out_row * RS);
+      for (int e = tid; e < O * RC; e += kTransWarps * 32)
+        *reinterpret_cast<uint4*>(X + (size_t)(e / RC) * XS + (size_t)(e % RC) * V) = src[e];
+    }
+    __syncthreads();
+    const int task_end = task.first_unit + task.nunits;
+    for (; u < task_end; u += kTransWarps, ++done) {
+      if (dead) continue;
+      const int s = done % kTransStages;
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bars[s], (uint32_t)((done / kTransStages) & 1), wlim))) {
+        if (lane == 0) {
+          atomicCAS(&err->failed, 0, 1);
+          for (int v = done; v < issued; ++v)
+            mbar_wait_bounded(&bars[v % kTransStages], (uint32_t)((v / kTransStages) & 1), drain_limit(err));
+        }
+        __syncwarp();
+        dead = true;
+        continue;
+      }
+      const int c = uslot[s].x;
+      const T* P = reinterpret_cast<const T*>(wbase + (size_t)s * stage_bytes);
+      const int* map = reinterpret_cast<const int*>(wbase + (size_t)s * stage_bytes + uslot[s].y);
+      for (int c0 = 0; c0 < c; c0 += CW) {
+        typename Ops::AV acc[CP];
+#pragma unroll
+        for (int a = 0; a < CP; ++a) Ops::zero_(acc[a]);
+        const int left = c - c0;
+        trans_dispatch<T, R, CP, SL>(0, min(CP, (left + CL - 1) / CL), P + (size_t)c0 * O, O, left, cl, CL, X, XS, sl,
+                                     conj != 0, acc);
+        constexpr int V = CP * R, VF = trans_left(V, CL);
+        T v[V];
+#pragma unroll
+        for (int a = 0; a < CP; ++a)
+#pragma unroll
+          for (int q = 0; q < R; ++q) v[a * R + q] = Ops::get(acc[a], q);
+        int off = 0;
+        bool mine = true;
+        slice_sum<T, CL, V, V, 16>(v, lane, off, mine);
+        const int col = cl + CL * (off / R);
+        if (mine && col < left) stg_vec<T, VF>(xz + (size_t)map[c0 + col] * RS + off % R, v);
+      }
+      __syncwarp();  // every lane is done with stage s
+      if (vnext < u_end) {
+        if (lane == 0) {
+          issue(nxt, vnext);
+          if (vnext + kTransWarps < u_end) nxt = load_unit(units + vnext + kTransWarps);
+        }
+        vnext += kTransWarps;
+      }
+    }
+  }
+}
+
+// Group pass: a task is up to CL x CP columns (rows of y) of an output block, a unit the task's
+// columns of one B^T group (all of them, or some of the CL-wide groups from column o0 of a tall
+// one) with the group's z' rows; the warp keeps the task's sums in registers and writes them as
+// partial rows.  The piece starts `shift` scalars after a 16-byte boundary.
+template <typename T, int R, int RS>
+__global__ void __launch_bounds__(kTransWarps * 32, (trans_ctas_per_sm((int)sizeof(T))))
+    trans_groups_kernel(const GemvTask* __restrict__ tasks, const int* __restrict__ warp_begin,
+                        const GemvTransUnit* __restrict__ units, const T* __restrict__ arena, T* xz, int conj,
+                        int stage_bytes, GemvStatus* err) {
+  using Ops = RowOps<T, R>;
+  constexpr int CL = trans_lanes((int)sizeof(T)), CP = trans_cols((int)sizeof(T)) / CL, SL = 32 / CL;
+  constexpr int kAlign = 16 / (int)sizeof(T);  // scalars of a 16-byte step
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cl = lane % CL, sl = lane / CL;
+  unsigned char* wbase = smem_raw + (size_t)warp * kTransStages * stage_bytes;
+  unsigned char* tail = smem_raw + (size_t)kTransWarps * kTransStages * stage_bytes;
+  // a unit's rows, columns, first column group, and piece shift << 20 | X offset in 16-byte steps
+  int4* uslot = reinterpret_cast<int4*>(tail) + warp * kTransStages;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(tail + kTransWarps * kTransStages * sizeof(int4)) + warp * kTransStages;
+  const int gw = blockIdx.x * kTransWarps + warp;
+  const int t0 = warp_begin[gw], t1 = warp_begin[gw + 1];
+  if (t0 >= t1) return;
+  const int u_begin = tasks[t0].first_unit;
+  const int u_end = tasks[t1 - 1].first_unit + tasks[t1 - 1].nunits;
+  const long long wlim = err->wait_limit;
+  if (lane == 0) {
+    for (int s = 0; s < kTransStages; ++s) mbar_init(&bars[s], 1);
+    mbar_fence_init();
+  }
+  __syncwarp();
+  GemvTransUnit nxt{};  // lane 0: the next unit to issue, loaded one issue ahead
+  int last_issued = u_begin - 1;
+  auto issue = [&](const GemvTransUnit& U, int v) {
+    const int s = (v - u_begin) % kTransStages;
+    last_issued = v;
+    const int shift = (int)(U.poff % kAlign);  // the copy starts at the 16-byte boundary below
+    const uint32_t pbytes = round16((uint64_t)(U.rows * U.cols + shift) * sizeof(T));
+    const uint32_t xbytes = (uint32_t)U.rows * RS * (uint32_t)sizeof(T);
+    unsigned char* st = wbase + (size_t)s * stage_bytes;
+    const T* src = arena + (U.poff - shift);
+    if (U.rows == 0 || U.cols == 0 || U.o0 % CL != 0 || U.o0 + U.cols > CL * CP ||
+        pbytes + xbytes > (uint32_t)stage_bytes || (reinterpret_cast<uintptr_t>(src) & 15) != 0) {
+      record_bad_unit(err, v);
+      uslot[s] = make_int4(0, 1, 0, 0);
+      mbar_arrive(&bars[s]);
+      return;
+    }
+    uslot[s] = make_int4(U.rows, U.cols, U.o0 / CL, (shift << 20) | (int)(pbytes >> 4));
+    mbar_expect_tx(&bars[s], pbytes + xbytes);
+    bulk_piece(st, src, pbytes, &bars[s]);
+    bulk_xrows(st + pbytes, xz + (size_t)U.x * RS, xbytes, &bars[s]);
+  };
+  if (lane == 0) {
+    for (int v = u_begin; v < u_end && v < u_begin + kTransStages; ++v) issue(load_unit(units + v), v);
+    if (u_begin + kTransStages < u_end) nxt = load_unit(units + u_begin + kTransStages);
+  }
+
+  int u = u_begin;
+  for (int t = t0; t < t1; ++t) {
+    const GemvTask task = tasks[t];
+    typename Ops::AV acc[CP];
+#pragma unroll
+    for (int a = 0; a < CP; ++a) Ops::zero_(acc[a]);
+    for (int kk = 0; kk < task.nunits; ++kk, ++u) {
+      const int s = (u - u_begin) % kTransStages;
+      const uint32_t parity = (uint32_t)(((u - u_begin) / kTransStages) & 1);
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bars[s], parity, wlim))) {
+        if (lane == 0) warp_give_up(err, bars, kTransStages, u_begin, u, last_issued);
+        return;
+      }
+      const int4 w = uslot[s];
+      const T* P = reinterpret_cast<const T*>(wbase + (size_t)s * stage_bytes) + (w.w >> 20);
+      const T* X = reinterpret_cast<const T*>(wbase + (size_t)s * stage_bytes + (size_t)((w.w & 0xfffff) << 4));
+      trans_dispatch<T, R, CP, SL>(w.z, (w.y + CL - 1) / CL, P, w.x, w.y, cl, CL, X, RS, sl, conj != 0, acc);
+      __syncwarp();  // every lane is done with stage s
+      if (lane == 0 && u + kTransStages < u_end) {
+        issue(nxt, u + kTransStages);
+        if (u + kTransStages + 1 < u_end) nxt = load_unit(units + u + kTransStages + 1);
+      }
+    }
+    constexpr int V = CP * R, VF = trans_left(V, CL);
+    T v[V];
+#pragma unroll
+    for (int a = 0; a < CP; ++a)
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[a * R + q] = Ops::get(acc[a], q);
+    int off = 0;
+    bool mine = true;
+    slice_sum<T, CL, V, V, 16>(v, lane, off, mine);
+    const int col = cl + CL * (off / R);
+    if (mine && col < task.O) stg_vec<T, VF>(xz + (size_t)(task.out_row + col) * RS + off % R, v);
+  }
+}
+
+// ---------------------------------------------------------------------------------
 // FP32 'N' product on the 5th-generation tensor cores (tcgen05.mma, accumulators in tensor
 // memory), one task at a time per CTA of 128 threads; thread t owns output row t.
 //
@@ -1238,44 +1402,79 @@ __global__ void __launch_bounds__(256) yfinal_kernel(const int2* __restrict__ ro
   }
 }
 
-// Sums the chunk partials of long leaves: xz[final + l] = sum_p xz[part + p k + l], the parts
-// added in part order.  A warp per sum (kZredWarps sums a CTA), lanes over 16-byte chunks of
-// the k x RS slot (a row of RS scalars is a multiple of 16 bytes).
+// Sums partial slots: xz[final + l] = sum_p xz[part + p k + l].  A warp per sum (kZredWarps sums
+// a CTA), lanes over 16-byte chunks of the k x RS slot (a row of RS scalars is a multiple of 16
+// bytes), the parts added in part order; the first `nwide` sums take a CTA each, its warps an
+// eighth of the parts, joined in warp order (the z' of long leaves in the transposed products:
+// hundreds of parts, one warp's loads being a chain).
 constexpr int kZredWarps = 8;
+constexpr int kZredBatch = 8;  // parts loaded before they are added (loads in flight together)
 template <typename T, int RS>
-__global__ void __launch_bounds__(kZredWarps * 32) zred_kernel(const GemvZred* __restrict__ zr, int n, T* xz) {
+__device__ __forceinline__ void zred_parts(const T* part, int k, int c, int p0, int p1, T (&s)[sizeof(T) >= 16 ? 1 : 16 / sizeof(T)]) {
   constexpr int V = sizeof(T) >= 16 ? 1 : 16 / (int)sizeof(T);  // scalars a 16-byte chunk
+#pragma unroll
+  for (int e = 0; e < V; ++e) s[e] = zero<T>();
+  for (int b = p0; b < p1; b += kZredBatch) {
+    uint4 raw[kZredBatch];
+#pragma unroll
+    for (int i = 0; i < kZredBatch; ++i)
+      if (b + i < p1) raw[i] = *reinterpret_cast<const uint4*>(part + ((size_t)(b + i) * k * RS + (size_t)c * V));
+#pragma unroll
+    for (int i = 0; i < kZredBatch; ++i)
+      if (b + i < p1) {
+        const T* v = reinterpret_cast<const T*>(&raw[i]);
+#pragma unroll
+        for (int e = 0; e < V; ++e) s[e] = s[e] + v[e];
+      }
+  }
+}
+template <typename T, int RS>
+__global__ void __launch_bounds__(kZredWarps * 32) zred_kernel(const GemvZred* __restrict__ zr, int n, int nwide, T* xz) {
+  constexpr int V = sizeof(T) >= 16 ? 1 : 16 / (int)sizeof(T);
   static_assert((RS * sizeof(T)) % 16 == 0, "xz rows are 16-byte multiples");
+  __shared__ uint4 s_part[kZredWarps][32];
   pdl_wait();
-  const int w = blockIdx.x * kZredWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if ((int)blockIdx.x < nwide) {
+    const GemvZred d = zr[blockIdx.x];
+    const int nchunk = d.k * RS / V;
+    const T* part = xz + (size_t)d.part_row * RS;
+    T* fin = xz + (size_t)d.final_row * RS;
+    const int p0 = (int)((long long)d.nparts * warp / kZredWarps), p1 = (int)((long long)d.nparts * (warp + 1) / kZredWarps);
+    for (int c0 = 0; c0 < nchunk; c0 += 32) {
+      const int c = c0 + lane;
+      T s[V];
+      if (c < nchunk) {
+        zred_parts<T, RS>(part, d.k, c, p0, p1, s);
+        s_part[warp][lane] = *reinterpret_cast<const uint4*>(s);
+      }
+      __syncthreads();
+      if (warp == 0 && c < nchunk) {
+        for (int w = 1; w < kZredWarps; ++w) {
+          const uint4 raw = s_part[w][lane];
+          const T* v = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+          for (int e = 0; e < V; ++e) s[e] = s[e] + v[e];
+        }
+        *reinterpret_cast<uint4*>(fin + (size_t)c * V) = *reinterpret_cast<const uint4*>(s);
+      }
+      __syncthreads();
+    }
+    return;
+  }
+  const int w = nwide + ((int)blockIdx.x - nwide) * kZredWarps + warp;
   if (w >= n) return;
   const GemvZred d = zr[w];
   const int nchunk = d.k * RS / V;
   const T* part = xz + (size_t)d.part_row * RS;
   T* fin = xz + (size_t)d.final_row * RS;
-  constexpr int kBatch = 8;  // parts loaded before they are added (loads in flight together)
   for (int c = lane; c < nchunk; c += 32) {
     T s[V];
-#pragma unroll
-    for (int e = 0; e < V; ++e) s[e] = zero<T>();
-    for (int p0 = 0; p0 < d.nparts; p0 += kBatch) {
-      uint4 raw[kBatch];
-#pragma unroll
-      for (int i = 0; i < kBatch; ++i)
-        if (p0 + i < d.nparts)
-          raw[i] = *reinterpret_cast<const uint4*>(part + ((size_t)(p0 + i) * d.k * RS + (size_t)c * V));
-#pragma unroll
-      for (int i = 0; i < kBatch; ++i)
-        if (p0 + i < d.nparts) {
-          const T* v = reinterpret_cast<const T*>(&raw[i]);
-#pragma unroll
-          for (int e = 0; e < V; ++e) s[e] = s[e] + v[e];
-        }
-    }
+    zred_parts<T, RS>(part, d.k, c, 0, d.nparts, s);
     *reinterpret_cast<uint4*>(fin + (size_t)c * V) = *reinterpret_cast<const uint4*>(s);
   }
 }
-inline unsigned zred_grid(int n) { return (unsigned)((n + kZredWarps - 1) / kZredWarps); }
+inline unsigned zred_grid(int n, int nwide) { return (unsigned)(nwide + (n - nwide + kZredWarps - 1) / kZredWarps); }
 
 // A launch with programmatic stream serialization (see pdl_wait): the kernel must begin with
 // pdl_wait() before it reads what the kernel before it wrote.
@@ -1295,21 +1494,6 @@ void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cuda
 }
 
 // ---------------------------------------------------------------------------------
-template <typename T, int R, int RS, int OL, int RPT, bool TRANSP>
-void launch_stream_t(const GemvLaunch& L, const GemvUnit* units, const T* arena, T* xz, int conj,
-                     const int* perm_out, T* y, int ldy, int q0, int r, T alpha, T beta, GemvStatus* err, cudaStream_t s) {
-  constexpr int NSTAGE = nstage_of<T>();
-  auto kern = stream_kernel<T, R, RS, OL, RPT, TRANSP, NSTAGE>;
-  const size_t smem = stream_smem_bytes(sizeof(T), R, RS, OL * RPT, TRANSP);
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr = true;
-  }
-  kern<<<L.ncta, kThreads, smem, s>>>(L.tasks, L.cta_begin, units, arena, xz, conj, L.out_is_y ? 1 : 0, perm_out, y,
-                                       ldy, q0, r, alpha, beta, err);
-}
-
 template <typename T, int R, int RS, int MODE, int A2>
 void launch_warp_t(const GemvLaunch& L, const GemvUnit* units, const T* arena, T* xz, GemvStatus* err, cudaStream_t s,
                    const GemvZred* zred, int* zcnt) {
@@ -1338,36 +1522,29 @@ void launch_mma_t(const GemvLaunch& L, const GemvUnit* units, const T* arena, T*
              zcnt);
 }
 
-// zred / zcnt: the sums of the z chunks, done by the warp-level z kernels themselves
-// (z_chunk_done); null for the y launches and the CTA-level kernels.
-template <typename T, int R, int RS, bool TRANSP>
-void launch_stream(const GemvLaunch& L, const GemvUnit* units, const T* arena, T* xz, int conj, const int* perm_out,
-                   T* y, int ldy, int q0, int r, T alpha, T beta, GemvStatus* err, cudaStream_t s,
+// The 'N' launches.  zred / zcnt: the sums of the z chunks, done by the warp-level z kernels
+// themselves (z_chunk_done); null for the y launches.
+template <typename T, int R, int RS>
+void launch_stream(const GemvLaunch& L, const GemvUnit* units, const T* arena, T* xz, GemvStatus* err, cudaStream_t s,
                    const GemvZred* zred = nullptr, int* zcnt = nullptr) {
   if (L.ntasks <= 0) return;
-  if constexpr (std::is_same<T, float>::value && !TRANSP) {
+  if constexpr (std::is_same<T, float>::value) {
     if (L.map == 4) {
       launch_umma_t<RS>(L, units, arena, xz, err, s);
       return;
     }
-  }
-  if (L.warp_level) {
-    if constexpr (std::is_same<T, float>::value) {
-      if (L.map == 3) {  // rpt = 8-row tiles of the launch's tallest task (exact up to 8)
-        switch (L.rpt) {
-          case 1: launch_mma_t<T, R, RS, 1>(L, units, arena, xz, err, s, zred, zcnt); break;
-          case 2: launch_mma_t<T, R, RS, 2>(L, units, arena, xz, err, s, zred, zcnt); break;
-          case 3: launch_mma_t<T, R, RS, 3>(L, units, arena, xz, err, s, zred, zcnt); break;
-          case 4: launch_mma_t<T, R, RS, 4>(L, units, arena, xz, err, s, zred, zcnt); break;
-          case 5: launch_mma_t<T, R, RS, 5>(L, units, arena, xz, err, s, zred, zcnt); break;
-          case 6: launch_mma_t<T, R, RS, 6>(L, units, arena, xz, err, s, zred, zcnt); break;
-          case 7: launch_mma_t<T, R, RS, 7>(L, units, arena, xz, err, s, zred, zcnt); break;
-          case 8: launch_mma_t<T, R, RS, 8>(L, units, arena, xz, err, s, zred, zcnt); break;
-          default: launch_mma_t<T, R, RS, 16>(L, units, arena, xz, err, s, zred, zcnt); break;
-        }
-        return;
-      }
+    switch (L.rpt) {  // map 3: rpt = 8-row tiles of the launch's tallest task (exact up to 8)
+      case 1: launch_mma_t<T, R, RS, 1>(L, units, arena, xz, err, s, zred, zcnt); break;
+      case 2: launch_mma_t<T, R, RS, 2>(L, units, arena, xz, err, s, zred, zcnt); break;
+      case 3: launch_mma_t<T, R, RS, 3>(L, units, arena, xz, err, s, zred, zcnt); break;
+      case 4: launch_mma_t<T, R, RS, 4>(L, units, arena, xz, err, s, zred, zcnt); break;
+      case 5: launch_mma_t<T, R, RS, 5>(L, units, arena, xz, err, s, zred, zcnt); break;
+      case 6: launch_mma_t<T, R, RS, 6>(L, units, arena, xz, err, s, zred, zcnt); break;
+      case 7: launch_mma_t<T, R, RS, 7>(L, units, arena, xz, err, s, zred, zcnt); break;
+      case 8: launch_mma_t<T, R, RS, 8>(L, units, arena, xz, err, s, zred, zcnt); break;
+      default: launch_mma_t<T, R, RS, 16>(L, units, arena, xz, err, s, zred, zcnt); break;
     }
+  } else {
     if (L.map == 2)
       launch_warp_t<T, R, RS, 2, 2>(L, units, arena, xz, err, s, zred, zcnt);
     else if (L.map == 5)
@@ -1376,16 +1553,51 @@ void launch_stream(const GemvLaunch& L, const GemvUnit* units, const T* arena, T
       launch_warp_t<T, R, RS, 1, 4>(L, units, arena, xz, err, s, zred, zcnt);
     else
       launch_warp_t<T, R, RS, 0, 4>(L, units, arena, xz, err, s, zred, zcnt);
-    return;
   }
-  if (L.ol == 16)
-    launch_stream_t<T, R, RS, 16, 1, TRANSP>(L, units, arena, xz, conj, perm_out, y, ldy, q0, r, alpha, beta, err, s);
-  else if (L.rpt == 1)
-    launch_stream_t<T, R, RS, 32, 1, TRANSP>(L, units, arena, xz, conj, perm_out, y, ldy, q0, r, alpha, beta, err, s);
-  else if (L.rpt == 2)
-    launch_stream_t<T, R, RS, 32, 2, TRANSP>(L, units, arena, xz, conj, perm_out, y, ldy, q0, r, alpha, beta, err, s);
-  else
-    launch_stream_t<T, R, RS, 32, 4, TRANSP>(L, units, arena, xz, conj, perm_out, y, ldy, q0, r, alpha, beta, err, s);
+}
+
+template <typename F>
+void allow_smem(F kern, bool& done) {
+  if (done) return;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxCtaSmem);
+  done = true;
+}
+
+template <typename T, int RS>
+void launch_zred(const GemvSide& side, T* xz, cudaStream_t s) {
+  if (side.nzred > 0 && !side.zfused)
+    launch_pdl(zred_kernel<T, RS>, dim3(zred_grid(side.nzred, side.nzwide)), dim3(kZredWarps * 32), 0, s, side.zred,
+               side.nzred, side.nzwide, xz);
+}
+
+// The column pass of the transposed products and its z' sums: afterwards xz holds the z' rows of
+// every Rk leaf and the full leaves' partial rows of y.
+template <typename T, int R, int RS>
+void run_trans_columns(const GemvSide& side, const T* arena, T* xz, int conj, GemvStatus* err, cudaStream_t s) {
+  const GemvLaunch& L = side.z[0];
+  if (side.nz > 0 && L.ntasks > 0) {
+    auto kern = trans_columns_kernel<T, R, RS>;
+    static bool attr = false;
+    allow_smem(kern, attr);
+    launch_pdl(kern, dim3(L.ncta), dim3(kTransWarps * 32),
+               trans_columns_smem(L.piece_bytes, L.xrows, trans_xstride<T, RS>() * (int)sizeof(T)), s, L.tasks,
+               L.cta_begin, side.tunits, side.colmap, arena, xz, conj, L.piece_bytes, L.xrows, err);
+  }
+  launch_zred<T, RS>(side, xz, s);
+}
+
+template <typename T, int R, int RS>
+void run_trans_groups(const GemvSide& side, const T* arena, T* xz, int conj, GemvStatus* err, cudaStream_t s) {
+  for (int c = 0; c < side.ng; ++c) {
+    const GemvLaunch& L = side.g[c];
+    if (L.ntasks <= 0) continue;
+    auto kern = trans_groups_kernel<T, R, RS>;
+    static bool attr = false;
+    allow_smem(kern, attr);
+    launch_pdl(kern, dim3(L.ncta), dim3(kTransWarps * 32),
+               trans_groups_smem(L.piece_bytes, L.xrows, RS * (int)sizeof(T)), s, L.tasks, L.cta_begin, side.tunits,
+               arena, xz, conj, L.piece_bytes + L.xrows * RS * (int)sizeof(T), err);
+  }
 }
 
 template <typename T, int R, bool TRANSP>
@@ -1395,21 +1607,24 @@ void run_tile(const GemvPlan& p, int nrhs, int q0, T alpha, T beta, const T* x, 
   const GemvSide& side = p.side[TRANSP ? 1 : 0];
   const int n_in = TRANSP ? p.n_rows : p.n_cols;
   const int* iperm_in = TRANSP ? p.iperm_rows : p.iperm_cols;
-  const int* perm_out = TRANSP ? p.perm_cols : p.perm_rows;
   const int ld_in = n_in, ld_out = TRANSP ? p.n_cols : p.n_rows;
   const T* arena = (const T*)p.arena;
   if (tm) cudaEventRecord(tm->ev[0], s);
-  const GemvSide& sn = p.side[0];
-  gather_kernel<T, R, RS><<<gather_grid(n_in), 256, 0, s>>>(x, n_in, ld_in, q0, nrhs, iperm_in, xz, p.n_in_max, sn.zcnt,
-                                                            sn.zfused ? sn.nzred : 0);
+  gather_kernel<T, R, RS><<<gather_grid(n_in), 256, 0, s>>>(x, n_in, ld_in, q0, nrhs, iperm_in, xz, p.n_in_max,
+                                                            side.zcnt, side.zfused ? side.nzred : 0);
   if (tm) cudaEventRecord(tm->ev[1], s);
-  for (int c = 0; c < side.nz; ++c)
-    launch_stream<T, R, RS, TRANSP>(side.z[c], side.units, arena, xz, conj, nullptr, nullptr, 0, 0, 0, alpha, beta,
-                                    err, s, side.zfused ? side.zred : nullptr, side.zcnt);
-  if (side.nzred > 0 && !side.zfused) launch_pdl(zred_kernel<T, RS>, dim3(zred_grid(side.nzred)), dim3(kZredWarps * 32), 0, s, side.zred, side.nzred, xz);
+  if constexpr (TRANSP) {
+    run_trans_columns<T, R, RS>(side, arena, xz, conj, err, s);
+  } else {
+    for (int c = 0; c < side.nz; ++c)
+      launch_stream<T, R, RS>(side.z[c], side.units, arena, xz, err, s, side.zfused ? side.zred : nullptr, side.zcnt);
+    launch_zred<T, RS>(side, xz, s);
+  }
   if (tm) cudaEventRecord(tm->ev[2], s);
-  launch_stream<T, R, RS, TRANSP>(side.y, side.units, arena, xz, conj, perm_out, y, ld_out, q0, nrhs, alpha, beta,
-                                  err, s);
+  if constexpr (TRANSP)
+    run_trans_groups<T, R, RS>(side, arena, xz, conj, err, s);
+  else
+    launch_stream<T, R, RS>(side.y, side.units, arena, xz, err, s);
   if (side.nyrows > 0) {
     const unsigned nb = (unsigned)((side.nyrows + kFinalRows - 1) / kFinalRows);
     launch_pdl(yfinal_kernel<T, R, RS>, dim3(nb), dim3(256), 0, s, side.yrows, side.nyrows, xz, y, ld_out, q0, nrhs,
@@ -1418,17 +1633,29 @@ void run_tile(const GemvPlan& p, int nrhs, int q0, T alpha, T beta, const T* x, 
   if (tm) cudaEventRecord(tm->ev[3], s);
 }
 
+// Right-hand sides are taken in tiles of at most max_tile (16, 8, 4 or 1; complex double never
+// more than 4: its accumulators).
 template <typename T, bool TRANSP>
 void run_all(const GemvPlan& p, int nrhs, T alpha, T beta, const T* x, T* y, T* xz, int conj, GemvStatus* err,
-             cudaStream_t s, const GemvTiming* tm) {
-  // complex double keeps tiles of at most 4 right-hand sides (shared-memory budget)
+             cudaStream_t s, const GemvTiming* tm, int max_tile) {
   constexpr int maxR = sizeof(T) >= 16 ? 4 : 16;
-  for (int q0 = 0; q0 < nrhs; q0 += maxR) {
+  const int most = max_tile < maxR ? max_tile : maxR;
+  int tile;
+  for (int q0 = 0; q0 < nrhs; q0 += tile) {
     const int rem = nrhs - q0;
-    if (maxR == 16 && rem > 8) run_tile<T, (maxR >= 16 ? 16 : 4), TRANSP>(p, nrhs, q0, alpha, beta, x, y, xz, conj, err, s, tm);
-    else if (maxR == 16 && rem > 4) run_tile<T, (maxR >= 16 ? 8 : 4), TRANSP>(p, nrhs, q0, alpha, beta, x, y, xz, conj, err, s, tm);
-    else if (rem > 1) run_tile<T, 4, TRANSP>(p, nrhs, q0, alpha, beta, x, y, xz, conj, err, s, tm);
-    else run_tile<T, 1, TRANSP>(p, nrhs, q0, alpha, beta, x, y, xz, conj, err, s, tm);
+    tile = 1;
+    if (most >= 16 && rem > 8) {
+      tile = 16;
+      run_tile<T, (maxR >= 16 ? 16 : 4), TRANSP>(p, nrhs, q0, alpha, beta, x, y, xz, conj, err, s, tm);
+    } else if (most >= 8 && rem > 4) {
+      tile = 8;
+      run_tile<T, (maxR >= 16 ? 8 : 4), TRANSP>(p, nrhs, q0, alpha, beta, x, y, xz, conj, err, s, tm);
+    } else if (most >= 4 && rem > 1) {
+      tile = 4;
+      run_tile<T, 4, TRANSP>(p, nrhs, q0, alpha, beta, x, y, xz, conj, err, s, tm);
+    } else {
+      run_tile<T, 1, TRANSP>(p, nrhs, q0, alpha, beta, x, y, xz, conj, err, s, tm);
+    }
   }
 }
 
@@ -1494,31 +1721,36 @@ __global__ void grad_rk_kernel(const GemvRkLeaf* __restrict__ rk, int nrk, const
   }
 }
 
+// x in cluster order (columns) and z = B^T x, in xz.
 template <typename T, int R>
-void grads_tile(const GemvPlan& p, int nrhs, const T* x, const T* r, T* xz, T* rz, T* gfull, T* grk, bool accumulate,
-                GemvStatus* err, cudaStream_t s) {
+void forward_z(const GemvPlan& p, int nrhs, const T* x, T* xz, GemvStatus* err, cudaStream_t s) {
   constexpr int RS = rs_of<T>(R);
-  const T* arena = (const T*)p.arena;
-  // x in cluster order (columns) and z = B^T x
   const GemvSide& sn = p.side[0];
   gather_kernel<T, R, RS><<<gather_grid(p.n_cols), 256, 0, s>>>(x, p.n_cols, p.n_cols, 0, nrhs, p.iperm_cols, xz,
-                                                                   p.n_in_max, sn.zcnt, sn.zfused ? sn.nzred : 0);
+                                                                p.n_in_max, sn.zcnt, sn.zfused ? sn.nzred : 0);
   for (int c = 0; c < sn.nz; ++c)
-    launch_stream<T, R, RS, false>(sn.z[c], sn.units, arena, xz, 0, nullptr, nullptr, 0, 0, 0, one<T>(), zero<T>(),
-                                   err, s, sn.zfused ? sn.zred : nullptr, sn.zcnt);
-  if (sn.nzred > 0 && !sn.zfused) launch_pdl(zred_kernel<T, RS>, dim3(zred_grid(sn.nzred)), dim3(kZredWarps * 32), 0, s, sn.zred, sn.nzred, xz);
-  // r in cluster order (rows) and w = A^T r
-  gather_kernel<T, R, RS><<<gather_grid(p.n_rows), 256, 0, s>>>(r, p.n_rows, p.n_rows, 0, nrhs, p.iperm_rows, rz,
-                                                                   p.n_in_max, sn.zcnt, sn.zfused ? sn.nzred : 0);
-  const GemvSide& st = p.side[1];
-  for (int c = 0; c < st.nz; ++c)
-    launch_stream<T, R, RS, true>(st.z[c], st.units, arena, rz, 0, nullptr, nullptr, 0, 0, 0, one<T>(), zero<T>(),
-                                  err, s);
-  if (st.nzred > 0) launch_pdl(zred_kernel<T, RS>, dim3(zred_grid(st.nzred)), dim3(kZredWarps * 32), 0, s, st.zred, st.nzred, rz);
+    launch_stream<T, R, RS>(sn.z[c], sn.units, (const T*)p.arena, xz, err, s, sn.zfused ? sn.zred : nullptr, sn.zcnt);
+  launch_zred<T, RS>(sn, xz, s);
+}
+template <typename T, int R>
+void grads_outer(const GemvPlan& p, const T* xz, const T* rz, T* gfull, T* grk, bool accumulate, cudaStream_t s) {
+  constexpr int RS = rs_of<T>(R);
   const int grid = persistent_grid(4);
   if (p.nfull > 0 && gfull)
     grad_full_kernel<T, RS, R><<<grid, 256, 0, s>>>(p.full, p.nfull, xz, rz, gfull, accumulate);
   if (p.nrk > 0 && grk) grad_rk_kernel<T, RS, R><<<grid, 256, 0, s>>>(p.rk, p.nrk, xz, rz, grk, accumulate);
+}
+
+template <typename T, int R>
+void grads_tile(const GemvPlan& p, int nrhs, const T* x, const T* r, T* xz, T* rz, T* gfull, T* grk, bool accumulate,
+                GemvStatus* err, cudaStream_t s) {
+  constexpr int RS = rs_of<T>(R);
+  forward_z<T, R>(p, nrhs, x, xz, err, s);
+  // r in cluster order (rows) and w = A^T r
+  gather_kernel<T, R, RS><<<gather_grid(p.n_rows), 256, 0, s>>>(r, p.n_rows, p.n_rows, 0, nrhs, p.iperm_rows, rz,
+                                                                p.n_in_max, nullptr, 0);
+  run_trans_columns<T, R, RS>(p.side[1], (const T*)p.arena, rz, 0, err, s);
+  grads_outer<T, R>(p, xz, rz, gfull, grk, accumulate, s);
 }
 
 // The adjoint of y = H x at the output gradient r in one pass: dx = H^T r (the 'T' product,
@@ -1527,30 +1759,21 @@ void grads_tile(const GemvPlan& p, int nrhs, const T* x, const T* r, T* xz, T* r
 template <typename T, int R>
 void adjoint_tile(const GemvPlan& p, int nrhs, const T* x, const T* r, T* dx, T* xz, T* rz, T* gfull, T* grk,
                   bool accumulate, GemvStatus* err, cudaStream_t s) {
-  constexpr int RS = rs_of<T>(R);
-  const T* arena = (const T*)p.arena;
   run_tile<T, R, true>(p, nrhs, 0, one<T>(), zero<T>(), r, dx, rz, 0, err, s, nullptr);
-  const GemvSide& sn = p.side[0];
-  gather_kernel<T, R, RS><<<gather_grid(p.n_cols), 256, 0, s>>>(x, p.n_cols, p.n_cols, 0, nrhs, p.iperm_cols, xz,
-                                                                   p.n_in_max, sn.zcnt, sn.zfused ? sn.nzred : 0);
-  for (int c = 0; c < sn.nz; ++c)
-    launch_stream<T, R, RS, false>(sn.z[c], sn.units, arena, xz, 0, nullptr, nullptr, 0, 0, 0, one<T>(), zero<T>(),
-                                   err, s, sn.zfused ? sn.zred : nullptr, sn.zcnt);
-  if (sn.nzred > 0 && !sn.zfused) launch_pdl(zred_kernel<T, RS>, dim3(zred_grid(sn.nzred)), dim3(kZredWarps * 32), 0, s, sn.zred, sn.nzred, xz);
-  const int grid = persistent_grid(4);
-  if (p.nfull > 0 && gfull)
-    grad_full_kernel<T, RS, R><<<grid, 256, 0, s>>>(p.full, p.nfull, xz, rz, gfull, accumulate);
-  if (p.nrk > 0 && grk) grad_rk_kernel<T, RS, R><<<grid, 256, 0, s>>>(p.rk, p.nrk, xz, rz, grk, accumulate);
+  forward_z<T, R>(p, nrhs, x, xz, err, s);
+  grads_outer<T, R>(p, xz, rz, gfull, grk, accumulate, s);
 }
 
 }  // namespace
 
-size_t stream_smem_bytes(int elem_bytes, int R, int RS, int omax, bool transposed) {
-  const int nstage = elem_bytes >= 16 ? 2 : 3;
-  const size_t xcap = (size_t)(transposed ? kMaxInner : kPieceCols) * RS;
-  const size_t pcap = (size_t)kPieceElems + 2 * omax + 16;
-  return (size_t)nstage * (pcap + xcap) * elem_bytes + (size_t)kWarps * omax * R * elem_bytes + nstage * 8 + 16;
+size_t trans_columns_smem(int stage_bytes, int xrows, int xrow_bytes) {
+  return (size_t)xrows * xrow_bytes + (size_t)kTransWarps * kTransStages * (stage_bytes + sizeof(int2) + sizeof(uint64_t));
 }
+size_t trans_groups_smem(int piece_bytes, int xrows, int xrow_bytes) {
+  return (size_t)kTransWarps * kTransStages *
+         ((size_t)piece_bytes + (size_t)xrows * xrow_bytes + sizeof(int4) + sizeof(uint64_t));
+}
+int trans_warps_per_cta() { return kTransWarps; }
 
 int gemv_rhs_stride(int elem_bytes, int R) { return R * elem_bytes >= 16 ? R : 16 / elem_bytes; }
 
@@ -1571,6 +1794,7 @@ int gemv_launch_count(const GemvPlan& p, char trans, int nrhs, int elem_bytes) {
   for (int c = 0; c < side.nz; ++c) per_tile += side.z[c].ntasks > 0;
   per_tile += side.nzred > 0 && !side.zfused;
   per_tile += side.y.ntasks > 0;
+  for (int c = 0; c < side.ng; ++c) per_tile += side.g[c].ntasks > 0;
   per_tile += side.nyrows > 0;  // final pass
   const int maxR = elem_bytes >= 16 ? 4 : 16;
   return per_tile * ((nrhs + maxR - 1) / maxR);
@@ -1598,16 +1822,16 @@ void launch_gemv_adjoint(const GemvPlan& p, int nrhs, const T* x, const T* r, T*
 
 template <typename T>
 void launch_gemv(const GemvPlan& p, char trans, int nrhs, T alpha, T beta, const T* x_client, T* y_client, T* xz,
-                 GemvStatus* err, cudaStream_t s, const GemvTiming* tm) {
-  if (trans == 'N') run_all<T, false>(p, nrhs, alpha, beta, x_client, y_client, xz, 0, err, s, tm);
+                 GemvStatus* err, cudaStream_t s, const GemvTiming* tm, int max_tile) {
+  if (trans == 'N') run_all<T, false>(p, nrhs, alpha, beta, x_client, y_client, xz, 0, err, s, tm, max_tile);
   else
     run_all<T, true>(p, nrhs, alpha, beta, x_client, y_client, xz, (trans == 'C' && Traits<T>::is_complex) ? 1 : 0,
-                     err, s, tm);
+                     err, s, tm, max_tile);
 }
 
 #define HB_INST(T)                                                                                            \
   template void launch_gemv<T>(const GemvPlan&, char, int, T, T, const T*, T*, T*, GemvStatus*, cudaStream_t,         \
-                               const GemvTiming*);                                                             \
+                               const GemvTiming*, int);                                                             \
   template void launch_leaf_gradients<T>(const GemvPlan&, int, const T*, const T*, T*, T*, T*, T*, bool, GemvStatus*, \
                                          cudaStream_t);                                                                  \
   template void launch_gemv_adjoint<T>(const GemvPlan&, int, const T*, const T*, T*, T*, T*, T*, T*, bool, GemvStatus*, \

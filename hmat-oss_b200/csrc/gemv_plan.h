@@ -26,46 +26,73 @@ struct GemvUnit {
   long long poff;  // element offset of the piece P in the arena (16-byte aligned)
   int xrow;        // first row of the X piece in the xz buffer (nruns == 0)
   int c;           // inner extent (rows of X)
-  int o0, ow;      // transposed units: output rows [o0, o0 + ow) this piece covers;
-                   // other units: o0 = byte offset of the X rows in a warp-level pipeline
-                   // stage (the piece's capacity; the FP32 tensor-core kernel reads it per unit)
-  int pel;         // elements of the piece P (O x c, or c x ow when transposed)
-  int shift;       // elements between the 16-byte aligned copy start and the piece
+  int o0, ow;      // o0 = byte offset of the X rows in a warp-level pipeline stage (the piece's
+                   // capacity; the FP32 tensor-core kernel reads it per unit); ow = output rows
+  int pel;         // elements of the piece P (O x c)
+  int shift;       // elements between the 16-byte aligned copy start and the piece (0)
   int nruns;       // 0: X rows xrow .. xrow + c - 1; else X rows from the runs below, in order
   int run_row[kUnitRuns];
   unsigned short run_len[kUnitRuns];
 };
 
+// A unit of a transposed product, 16 bytes (one load): a column-major piece of `rows` x `cols`
+// from element poff, `cols` of its columns from column o0 of the task (group pass; 0 in the column
+// pass).  x: the first xz row of its X rows (group pass), or its first entry of the column map.
+struct GemvTransUnit {
+  long long poff;
+  int x;
+  unsigned char rows, cols, o0, pad;
+};
+static_assert(sizeof(GemvTransUnit) == 16, "one 16-byte load");
+
 struct GemvTask {
   int O;           // output rows
   int first_unit;  // units [first_unit, first_unit + nunits) in order
   int nunits;
-  int out_row;     // y: first output row (cluster order); z: first xz row of the slot
+  int out_row;     // first xz row of the output slot; column pass: first xz row of the x rows
   int red = -1;    // 'N' z chunk of a long group: its z sum (GemvZred index); the last chunk of
                    // the sum to finish adds the partial slots in part order
 };
 
-// One launch: tasks of one shape class, each CTA of a persistent grid takes a contiguous
-// range [cta_begin[b], cta_begin[b + 1]) of tasks.
+// One launch: tasks of one shape class; each CTA (column pass) or warp of a persistent grid takes
+// a contiguous range [cta_begin[b], cta_begin[b + 1]) of tasks.
 struct GemvLaunch {
   int ntasks = 0;
   int ncta = 0;
   const GemvTask* tasks = nullptr;
-  const int* cta_begin = nullptr;  // warp-level launches: one range per warp (ncta * 4 + 1 entries)
-  int rpt = 1;          // rows per lane: output rows <= 32 * rpt
-  int ol = 32;          // output lanes (16 or 32)
-  bool transposed = false;
-  bool out_is_y = false;
-  // Warp-level launches ('N' products): each warp owns whole tasks and pipelines its own
-  // units.  map 3 (FP32): tensor-core tiles, at most 16 * rpt rows; map 2: column-slice
-  // window over tasks of at most 32 rows (rpt rows per lane); map 1: half-warp row groups
-  // (at most 64 rows); map 0: lanes over rows (at most 128).
-  bool warp_level = false;
-  // map 4 (FP32 'N' y launches, not warp-level): the tensor-memory kernel, one task at a time
-  // per CTA, units of at most kTcCols columns and kTcPieceBytes bytes; it writes partial rows
-  // like the warp-level launches.
+  const int* cta_begin = nullptr;  // one range per warp (ncta * 4 + 1 entries); column pass: per CTA
+  // 'N' launches: map 3 (FP32) tensor-core tiles, rpt 8-row tiles held; map 2: column-slice
+  // window over tasks of at most 32 rows; map 1: half-warp row groups (at most 64 rows); maps 5
+  // and 0: lanes over rows (at most 64 / 128); map 4 (FP32 y launches): the tensor-memory
+  // kernel, one task at a time per CTA, units of at most kTcCols columns and kTcPieceBytes bytes.
+  int rpt = 1;
   int map = 0;
+  // 'T' launches: the most bytes of a unit's piece (column pass: with its column map) and the
+  // most X rows of a unit (column pass: of a block).
+  int piece_bytes = 0;
+  int xrows = 0;
 };
+
+// Transposed products: a warp takes trans_cols columns at a time, trans_lanes lanes side by side
+// (the other lanes split the rows); its accumulators are at most 64 registers at 16 (complex
+// double: 4) right-hand sides.
+__host__ __device__ constexpr int trans_lanes(int elem_bytes) { return elem_bytes >= 16 ? 4 : 8; }
+__host__ __device__ constexpr int trans_cols(int elem_bytes) { return elem_bytes == 4 ? 32 : (elem_bytes == 8 ? 16 : 8); }
+// CTAs an SM of a transposed launch.  8-byte types: three, which leaves the kernels at 16 right-hand
+// sides their registers (FP64, 60,000-point cylinder, 11 right-hand sides: 382 us against 471 with
+// spills at four) and is what their shared memory mostly allows; the others four (three: FP32 at
+// one right-hand side 5 to 8% slower).
+__host__ __device__ constexpr int trans_ctas_per_sm(int elem_bytes) { return elem_bytes == 8 ? 3 : 4; }
+// Most bytes of a unit's piece (a unit holds trans_lanes columns at least, however tall), and the
+// shared memory a CTA may use.
+constexpr int kTransPieceBytes = 8192;
+// Shape of a warp in the column pass: at 16 FP32 right-hand sides two columns on 16 lanes, since
+// joining the slices of four columns on 8 lanes takes a third as many instructions as their sums
+// (50,001-point cylinder, column pass with the z' sums: 107.6 -> 103.5 us).
+__host__ __device__ constexpr int trans_column_lanes(int elem_bytes, int R) {
+  return elem_bytes == 4 && R >= 16 ? 16 : trans_lanes(elem_bytes);
+}
+constexpr int kMaxCtaSmem = 227 * 1024;
 
 // The arena's y region: per output block, the row panels of every leaf covering it side by side
 // (full leaves n columns, Rk leaves their A panel of k columns) as one column-major matrix
@@ -96,26 +123,31 @@ constexpr int kWarpXBytes = 2048;
 // other way, kWarpXBytesWide bytes of X rows after a piece of the rest.
 constexpr int kWarpXBytesWide = 3584;
 
-// A long leaf whose z is computed in several chunks: the chunks' partial slots
+// A long group or leaf whose z is computed in several parts: the parts' slots
 // (nparts consecutive slots of k rows from part_row) are summed into final_row.
 struct GemvZred {
   int final_row, k, part_row, nparts;
 };
 
 struct GemvSide {
-  static const int kMaxLaunch = 8;
-  int nz = 0;  // z-phase launches (one per rank class)
+  static const int kMaxLaunch = 4;
+  int nz = 0;  // 'N': z-phase launches (one per rank class); 'T': the column pass
   GemvLaunch z[kMaxLaunch];
   int nzred = 0;
+  int nzwide = 0;  // sums at the front of zred that take a CTA each
   const GemvZred* zred = nullptr;
-  // zfused: the z kernels sum the parts themselves (the 'N' side); zcnt[i]: chunks of sum i
+  const int* colmap = nullptr;  // 'T': destination rows of the column pass
+  int ng = 0;                   // 'T': group-pass launches (one per group height class)
+  GemvLaunch g[2];
+  // zfused: the z kernels sum the parts themselves ('N', FP64 and complex); zcnt[i]: chunks of sum i
   // finished in the current product (cleared by the gather that opens every product)
   bool zfused = false;
   int* zcnt = nullptr;
-  GemvLaunch y;
-  const GemvUnit* units = nullptr;
-  // The y launches write partial rows (chunks of the output blocks) into xz; the final pass
-  // reads, per client row i, yrows[i] = {xz row of part 0, nparts << 8 | O}.
+  GemvLaunch y;  // 'N'
+  const GemvUnit* units = nullptr;         // 'N'
+  const GemvTransUnit* tunits = nullptr;   // 'T'
+  // The y launches, the group pass and the column pass (full leaves) write partial rows of the
+  // output blocks into xz; the final pass reads, per client row i, yrows[i] = {xz row of part 0, nparts << 8 | O}.
   int nyrows = 0;
   const int2* yrows = nullptr;
 };
@@ -127,7 +159,7 @@ struct GemvFullLeaf {
 struct GemvRkLeaf {
   int row_off, m, col_off, n, k, pad;
   long long goff;   // canonical offset: A (m x k) then B (n x k), column-major
-  int zrow_n, zrow_t;  // xz rows of z = B^T x ('N') and z' = A^T x ('T' / 'C')
+  int zrow_n, zrow_t;  // xz rows of z = B^T x ('N') and z' = A^T x ('T' / 'C'), each in its numbering
 };
 
 // Status block of the products of one matrix, in device memory.  A kernel whose bounded
@@ -149,7 +181,9 @@ struct GemvTiming {
 struct GemvPlan {
   int n_rows = 0, n_cols = 0;
   int n_in_max = 0;      // rows of the x part of the xz buffer (kZeroRows zero rows follow it)
-  long long xz_rows = 0; // total rows of the xz buffer (x part, zero rows, z slots, partial slots)
+  // rows of the xz buffer of an 'N' and of a 'T' / 'C' product (x part, zero rows, z slots,
+  // partial slots); the two numberings are independent (rows past the zero rows overlap)
+  long long xz_rows[2] = {0, 0};
   const int* perm_rows = nullptr;  // internal -> client
   const int* perm_cols = nullptr;
   const int* iperm_rows = nullptr;  // client -> internal

@@ -190,18 +190,21 @@ void launch_tsapply_cta(const TsItem* items, int nitems, T* ws, const typename T
 }  // namespace hmatb200
 #include "gemv_plan.h"
 namespace hmatb200 {
-// y = alpha op(H) x + beta y on device buffers (client numbering); `xz` is the scratch
-// buffer of plan.xz_rows rows of gemv_rhs_stride(sizeof(T), 16) scalars; `err` is set when
-// a pipeline wait gives up.
+// y = alpha op(H) x + beta y on device buffers (client numbering), right-hand sides in tiles of at
+// most max_tile (16, 8, 4 or 1); `xz` is the scratch buffer of the side's rows (plan.xz_rows) of
+// gemv_rhs_stride(sizeof(T), max_tile) scalars; `err` is set when a pipeline wait gives up.
 template <typename T>
 void launch_gemv(const GemvPlan& p, char trans, int nrhs, T alpha, T beta, const T* x_client, T* y_client, T* xz,
-                 GemvStatus* err, cudaStream_t s, const GemvTiming* timing = nullptr);
+                 GemvStatus* err, cudaStream_t s, const GemvTiming* timing = nullptr, int max_tile = 16);
 // Row stride (scalars) of the xz buffer for R right-hand sides.
 int gemv_rhs_stride(int elem_bytes, int R);
 // Kernel launches of one product with nrhs right-hand sides.
 int gemv_launch_count(const GemvPlan& p, char trans, int nrhs, int elem_bytes);
-// Dynamic shared memory of one streamed-task CTA, and of one warp-level CTA (and its warps).
-size_t stream_smem_bytes(int elem_bytes, int R, int RS, int omax, bool transposed);
+// Dynamic shared memory of a CTA of the transposed products' two passes (and its warps), and of
+// one warp-level 'N' CTA (and its warps).
+size_t trans_columns_smem(int stage_bytes, int xrows, int xrow_bytes);
+size_t trans_groups_smem(int piece_bytes, int xrows, int xrow_bytes);
+int trans_warps_per_cta();
 size_t warp_stream_smem_bytes(int elem_bytes);
 size_t umma_smem_bytes();
 int warp_stream_warps_per_cta();

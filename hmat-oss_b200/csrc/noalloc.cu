@@ -26,11 +26,15 @@ using namespace hmatb200;
 
 namespace {
 
-// 16 MiB: the cluster-ordered x (N x 16 scalars) plus the z buffer of the matrix must fit.
+// A matrix is taken when its gemv_scratch_bytes (the cluster-ordered x, N x 16 scalars, plus the
+// z buffer) are at most 16 MiB.  The array is larger: a transposed product of such a matrix runs
+// in the widest tile of right-hand sides whose partial rows fit it, and at one right-hand side
+// the rows of an FP32 matrix of mostly full leaves take up to about 18 MB.
 // The address looked up for a device stays valid for the life of the process's context on
 // that device; a cudaDeviceReset (which destroys that context) is not supported.
 constexpr size_t kNoAllocScratchBytes = 16u << 20;
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
+constexpr size_t kNoAllocArrayBytes = 24u << 20;
+static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocArrayBytes];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_mutex;
@@ -72,7 +76,7 @@ extern "C" int hmat_b200_gemv_device_noalloc(hmat_matrix_t* m, char trans, const
     if (dev < 0 || dev >= kMaxDevices) throw Error("device index out of range");
     void* scratch = scratch_address(dev);
     e->gemv_device_with_scratch(trans, alpha, x_dev, beta, y_dev, nrhs, (cudaStream_t)stream, scratch,
-                                kNoAllocScratchBytes);
+                                kNoAllocArrayBytes);
   } catch (const std::exception& ex) {
     return report_failure("hmat_b200_gemv_device_noalloc", ex.what());
   }
