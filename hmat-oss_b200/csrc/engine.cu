@@ -4,12 +4,14 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <future>
 #include <map>
 #include <mutex>
 #include <numeric>
 #include <string>
 #include <tuple>
 #include <type_traits>
+#include <unordered_map>
 
 #include "engine.h"
 #include "gemv_plan.h"
@@ -170,12 +172,36 @@ std::vector<Block> output_blocks(const ClusterTree& t) {
   }
   return b;
 }
-// Blocks covering [off, off + len) (a union of blocks, since cluster ranges are).
-std::pair<int, int> block_range(const std::vector<Block>& b, const std::vector<int>& starts, int off, int len) {
-  int first = (int)(std::upper_bound(starts.begin(), starts.end(), off) - starts.begin()) - 1;
-  int last = first;
-  while (last < (int)b.size() && b[last].off < off + len) ++last;
-  return {first, last};
+// The block of every row.
+std::vector<int> block_of_rows(const std::vector<Block>& b, int n) {
+  std::vector<int> of(n, 0);
+  for (int i = 0; i < (int)b.size(); ++i) std::fill(of.begin() + b[i].off, of.begin() + b[i].off + b[i].len, i);
+  return of;
+}
+
+// Stable order of `items` by decreasing rows (at most kTsSegRows a warp-level item: counted, not
+// compared).
+template <typename I>
+void longest_first(std::vector<I>& items) {
+  int most = 0;
+  for (const I& it : items) most = std::max(most, it.rows);
+  std::vector<size_t> at(most + 2, 0);
+  for (const I& it : items) at[most - it.rows + 1]++;
+  for (int r = 0; r <= most; ++r) at[r + 1] += at[r];
+  std::vector<I> out(items.size());
+  for (const I& it : items) out[at[most - it.rows]++] = it;
+  items.swap(out);
+}
+
+// Stable order of the indices in v by decreasing key(index), every key computed once.
+template <typename F>
+void by_decreasing(std::vector<int>& v, F key) {
+  std::vector<std::pair<double, int>> k(v.size());
+  for (size_t i = 0; i < v.size(); ++i) k[i] = {-key(v[i]), (int)i};
+  std::sort(k.begin(), k.end());
+  std::vector<int> out(v.size());
+  for (size_t i = 0; i < v.size(); ++i) out[i] = v[k[i].second];
+  v.swap(out);
 }
 
 template <typename T>
@@ -200,8 +226,9 @@ class Engine : public EngineBase {
       if (bt_->leaves[i].type == 1) ranks[i] = 0;
     rblocks_ = output_blocks(*R_);
     cblocks_ = output_blocks(*C_);
-    for (auto& b : rblocks_) rstarts_.push_back(b.off);
-    for (auto& b : cblocks_) cstarts_.push_back(b.off);
+    persistent_grid(1);  // looks the device's SM count up before the planning threads ask for it
+    rblock_of_ = block_of_rows(rblocks_, R_->n);
+    cblock_of_ = block_of_rows(cblocks_, C_->n);
     HB_CUDA(cudaGetDevice(&device));
     err_.alloc(1);
     HB_CUDA(cudaMallocHost(&h_err_, sizeof(GemvStatus)));
@@ -289,8 +316,7 @@ class Engine : public EngineBase {
     pieces_.clear();
     // ---- the further strata, each joined to the factors the leaves hold ----
     for (int st = 1; st < nstrata; ++st) add_stratum(st, eps_aca, eps_trunc);
-    build_plan();
-    tune_gemv_plan();
+    plan_products();
     HB_CUDA(cudaStreamSynchronize(stream_));
     assembled = true;
   }
@@ -359,7 +385,7 @@ class Engine : public EngineBase {
     if (layout_.first[leaf] < 0) return 0;
     const int k = ranks[leaf];
     const int w = L.type == 0 ? L.n : k;  // columns of a row panel
-    auto br = block_range(rblocks_, rstarts_, L.row_off, L.m);
+    auto br = row_blocks(L.row_off, L.m);
     T* o = (T*)out;
     std::vector<T> h;
     for (int b = br.first; b < br.second; ++b) {  // row panels -> column-major m x w
@@ -490,8 +516,7 @@ class Engine : public EngineBase {
     launch_compact<T>(d_rd.p, (int)rd.size(), src.p, d_rk.p, d_store.p, d_panels.p, arena_.p, stream_);
     HB_CUDA(cudaGetLastError());
     HB_CUDA(cudaStreamSynchronize(stream_));
-    build_plan();
-    tune_gemv_plan();
+    plan_products();
     HB_CUDA(cudaStreamSynchronize(stream_));
     for (int i = 0; i < 4; ++i) times_ms[i] = 0;
     assembled = true;
@@ -539,8 +564,7 @@ class Engine : public EngineBase {
       cudaGraphExecDestroy(gexec_);
       gexec_ = nullptr;
     }
-    build_plan();
-    tune_gemv_plan();
+    plan_products();
     HB_CUDA(cudaStreamSynchronize(stream_));
     for (int i = 0; i < 4; ++i) times_ms[i] = saved[i];
   }
@@ -768,9 +792,7 @@ class Engine : public EngineBase {
     // on CTAs (512 threads from m + n >= kAcaBigRows, where the retried ranks are high).
     std::vector<int> svd_order, bucket_list[kAcaBuckets], shape_order[kAcaShapes];
     auto cost = [&](int b) { return (double)(desc[b].m + desc[b].n) * std::min(desc[b].m, desc[b].n); };
-    auto by_cost = [&](std::vector<int>& v) {
-      std::stable_sort(v.begin(), v.end(), [&](int x, int y) { return cost(x) > cost(y); });
-    };
+    auto by_cost = [&](std::vector<int>& v) { by_decreasing(v, cost); };
     const int forced = forced_aca_shape();
     if (!src || add_stratum) {
       for (int b = 0; b < nb; ++b) {
@@ -1008,7 +1030,7 @@ class Engine : public EngineBase {
       if (h_ranks[b] > 0 && !jobs[b].pass) good.push_back(b);
     }
     auto tcost = [&](int b) { return (double)(desc[b].m + desc[b].n) * h_ranks[b] * h_ranks[b]; };
-    std::stable_sort(good.begin(), good.end(), [&](int x, int y) { return tcost(x) > tcost(y); });
+    by_decreasing(good, tcost);
 
     typedef typename Traits<T>::wide W;
     DevArray<W> d_scratch, d_tri, d_maps;
@@ -1038,6 +1060,17 @@ class Engine : public EngineBase {
       long long tri_n = 0, map_n = 0, tb_tri = 0, tb_map = 0;
       int tb_rows = 1, tb_k = 1;
       const int kmax = ts_kmax<T>();
+      size_t nseg[4] = {}, ncore[4] = {};
+      for (int b : good) {
+        const int K = jobs[b].svd ? 0 : ts_bucket(h_ranks[b], kmax);
+        if (!K) continue;
+        nseg[K / 8 - 1] += (desc[b].m + kTsSegRows - 1) / kTsSegRows + (desc[b].n + kTsSegRows - 1) / kTsSegRows;
+        ncore[K / 8 - 1]++;
+      }
+      for (int q = 0; q < 4; ++q) {
+        ts_seg[q].reserve(nseg[q]);
+        ts_core[q].reserve(ncore[q]);
+      }
       for (int b : good) {
         if (jobs[b].svd) {
           large.push_back(b);
@@ -1153,10 +1186,8 @@ class Engine : public EngineBase {
         d_maps.alloc((size_t)map_n);
         for (int q = 0; q < 4; ++q) {
           // longest segments first: the warps take items in order
-          std::stable_sort(ts_seg[q].begin(), ts_seg[q].end(),
-                           [](const TsItem& x, const TsItem& y) { return x.rows > y.rows; });
-          std::stable_sort(ts_stack[q].begin(), ts_stack[q].end(),
-                           [](const TsItem& x, const TsItem& y) { return x.rows > y.rows; });
+          longest_first(ts_seg[q]);
+          longest_first(ts_stack[q]);
           d_ts_seg[q].upload(ts_seg[q], stream_);
           d_ts_stack[q].upload(ts_stack[q], stream_);
           d_ts_core[q].upload(ts_core[q], stream_);
@@ -1174,9 +1205,8 @@ class Engine : public EngineBase {
         d_tb_scratch.alloc((size_t)(g * tb_slab));
         d_tb_tri.alloc((size_t)tb_tri);
         d_tb_maps.alloc((size_t)tb_map);
-        std::stable_sort(tb_seg.begin(), tb_seg.end(), [](const TsItem& x, const TsItem& y) { return x.rows > y.rows; });
-        std::stable_sort(tb_stack.begin(), tb_stack.end(),
-                         [](const TsItem& x, const TsItem& y) { return x.rows > y.rows; });
+        longest_first(tb_seg);
+        longest_first(tb_stack);
         d_tb_seg.upload(tb_seg, stream_);
         d_tb_stack.upload(tb_stack, stream_);
         d_tb_core.upload(tb_core, stream_);
@@ -1247,7 +1277,7 @@ class Engine : public EngineBase {
       if (k <= 0) continue;
       const LeafInfo& l = L[jobs[b].leaf];
       loff[b] = pe;
-      auto br = block_range(rblocks_, rstarts_, l.row_off, l.m);
+      auto br = row_blocks(l.row_off, l.m);
       for (int q = br.first; q < br.second; ++q) {
         panels.push_back(PanelDesc{rblocks_[q].off - l.row_off, rblocks_[q].len, pe});
         pe += padded((long long)rblocks_[q].len * k);
@@ -1324,9 +1354,8 @@ class Engine : public EngineBase {
     }
     if (small.empty() && large.empty()) return;
     auto cost = [&](int b) { return (double)(desc[b].m + desc[b].n) * h_ranks[b] * h_ranks[b]; };
-    auto by_cost = [&](int x, int y) { return cost(x) > cost(y); };
-    std::stable_sort(small.begin(), small.end(), by_cost);
-    std::stable_sort(large.begin(), large.end(), by_cost);
+    by_decreasing(small, cost);
+    by_decreasing(large, cost);
     DevArray<int> d_small, d_large;
     DevArray<W> d_scratch;
     d_small.upload(small, stream_);
@@ -1569,7 +1598,7 @@ class Engine : public EngineBase {
     std::vector<CopySeg> segs;
     for (int i = 0; i < nleaves; ++i) {
       if (L[i].type != 0 || layout_.first[i] < 0) continue;
-      auto br = block_range(rblocks_, rstarts_, L[i].row_off, L[i].m);
+      auto br = row_blocks(L[i].row_off, L[i].m);
       for (int b = br.first; b < br.second; ++b)
         segs.push_back(CopySeg{old.panel[old.first[i] + (b - br.first)], layout_.panel[layout_.first[i] + (b - br.first)],
                                rblocks_[b].len * L[i].n, 1, 0, 0});
@@ -1612,6 +1641,15 @@ class Engine : public EngineBase {
     long long total = 0;
   };
 
+  // Output blocks [first, second) covering rows / columns [off, off + len) (cluster ranges are
+  // unions of blocks; none for an empty range).
+  std::pair<int, int> row_blocks(int off, int len) const {
+    return len > 0 ? std::make_pair(rblock_of_[off], rblock_of_[off + len - 1] + 1) : std::make_pair(0, 0);
+  }
+  std::pair<int, int> col_blocks(int off, int len) const {
+    return len > 0 ? std::make_pair(cblock_of_[off], cblock_of_[off + len - 1] + 1) : std::make_pair(0, 0);
+  }
+
   bool has_storage(int i) const {
     const LeafInfo& l = bt_->leaves[i];
     if (l.m == 0 || l.n == 0) return false;
@@ -1628,7 +1666,7 @@ class Engine : public EngineBase {
     for (int i = 0; i < nleaves; ++i) {
       if (!has_storage(i)) continue;
       const int w = L[i].type == 0 ? L[i].n : ranks[i];
-      auto br = block_range(rblocks_, rstarts_, L[i].row_off, L[i].m);
+      auto br = row_blocks(L[i].row_off, L[i].m);
       y.first[i] = (int)y.pcol.size();
       for (int b = br.first; b < br.second; ++b) {
         y.pcol.push_back(width[b]);
@@ -1646,7 +1684,7 @@ class Engine : public EngineBase {
     y.panel.resize(y.pcol.size());
     for (int i = 0; i < nleaves; ++i) {
       if (y.first[i] < 0) continue;
-      auto br = block_range(rblocks_, rstarts_, L[i].row_off, L[i].m);
+      auto br = row_blocks(L[i].row_off, L[i].m);
       for (int b = br.first; b < br.second; ++b) {
         const int e = y.first[i] + (b - br.first);
         y.panel[e] = y.yblock[b] + (long long)y.pcol[e] * rblocks_[b].len;
@@ -1656,17 +1694,13 @@ class Engine : public EngineBase {
     // in groups of at most kZGroupRows rows
     pos = pad32(pos);
     y.bt_ld.assign(nleaves, 0);
-    std::map<std::pair<int, int>, int> by_cols;
+    std::unordered_map<long long, int> by_cols;
     std::vector<std::vector<int>> members;
     for (int i = 0; i < nleaves; ++i) {
       if (L[i].type != 1 || y.first[i] < 0) continue;
-      auto key = std::make_pair(L[i].col_off, L[i].n);
-      auto it = by_cols.find(key);
-      if (it == by_cols.end()) {
-        it = by_cols.emplace(key, (int)members.size()).first;
-        members.emplace_back();
-      }
-      members[it->second].push_back(i);
+      auto it = by_cols.emplace(((long long)L[i].col_off << 32) | L[i].n, (int)members.size());
+      if (it.second) members.emplace_back();
+      members[it.first->second].push_back(i);
     }
     for (const auto& mem : members) {
       ZGroup g{0, 0, L[mem[0]].col_off, L[mem[0]].n, {}};
@@ -1680,9 +1714,8 @@ class Engine : public EngineBase {
           r += ranks[i];
         }
         pos += padded((long long)g.h * g.n);
-        y.zgroups.push_back(g);
-        g.leaves.clear();
-        g.h = 0;
+        y.zgroups.push_back(std::move(g));
+        g = ZGroup{0, 0, L[mem[0]].col_off, L[mem[0]].n, {}};
       };
       for (int i : mem) {
         if (g.h > 0 && g.h + ranks[i] > kZGroupRows) close();
@@ -1703,7 +1736,7 @@ class Engine : public EngineBase {
     for (int i = 0; i < (int)L.size(); ++i) {
       if (L[i].type != 0 || layout_.first[i] < 0) continue;
       FullLeafDesc d{L[i].row_off, L[i].m, L[i].col_off, L[i].n, (int)fp.size(), 0};
-      auto br = block_range(rblocks_, rstarts_, L[i].row_off, L[i].m);
+      auto br = row_blocks(L[i].row_off, L[i].m);
       for (int b = br.first; b < br.second; ++b) {
         fp.push_back(PanelDesc{rblocks_[b].off - L[i].row_off, rblocks_[b].len,
                                layout_.panel[layout_.first[i] + (b - br.first)]});
@@ -1719,7 +1752,7 @@ class Engine : public EngineBase {
     const LeafInfo& l = bt_->leaves[i];
     RkStoreDesc st{(int)panels.size(), 0, layout_.bt[i], layout_.first[i] < 0 ? 0 : layout_.bt_ld[i], 0};
     if (layout_.first[i] < 0) return st;
-    auto br = block_range(rblocks_, rstarts_, l.row_off, l.m);
+    auto br = row_blocks(l.row_off, l.m);
     for (int b = br.first; b < br.second; ++b) {
       panels.push_back(PanelDesc{rblocks_[b].off - l.row_off, rblocks_[b].len,
                                  layout_.panel[layout_.first[i] + (b - br.first)]});
@@ -1734,10 +1767,17 @@ class Engine : public EngineBase {
   void scatter_pieces(T* dst, float* timed = nullptr) {
     const auto& L = bt_->leaves;
     std::vector<std::vector<CopySeg>> segs(pieces_.size());
+    std::vector<size_t> nsegs(pieces_.size(), 0);
+    for (int i = 0; i < (int)L.size(); ++i) {
+      if (L[i].type != 1 || piece_of_[i] < 0 || layout_.first[i] < 0) continue;
+      const auto br = row_blocks(L[i].row_off, L[i].m);
+      nsegs[piece_of_[i]] += 1 + br.second - br.first;
+    }
+    for (size_t q = 0; q < segs.size(); ++q) segs[q].reserve(nsegs[q]);
     for (int i = 0; i < (int)L.size(); ++i) {
       if (L[i].type != 1 || piece_of_[i] < 0 || layout_.first[i] < 0) continue;
       const int k = ranks[i];
-      auto br = block_range(rblocks_, rstarts_, L[i].row_off, L[i].m);
+      auto br = row_blocks(L[i].row_off, L[i].m);
       long long p = piece_loff_[i];
       for (int b = br.first; b < br.second; ++b) {
         const int len = rblocks_[b].len * k;
@@ -1848,7 +1888,7 @@ class Engine : public EngineBase {
 
   // Units of out(O rows) += P X for a column-major O x C block at `poff`, X rows from `xrow`,
   // `cols` columns per unit.
-  void px_units(std::vector<GemvUnit>& u, long long poff, int O, int C, int xrow, int cols = 32,
+  static void px_units(std::vector<GemvUnit>& u, long long poff, int O, int C, int xrow, int cols = 32,
                 int xoff = warp_piece_bytes((int)sizeof(T))) {
     for (int j0 = 0; j0 < C; j0 += cols) {
       GemvUnit g{};  // nruns = 0: contiguous X rows
@@ -1884,7 +1924,7 @@ class Engine : public EngineBase {
 
   // Contiguous ranges of tasks of about equal bytes, one per warp of the grid.  Returns the
   // range starts; *ncta is the grid.
-  std::vector<int> partition(const std::vector<GemvTask>& tasks, const std::vector<GemvUnit>& units, int omax, int map,
+  static std::vector<int> partition(const std::vector<GemvTask>& tasks, const std::vector<GemvUnit>& units, int omax, int map,
                              int* ncta) {
     const int Rmax = sizeof(T) >= 16 ? 4 : 16;
     const int RS16 = gemv_rhs_stride((int)sizeof(T), Rmax);
@@ -1934,10 +1974,22 @@ class Engine : public EngineBase {
     L.rpt = omax <= 32 ? 2 : 4;
   }
 
+  // A side's schedule as built on the host, before its upload.
+  struct SidePlan {
+    std::vector<GemvUnit> units;
+    std::vector<GemvTransUnit> tunits;
+    std::vector<GemvTask> tasks[GemvSide::kMaxLaunch + 2];
+    std::vector<int> begin[GemvSide::kMaxLaunch + 2];
+    std::vector<GemvZred> zred;
+    std::vector<int> colmap;
+    std::vector<int2> yrows;
+  };
+
   // With `begin` given (one range of tasks per warp, or per CTA for map 4, of the full persistent
   // grid), the ranges are taken as they are instead of being cut by cost here.
-  void finish_launch(GemvLaunch& L, SideBuf& sb, int slot, std::vector<GemvTask>& tasks,
-                     const std::vector<GemvUnit>& units, const std::vector<int>* begin_given = nullptr) {
+  static void finish_launch(GemvLaunch& L, SidePlan& sp, int slot, std::vector<GemvTask>& tasks,
+                            std::vector<int>* begin_given = nullptr) {
+    const std::vector<GemvUnit>& units = sp.units;
     L.ntasks = (int)tasks.size();
     if (tasks.empty()) return;
     // X rows of every unit: contiguous, or at most kUnitRuns runs covering exactly c rows
@@ -1986,25 +2038,22 @@ class Engine : public EngineBase {
     if (begin_given) {
       const int wpc = L.map != 4 ? warp_stream_warps_per_cta() : 1;
       L.ncta = launch_ctas(omax, L.map);
-      begin = *begin_given;
+      begin.swap(*begin_given);
       if ((int)begin.size() != L.ncta * wpc + 1 || begin.front() != 0 || begin.back() != (int)tasks.size())
         throw Error("gemv plan: task ranges do not match the launch grid");
     } else {
       begin = partition(tasks, units, omax, L.map, &L.ncta);
     }
-    sb.tasks[slot].upload(tasks, stream_);
-    sb.begin[slot].upload(begin, stream_);
-    L.tasks = sb.tasks[slot].p;
-    L.cta_begin = sb.begin[slot].p;
+    sp.tasks[slot].swap(tasks);
+    sp.begin[slot].swap(begin);
   }
 
-  // The 'N' side.
+  // The 'N' side (host work only: it may run beside build_trans_side).
   void build_side(const std::vector<GemvRkLeaf>& K, const std::vector<int>& rk_leaf, long long& next_row,
-                  GemvSide& side, SideBuf& sb) {
+                  GemvSide& side, SidePlan& sp) const {
     const auto& L = bt_->leaves;
     const std::vector<Block>& oblocks = rblocks_;
-    const std::vector<int>& ostarts = rstarts_;
-    std::vector<GemvUnit> units;
+    std::vector<GemvUnit>& units = sp.units;
     // a longer z task is cut into chunks summed afterwards (spreads long groups over warps): the
     // chunk size is the gemv tuner's choice
     const int kMaxUnits = tune_zparts_;
@@ -2014,52 +2063,54 @@ class Engine : public EngineBase {
     // ---- z-phase: one task per B^T group (z = B^T x_J of its leaves at once, the x rows read
     // once); long ones cut into chunks; one launch per height class ----
     std::vector<GemvTask> zt[4];
-    std::vector<GemvUnit> zunits[4];
-    std::vector<GemvZred> zred;
-    std::vector<GemvUnit> lu;
+    std::vector<GemvZred>& zred = sp.zred;
     const auto& G = layout_.zgroups;
-    const size_t nz = G.size();
-    for (size_t t = 0; t < nz; ++t) {
-      lu.clear();
-      // the group's stacked B^T: h x n column-major
-      const ZGroup& g = G[t];
-      int xoff = 0;
-      const int zc = kTensorN ? mma_unit_cols(g.h, &xoff) : warp_unit_cols_wide(g.h, &xoff);
-      px_units(lu, g.base, g.h, g.n, g.col_off, zc, xoff);
-      const int O = g.h, zrow = zgroup_row_[0][t];
-      if (O > 128) throw Error("gemv plan: ranks above 128 are not supported by the streamed kernels");
-      // one launch takes every height up to 32; the tensor-core kernel takes every height up to 64
-      // in one (its tile count is a per-task constant), so one wave covers them
-      const int cls = kTensorN && O <= 64 ? 2 : std::max(1, rank_class(O));
-      // units of one launch must be contiguous in task order: collect them per class
-      std::vector<GemvUnit>& cu = zunits[cls];
-      if ((int)lu.size() <= kMaxUnits) {
-        zt[cls].push_back(GemvTask{O, (int)cu.size(), (int)lu.size(), zrow});
-        cu.insert(cu.end(), lu.begin(), lu.end());
-      } else {
-        const int nparts = ((int)lu.size() + kMaxUnits - 1) / kMaxUnits;
+    // one launch takes every height up to 32; the tensor-core kernel takes every height up to 64
+    // in one (its tile count is a per-task constant), so one wave covers them
+    auto z_class = [](int O) { return kTensorN && O <= 64 ? 2 : std::max(1, rank_class(O)); };
+    bool present[4] = {};
+    long long nunits = 0;
+    for (const ZGroup& g : G) {
+      if (g.h > 128) throw Error("gemv plan: ranks above 128 are not supported by the streamed kernels");
+      present[z_class(g.h)] = true;
+      nunits += (long long)g.h * g.n;
+    }
+    for (size_t b = 0; b < rblocks_.size(); ++b) nunits += (long long)rblocks_[b].len * layout_.ywidth[b];
+    // pieces are mostly full: about 4 KB each
+    units.reserve((size_t)(nunits * (long long)sizeof(T) / 4096 + 2 * G.size() + 4 * rblocks_.size()));
+    for (int cls = 0; cls < 4; ++cls) {
+      if (!present[cls]) continue;
+      // units of one launch must be contiguous in task order
+      for (size_t t = 0; t < G.size(); ++t) {
+        // the group's stacked B^T: h x n column-major
+        const ZGroup& g = G[t];
+        if (z_class(g.h) != cls) continue;
+        int xoff = 0;
+        const int zc = kTensorN ? mma_unit_cols(g.h, &xoff) : warp_unit_cols_wide(g.h, &xoff);
+        const int O = g.h, zrow = zgroup_row_[0][t], first = (int)units.size();
+        px_units(units, g.base, g.h, g.n, g.col_off, zc, xoff);
+        const int nu = (int)units.size() - first;
+        if (nu <= kMaxUnits) {
+          zt[cls].push_back(GemvTask{O, first, nu, zrow});
+          continue;
+        }
+        const int nparts = (nu + kMaxUnits - 1) / kMaxUnits;
         const int part_row = (int)next_row;
         next_row += (long long)nparts * O;
         for (int pidx = 0; pidx < nparts; ++pidx) {
-          const int u0 = pidx * kMaxUnits, u1 = std::min((int)lu.size(), u0 + kMaxUnits);
-          GemvTask task{O, (int)cu.size(), u1 - u0, part_row + pidx * O};
+          const int u0 = pidx * kMaxUnits, u1 = std::min(nu, u0 + kMaxUnits);
+          GemvTask task{O, first + u0, u1 - u0, part_row + pidx * O};
           if (kZsumInKernel) task.red = (int)zred.size();
           zt[cls].push_back(task);
-          cu.insert(cu.end(), lu.begin() + u0, lu.begin() + u1);
         }
         zred.push_back(GemvZred{zrow, O, part_row, nparts});
       }
-    }
-    for (int c = 0; c < 4; ++c) {
-      const int shift = (int)units.size();
-      for (auto& t : zt[c]) t.first_unit += shift;
-      units.insert(units.end(), zunits[c].begin(), zunits[c].end());
     }
     // ---- y-phase ----
     std::vector<std::vector<int>> per_block(oblocks.size());  // leaves with storage covering each block
     for (int i = 0; i < (int)L.size(); ++i) {
       if (layout_.first[i] < 0) continue;
-      auto br = block_range(oblocks, ostarts, L[i].row_off, L[i].m);
+      auto br = row_blocks(L[i].row_off, L[i].m);
       for (int b = br.first; b < br.second; ++b) per_block[b].push_back(i);
     }
     std::vector<int> rk_index(L.size(), -1);
@@ -2068,7 +2119,8 @@ class Engine : public EngineBase {
     std::vector<int> ybegin;  // the warps' task ranges, cut here by cost
     int maxlen = 1;
     for (const Block& ob : oblocks) maxlen = std::max(maxlen, ob.len);
-    std::vector<int2> yrows(R_->n, int2{0, 0});
+    std::vector<int2>& yrows = sp.yrows;
+    yrows.assign(R_->n, int2{0, 0});
     {
       // Each output block's matrix (the y region of the arena) in units of whole columns; the X
       // rows of its columns are the leaves' x rows (full) and z rows (Rk), merged into runs where
@@ -2076,22 +2128,27 @@ class Engine : public EngineBase {
       const int RS16 = gemv_rhs_stride((int)sizeof(T), sizeof(T) >= 16 ? 4 : 16);
       const int galign = sizeof(T) >= 16 ? 1 : 16 / (int)sizeof(T);  // columns keeping a piece aligned
       std::vector<int> ublock;  // output block of each y unit
-      std::vector<int> colrow;
+      std::vector<std::pair<int, int>> runs;  // X rows of the block's columns: (first row, rows), adjacent ones merged
       const int first_y = (int)units.size();
       for (size_t b = 0; b < oblocks.size(); ++b) {
         const int O = oblocks[b].len, W = layout_.ywidth[b];
         if (W == 0) continue;
-        colrow.clear();
+        runs.clear();
+        int used = 0;
+        auto add_run = [&](int row, int w) {
+          if (!runs.empty() && runs.back().first + runs.back().second == row)
+            runs.back().second += w;
+          else
+            runs.push_back({row, w});
+          used += w;
+        };
         for (int i : per_block[b]) {
           const bool full = L[i].type == 0;
-          const int w = full ? L[i].n : ranks[i], row = full ? L[i].col_off : K[rk_index[i]].zrow_n;
-          if ((int)colrow.size() != layout_.pcol[layout_.first[i] + (int)b - block_range(rblocks_, rstarts_,
-                                                                                          L[i].row_off, L[i].m).first])
+          if (used != layout_.pcol[layout_.first[i] + (int)b - rblock_of_[L[i].row_off]])
             throw Error("gemv plan: block matrix columns out of order");
-          for (int j = 0; j < w; ++j) colrow.push_back(row + j);
+          add_run(full ? L[i].col_off : K[rk_index[i]].zrow_n, full ? L[i].n : ranks[i]);
         }
-        const int used = (int)colrow.size();  // at most kYColAlign - 1 = kZeroRows - 1 padding columns
-        for (int j = used; j < W; ++j) colrow.push_back(plan_.n_in_max + (j - used));
+        if (used < W) add_run(plan_.n_in_max, W - used);  // at most kYColAlign - 1 = kZeroRows - 1 padding columns
         int xoff = warp_piece_bytes((int)sizeof(T)), cols;
         if (tc_y)
           cols = kTcCols;
@@ -2103,36 +2160,36 @@ class Engine : public EngineBase {
           const int step = kTensorN ? 8 : galign;
           cols = std::max(step, cols / 2 / step * step);
         }
+        size_t ri = 0;  // the run of column j0, of which `taken` columns lie before it
+        int taken = 0;
         for (int j0 = 0; j0 < W;) {
           const int want = std::min(cols, W - j0);
           // the columns the unit can take with at most kUnitRuns runs of X rows
-          int c = 0, nr = 0;
-          while (c < want) {
-            if (c == 0 || colrow[j0 + c] != colrow[j0 + c - 1] + 1) {
-              if (nr == kUnitRuns) break;
-              ++nr;
-            }
-            ++c;
-          }
+          int c = 0;
+          for (size_t r = ri; r < runs.size() && r < ri + kUnitRuns && c < want; ++r)
+            c += runs[r].second - (r == ri ? taken : 0);
+          c = std::min(c, want);
           if (c < want) c -= c % galign;  // cut short: the next piece must start 16-byte aligned
           if (c <= 0) throw Error("gemv plan: unit without columns");
           GemvUnit u{};
           u.poff = layout_.yblock[b] + (long long)j0 * O;
-          u.xrow = colrow[j0];
+          u.xrow = runs[ri].first + taken;
           u.c = c;
           u.o0 = xoff;
           u.ow = O;
           u.pel = O * c;
           u.shift = (int)(u.poff % kPad);
           if (u.shift) throw Error("gemv plan: misaligned block piece");
-          u.nruns = 0;
-          for (int j = 0; j < c; ++j) {
-            if (j == 0 || colrow[j0 + j] != colrow[j0 + j - 1] + 1) {
-              u.run_row[u.nruns] = colrow[j0 + j];
-              u.run_len[u.nruns] = 0;
-              ++u.nruns;
+          for (int left = c; left > 0;) {
+            const int len = std::min(left, runs[ri].second - taken);
+            u.run_row[u.nruns] = runs[ri].first + taken;
+            u.run_len[u.nruns++] = (unsigned short)len;
+            left -= len;
+            taken += len;
+            if (taken == runs[ri].second) {
+              ++ri;
+              taken = 0;
             }
-            ++u.run_len[u.nruns - 1];
           }
           units.push_back(u);
           ublock.push_back((int)b);
@@ -2197,7 +2254,7 @@ class Engine : public EngineBase {
       int om = 1;  // the class's tallest task (FP32 launches hold exactly its tiles)
       for (const GemvTask& t : zt[c]) om = std::max(om, t.O);
       warp_shape(L, kTensorN ? om : kClassMax[c]);
-      finish_launch(L, sb, side.nz, zt[c], units);
+      finish_launch(L, sp, side.nz, zt[c]);
       side.nz++;
     }
     side.y = GemvLaunch();
@@ -2205,18 +2262,38 @@ class Engine : public EngineBase {
       side.y.map = 4;
     else
       warp_shape(side.y, maxlen);
-    finish_launch(side.y, sb, GemvSide::kMaxLaunch, yt, units, &ybegin);
-    sb.units.upload(units, stream_);
-    side.units = sb.units.p;
-    sb.zred.upload(zred, stream_);
-    side.nzred = (int)zred.size();
-    side.zred = sb.zred.p;
+    finish_launch(side.y, sp, GemvSide::kMaxLaunch, yt, &ybegin);
     side.zfused = kZsumInKernel;
-    sb.zcnt.alloc((size_t)std::max<size_t>(zred.size(), 1));
+  }
+
+  // Uploads a side's schedule and points its launches at it.
+  void upload_side(SidePlan& sp, GemvSide& side, SideBuf& sb) {
+    for (int i = 0; i < GemvSide::kMaxLaunch + 2; ++i) {
+      if (sp.tasks[i].empty()) continue;
+      sb.tasks[i].upload(sp.tasks[i], stream_);
+      sb.begin[i].upload(sp.begin[i], stream_);
+    }
+    auto point = [&](GemvLaunch& l, int slot) {
+      l.tasks = sb.tasks[slot].p;
+      l.cta_begin = sb.begin[slot].p;
+    };
+    for (int c = 0; c < side.nz; ++c) point(side.z[c], c);
+    for (int c = 0; c < side.ng; ++c) point(side.g[c], GemvSide::kMaxLaunch + c);
+    if (side.y.ntasks > 0) point(side.y, GemvSide::kMaxLaunch);
+    sb.units.upload(sp.units, stream_);
+    side.units = sb.units.p;
+    sb.tunits.upload(sp.tunits, stream_);
+    side.tunits = sb.tunits.p;
+    sb.colmap.upload(sp.colmap, stream_);
+    side.colmap = sb.colmap.p;
+    sb.zred.upload(sp.zred, stream_);
+    side.nzred = (int)sp.zred.size();
+    side.zred = sb.zred.p;
+    sb.zcnt.alloc(std::max<size_t>(sp.zred.size(), 1));
     HB_CUDA(cudaMemsetAsync(sb.zcnt.p, 0, sb.zcnt.n * sizeof(int), stream_));
     side.zcnt = sb.zcnt.p;
-    sb.yrows.upload(yrows, stream_);
-    side.nyrows = (int)yrows.size();
+    sb.yrows.upload(sp.yrows, stream_);
+    side.nyrows = (int)sp.yrows.size();
     side.yrows = sb.yrows.p;
   }
 
@@ -2243,25 +2320,19 @@ class Engine : public EngineBase {
     for (++w; w <= G; ++w) begin[w] = (int)tasks.size();
   }
 
-  void upload_launch(GemvLaunch& L, SideBuf& sb, int slot, const std::vector<GemvTask>& tasks,
-                     const std::vector<int>& begin) {
-    L.ntasks = (int)tasks.size();
-    sb.tasks[slot].upload(tasks, stream_);
-    sb.begin[slot].upload(begin, stream_);
-    L.tasks = sb.tasks[slot].p;
-    L.cta_begin = sb.begin[slot].p;
-  }
-
   // The 'T' / 'C' side: the column pass over the output blocks' matrices, the sums of the z' parts
   // of leaves over several blocks, the group pass over the B^T groups, the final sum.
   void build_trans_side(const std::vector<GemvRkLeaf>& K, const std::vector<int>& rk_leaf, long long& next_row,
-                        GemvSide& side, SideBuf& sb) {
+                        GemvSide& side, SidePlan& sp) const {
     const auto& L = bt_->leaves;
     const auto& G = layout_.zgroups;
     const int s = (int)sizeof(T);
     const int CL = trans_lanes(s), CW = trans_cols(s);
     const int RS16 = gemv_rhs_stride(s, s >= 16 ? 4 : 16);
-    std::vector<GemvTransUnit> units;
+    std::vector<GemvTransUnit>& units = sp.tunits;
+    long long scalars = 0;
+    for (const ZGroup& g : G) scalars += (long long)g.h * g.n;
+    units.reserve((size_t)(scalars * s / 2048) + 2 * G.size());  // pieces of a strip's columns, 2 to 4 KB
 
     // the rows of y: the column blocks cut into strips of at most CW columns, CL-wide but the last
     std::vector<Block> strips;
@@ -2281,7 +2352,7 @@ class Engine : public EngineBase {
     // launch (small stages, more CTAs), taller ones (one leaf of higher rank) in another ----
     std::vector<std::vector<int>> groups_of(cblocks_.size());
     for (size_t gi = 0; gi < G.size(); ++gi) {
-      auto br = block_range(cblocks_, cstarts_, G[gi].col_off, G[gi].n);
+      auto br = col_blocks(G[gi].col_off, G[gi].n);
       for (int b = br.first; b < br.second; ++b) groups_of[b].push_back((int)gi);
     }
     std::vector<int> nparts(strips.size(), 0);
@@ -2332,12 +2403,13 @@ class Engine : public EngineBase {
     std::vector<int> fullparts(strips.size(), 0);
     for (int i = 0; i < (int)L.size(); ++i) {
       if (layout_.first[i] < 0 || L[i].type != 0) continue;
-      auto br = block_range(rblocks_, rstarts_, L[i].row_off, L[i].m);
+      auto br = row_blocks(L[i].row_off, L[i].m);
       const int last = strip_of[L[i].col_off + L[i].n - 1];
       for (int st = strip_of[L[i].col_off]; st <= last; ++st) fullparts[st] += br.second - br.first;
     }
     std::vector<int> part_row(strips.size(), 0), taken(strips.size(), 0);
-    std::vector<int2> yrows(C_->n, int2{0, 0});
+    std::vector<int2>& yrows = sp.yrows;
+    yrows.assign(C_->n, int2{0, 0});
     for (size_t st = 0; st < strips.size(); ++st) {
       const int np = fullparts[st] + nparts[st];
       part_row[st] = (int)next_row;
@@ -2358,13 +2430,15 @@ class Engine : public EngineBase {
     std::vector<long long> colbase(rblocks_.size() + 1, 0);
     for (size_t b = 0; b < rblocks_.size(); ++b) colbase[b + 1] = colbase[b] + layout_.ywidth[b];
     if (colbase.back() >= (1LL << 31)) throw Error("gemv plan: too many columns");
-    std::vector<int> colmap((size_t)colbase.back() + 4, 0), used(rblocks_.size(), 0);
-    std::vector<GemvZred> zred;
+    std::vector<int>& colmap = sp.colmap;
+    colmap.assign((size_t)colbase.back() + 4, 0);
+    std::vector<int> used(rblocks_.size(), 0);
+    std::vector<GemvZred>& zred = sp.zred;
     std::vector<int> rk_index(L.size(), -1);
     for (size_t t = 0; t < rk_leaf.size(); ++t) rk_index[rk_leaf[t]] = (int)t;
     for (int i = 0; i < (int)L.size(); ++i) {
       if (layout_.first[i] < 0) continue;
-      auto br = block_range(rblocks_, rstarts_, L[i].row_off, L[i].m);
+      auto br = row_blocks(L[i].row_off, L[i].m);
       const int nb = br.second - br.first, w = L[i].type == 0 ? L[i].n : ranks[i];
       int zrow = 0;
       if (L[i].type != 0) {
@@ -2434,33 +2508,33 @@ class Engine : public EngineBase {
         ct[t].O = rblocks_[cblock[t]].len;
         ct[t].out_row = rblocks_[cblock[t]].off;  // the block's x rows
       }
-      upload_launch(l, sb, 0, ct, cbegin);
+      l.ntasks = (int)ct.size();
+      sp.tasks[0].swap(ct);
+      sp.begin[0].swap(cbegin);
       side.nz = 1;
     }
-    for (int c = 0; c < side.ng; ++c) upload_launch(side.g[c], sb, GemvSide::kMaxLaunch + c, gt[c], gbegin[c]);
+    for (int c = 0; c < side.ng; ++c) {
+      side.g[c].ntasks = (int)gt[c].size();
+      sp.tasks[GemvSide::kMaxLaunch + c].swap(gt[c]);
+      sp.begin[GemvSide::kMaxLaunch + c].swap(gbegin[c]);
+    }
     for (int m : colmap)
       if (m < 0 || m >= next_row) throw Error("gemv plan: column map out of range");
-    sb.tunits.upload(units, stream_);
-    side.tunits = sb.tunits.p;
-    sb.colmap.upload(colmap, stream_);
-    side.colmap = sb.colmap.p;
-    sb.zred.upload(zred, stream_);
-    side.nzred = (int)zred.size();
-    side.zred = sb.zred.p;
     side.zfused = false;
-    sb.yrows.upload(yrows, stream_);
-    side.nyrows = (int)yrows.size();
-    side.yrows = sb.yrows.p;
   }
   // Sums of z' parts above this many take a CTA of eight warps instead of one warp.
   static constexpr int kZredWideParts = 16;
 
-  void build_plan() {
+  // The products' schedules.  The two sides are built on two threads (host work of about the same
+  // length), then uploaded.  With `only_n` (the tuner's candidates) the 'T' side stays as it is.
+  void build_plan(bool only_n = false) {
     const auto& L = bt_->leaves;
     std::vector<GemvFullLeaf> F;
     std::vector<GemvRkLeaf> K;
     std::vector<int> rk_leaf;
     long long goff = 0;
+    const GemvSide trans_side = plan_.side[1];
+    const long long trans_rows = plan_.xz_rows[1];
     plan_ = GemvPlan();
     plan_.n_rows = R_->n;
     plan_.n_cols = C_->n;
@@ -2513,12 +2587,26 @@ class Engine : public EngineBase {
     plan_.rk = g_rk_.p;
     plan_.nfull = (int)F.size();
     plan_.nrk = (int)K.size();
-    build_side(K, rk_leaf, next_row[0], plan_.side[0], side_buf_[0]);
-    build_trans_side(K, rk_leaf, next_row[1], plan_.side[1], side_buf_[1]);
-    for (int side = 0; side < 2; ++side) {
-      plan_.xz_rows[side] = next_row[side];
-      if (next_row[side] >= (1LL << 31)) throw Error("gemv plan: z buffer too large");
+    {
+      SidePlan sp[2];
+      std::future<void> trans;
+      if (!only_n)
+        trans = std::async(std::launch::async,
+                           [&] { build_trans_side(K, rk_leaf, next_row[1], plan_.side[1], sp[1]); });
+      build_side(K, rk_leaf, next_row[0], plan_.side[0], sp[0]);
+      if (!only_n) trans.get();
+      upload_side(sp[0], plan_.side[0], side_buf_[0]);
+      if (!only_n) upload_side(sp[1], plan_.side[1], side_buf_[1]);
+      HB_CUDA(cudaStreamSynchronize(stream_));  // the host vectors go out of scope
     }
+    plan_.xz_rows[0] = next_row[0];
+    plan_.xz_rows[1] = next_row[1];
+    if (only_n) {
+      plan_.side[1] = trans_side;
+      plan_.xz_rows[1] = trans_rows;
+    }
+    for (int side = 0; side < 2; ++side)
+      if (plan_.xz_rows[side] >= (1LL << 31)) throw Error("gemv plan: z buffer too large");
     noalloc_rows_ = next_row[0] + noalloc_trans_rows(K);
   }
 
@@ -2533,19 +2621,19 @@ class Engine : public EngineBase {
     long long rows = 0;
     for (const GemvRkLeaf& k : K) {
       rows += k.k;
-      auto br = block_range(rblocks_, rstarts_, k.row_off, k.m);
+      auto br = row_blocks(k.row_off, k.m);
       const long long nu = (br.second - br.first) * strips32(k.k);
       if (nu > kUnits) rows += (nu + kUnits - 1) / kUnits * k.k;
     }
     std::vector<long long> nu(cblocks_.size(), 0);
     for (int i = 0; i < (int)L.size(); ++i) {
       if (L[i].type != 0 || layout_.first[i] < 0) continue;
-      auto rb = block_range(rblocks_, rstarts_, L[i].row_off, L[i].m);
-      auto cb = block_range(cblocks_, cstarts_, L[i].col_off, L[i].n);
+      auto rb = row_blocks(L[i].row_off, L[i].m);
+      auto cb = col_blocks(L[i].col_off, L[i].n);
       for (int b = cb.first; b < cb.second; ++b) nu[b] += (rb.second - rb.first) * strips32(cblocks_[b].len);
     }
     for (const ZGroup& g : layout_.zgroups) {
-      auto cb = block_range(cblocks_, cstarts_, g.col_off, g.n);
+      auto cb = col_blocks(g.col_off, g.n);
       for (int b = cb.first; b < cb.second; ++b) nu[b] += strips32(cblocks_[b].len);
     }
     for (size_t b = 0; b < cblocks_.size(); ++b) rows += (nu[b] + kUnits - 1) / kUnits * cblocks_[b].len;
@@ -2595,25 +2683,29 @@ class Engine : public EngineBase {
     *yms = b;
   }
 
-  void tune_gemv_plan() {
+  // Builds the products' schedules, with the tuner's choice for the matrix's class.
+  void plan_products() {
     gemv_tuned = 0;
     gemv_choice[0] = tune_zparts_ = 16;
     gemv_choice[1] = 0;
     tune_yhalf_ = false;
     for (double& v : gemv_rate) v = 0.0;
     const int mode = gemv_tuning_mode();
-    if (mode == 0) return;
     const long long bytes = layout_.total * (long long)sizeof(T);
-    if (mode == 1 && bytes < (64LL << 20)) return;
+    if (mode == 0 || (mode == 1 && bytes < (64LL << 20))) {
+      build_plan();
+      return;
+    }
     int maxlen = 1;
     for (const Block& b : rblocks_) maxlen = std::max(maxlen, b.len);
     const auto key = std::make_tuple((int)sizeof(T) * 2 + (Traits<T>::is_complex ? 1 : 0), (maxlen + 15) / 16, 0, 0);
     if (mode == 1) {
-      std::lock_guard<std::mutex> g(g_tune_mu);
+      std::unique_lock<std::mutex> g(g_tune_mu);
       auto it = g_gemv_tune_cache.find(key);
       if (it != g_gemv_tune_cache.end()) {
         tune_zparts_ = it->second.first;
         tune_yhalf_ = it->second.second;
+        g.unlock();
         gemv_choice[0] = tune_zparts_;
         gemv_choice[1] = tune_yhalf_ ? 1 : 0;
         gemv_tuned = 2;
@@ -2627,7 +2719,7 @@ class Engine : public EngineBase {
     for (int i = 0; i < 3; ++i) {
       tune_zparts_ = kZparts[i];
       tune_yhalf_ = false;
-      build_plan();
+      build_plan(i > 0);
       double z, y;
       time_phases(&z, &y);
       gemv_rate[i] = z;
@@ -2639,12 +2731,12 @@ class Engine : public EngineBase {
     }
     tune_zparts_ = zp;
     tune_yhalf_ = true;
-    build_plan();
+    build_plan(true);
     double z, yh;
     time_phases(&z, &yh);
     gemv_rate[4] = yh;
     tune_yhalf_ = yh < gemv_rate[3];
-    if (!tune_yhalf_) build_plan();
+    if (!tune_yhalf_) build_plan(true);
     gemv_choice[0] = tune_zparts_;
     gemv_choice[1] = tune_yhalf_ ? 1 : 0;
     gemv_tuned = 1;
@@ -2658,7 +2750,7 @@ class Engine : public EngineBase {
   const ClusterTree* C_;
   const BlockTree* bt_;
   std::vector<Block> rblocks_, cblocks_;
-  std::vector<int> rstarts_, cstarts_;
+  std::vector<int> rblock_of_, cblock_of_;  // the block of every row / column
   cudaStream_t stream_ = nullptr;
   cudaStream_t stream2_ = nullptr;  // runs the tall-skinny truncation beside the CTA kernel
   cudaStream_t stream3_ = nullptr;  // runs the 512-thread ACA beside the other ACA kernels
