@@ -48,3 +48,31 @@ def test_transposed_products(hb, vt, n, leaf, leaf_cols, eta, eps):
                 assert np.all(np.abs(got - want) <= bound + 1e-300), (trans, nrhs, np.max(np.abs(got - want) / bound))
     finally:
         h.close()
+
+
+@pytest.mark.parametrize("n,leaf,leaf_cols,eta,eps", [
+    (1, 1, None, 2.0, 1e-6), (40, 1, None, 2.0, 1e-6), (300, 7, None, 2.0, 1e-6), (900, 32, None, 2.0, 1e-6),
+    (900, 33, None, 2.0, 1e-6), (1500, 64, None, 2.0, 1e-6), (1500, 100, None, 2.0, 1e-4),
+    (1500, 128, None, 2.0, 1e-4), (1500, 190, None, 2.0, 1e-4), (1500, 90, 20, 2.0, 1e-6),
+    (3000, 50, None, 6.0, 1e-6)])
+def test_single_fp32_product(hb, n, leaf, leaf_cols, eta, eps):
+    """'N' with one FP32 right-hand side, on its own kernels, against the stored leaves in FP64."""
+    pts = np.random.default_rng(n + leaf).random((n, 3))
+    hb.set_parameters(compressionMinLeafSize=0)
+    h = hb.HMatrix(pts, hb.kernel(hb.EXP_COV, ell=0.3, nugget=1e-6), value_type=0, leaf_size=leaf,
+                   leaf_size_cols=leaf_cols, eta=eta, epsilon=eps)
+    try:
+        H = np.zeros((n, n))
+        pr, pc = h.perm(), h.perm(cols=True)
+        for i, (r0, m, c0, nn, _, _) in enumerate(h.leaf_table()):
+            H[np.ix_(pr[r0:r0 + m], pc[c0:c0 + nn])] = h.leaf_block(i)
+        rng = np.random.default_rng(1)
+        for nrhs in (1, 17):  # 17: a tile of 16 and one of 1
+            x, y0 = (rng.standard_normal((n, nrhs)).astype(np.float32) for _ in range(2))
+            want = 0.5 * (H @ x.astype(np.float64)) + 2.0 * y0
+            got = h.gemv(x, alpha=0.5, beta=2.0, y=y0)
+            # the bound of test_transposed_products
+            bound = 16.0 * 2.0 ** -24 * (np.abs(H) @ np.abs(x) * np.sqrt(n) + np.abs(y0))
+            assert np.all(np.abs(got - want) <= bound + 1e-300), nrhs
+    finally:
+        h.close()
