@@ -1049,7 +1049,7 @@ class Engine : public EngineBase {
     DevArray<TsCore> d_tb_core;
     DevArray<W> d_tb_tri, d_tb_maps, d_tb_scratch;
     long long tb_slab = 0;
-    int tb_grid = 0;
+    int tb_grid = 0, tb_kmax = 0;
     if (!good.empty()) {
       // Leaves up to rank ts_kmax go to the tall-skinny phases (row segments of A and B
       // reduced to triangles, stacks of triangles reduced again, core, apply), higher ranks
@@ -1199,6 +1199,7 @@ class Engine : public EngineBase {
         size_t budget = workspace_budget();
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) budget = std::max(budget, free_b / 3);
+        tb_kmax = tb_k;
         long long g = std::min<long long>((long long)tb_seg.size(), persistent_grid(4));
         g = std::max(1LL, std::min<long long>(g, (long long)(budget / (tb_slab * sizeof(W)))));
         tb_grid = (int)g;
@@ -1243,7 +1244,7 @@ class Engine : public EngineBase {
                            tb_grid, d_counter.p, stream_);
         launch_tsqr_cta<T>(d_tb_stack.p, (int)tb_stack.size(), d_ws.p, d_tb_tri.p, true, d_tb_scratch.p, tb_slab,
                            tb_grid, d_counter.p, stream_);
-        launch_tscore_cta<T>(d_tb_core.p, (int)tb_core.size(), d_tb_tri.p, d_tb_maps.p, d_ranks.p, d_status.p,
+        launch_tscore_cta<T>(d_tb_core.p, (int)tb_core.size(), tb_kmax, d_tb_tri.p, d_tb_maps.p, d_ranks.p, d_status.p,
                              eps_trunc, d_tb_scratch.p, tb_slab, tb_grid, d_counter.p, stream_);
         launch_tsapply_cta<T>(d_tb_seg.p, (int)tb_seg.size(), d_ws.p, d_tb_maps.p, d_ranks.p, d_tb_scratch.p, tb_slab,
                               tb_grid, d_counter.p, stream_);

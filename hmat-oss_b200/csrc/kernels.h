@@ -178,7 +178,7 @@ template <typename T>
 void launch_tsqr_cta(const TsItem* items, int nitems, const T* ws, typename Traits<T>::wide* tri, bool from_tri,
                      typename Traits<T>::wide* scratch, long long slab, int grid, int* counter, cudaStream_t s);
 template <typename T>
-void launch_tscore_cta(const TsCore* items, int nitems, const typename Traits<T>::wide* tri,
+void launch_tscore_cta(const TsCore* items, int nitems, int kmax, const typename Traits<T>::wide* tri,
                        typename Traits<T>::wide* maps, int* ranks, int* status, double eps,
                        typename Traits<T>::wide* scratch, long long slab, int grid, int* counter, cudaStream_t s);
 template <typename T>

@@ -10,6 +10,7 @@
 // complex FP64) whatever the storage type, and the new factors are narrowed back into the
 // leaf's workspace slot.
 #include <cstdlib>
+#include <type_traits>
 
 #include "block_reduce.cuh"
 #include "kernels.h"
@@ -30,6 +31,11 @@ __device__ inline cdouble phase_of(cdouble a, double absa) {
 }
 __device__ inline double scal(double s, double a) { return s * a; }
 __device__ inline cdouble scal(double s, cdouble a) { return cdouble{s * a.x, s * a.y}; }
+
+// Real columns a warp updates together in a Householder step: their loads of v are shared and
+// their sums overlap.  Complex columns go one at a time (at four a warp, a 30,000-point Helmholtz
+// cylinder's tsqr_cta took 9.5 ms instead of 7.2: twice the registers, fewer columns than warps).
+constexpr int kQrBatch = 4;
 
 // Householder QR of X (len x k, ld = len) in place: v_j stored in X[j:, j] (v_j[j] explicit),
 // tau[j], and R (k x k, column-major, upper) written separately.
@@ -61,19 +67,51 @@ __device__ void householder_qr(W* X, int len, int k, W* tau, W* R, RedScratch& r
       R[j + (size_t)j * k] = beta;
       for (int i = j + 1; i < k; ++i) R[i + (size_t)j * k] = zero<W>();
     }
-    // apply H_j = I - t v v^H to columns c > j, warp per column
-    for (int c = j + 1 + warp; c < k; c += nw) {
-      W* y = X + (size_t)c * len;
-      W s = zero<W>();
-      if (nrm > 0.0)
-        for (int i = j + lane; i < len; i += 32) s = s + conjg(x[i]) * y[i];
-      s = warp_sum(s);
-      s = warp_bcast(s);
-      W ts = t * s;
-      if (nrm > 0.0)
-        for (int i = j + lane; i < len; i += 32) y[i] = y[i] - ts * x[i];
-      __syncwarp();
-      if (lane == 0) R[j + (size_t)c * k] = y[j];
+    // apply H_j = I - t v v^H to columns c > j
+    if constexpr (std::is_same<W, double>::value) {
+      for (int c0 = j + 1 + warp; c0 < k; c0 += nw * kQrBatch) {
+        W s[kQrBatch];
+  #pragma unroll
+        for (int b = 0; b < kQrBatch; ++b) s[b] = zero<W>();
+        if (nrm > 0.0)
+          for (int i = j + lane; i < len; i += 32) {
+            const W v = conjg(x[i]);
+  #pragma unroll
+            for (int b = 0; b < kQrBatch; ++b)
+              if (c0 + b * nw < k) s[b] = s[b] + v * X[(size_t)(c0 + b * nw) * len + i];
+          }
+  #pragma unroll
+        for (int b = 0; b < kQrBatch; ++b) s[b] = t * warp_bcast(warp_sum(s[b]));
+        if (nrm > 0.0)
+          for (int i = j + lane; i < len; i += 32) {
+            const W v = x[i];
+  #pragma unroll
+            for (int b = 0; b < kQrBatch; ++b)
+              if (c0 + b * nw < k) {
+                W* y = X + (size_t)(c0 + b * nw) * len;
+                y[i] = y[i] - s[b] * v;
+              }
+          }
+        __syncwarp();
+        if (lane == 0)
+  #pragma unroll
+          for (int b = 0; b < kQrBatch; ++b)
+            if (c0 + b * nw < k) R[j + (size_t)(c0 + b * nw) * k] = X[(size_t)(c0 + b * nw) * len + j];
+      }
+    } else {
+      for (int c = j + 1 + warp; c < k; c += nw) {
+        W* y = X + (size_t)c * len;
+        W s = zero<W>();
+        if (nrm > 0.0)
+          for (int i = j + lane; i < len; i += 32) s = s + conjg(x[i]) * y[i];
+        s = warp_sum(s);
+        s = warp_bcast(s);
+        W ts = t * s;
+        if (nrm > 0.0)
+          for (int i = j + lane; i < len; i += 32) y[i] = y[i] - ts * x[i];
+        __syncwarp();
+        if (lane == 0) R[j + (size_t)c * k] = y[j];
+      }
     }
     __syncthreads();
   }
@@ -1030,27 +1068,49 @@ __host__ __device__ constexpr size_t dense_jacobi_smem(int len, int k) {
   return (size_t)3 * len * k * sizeof(double) + 2 * (size_t)k * sizeof(double) + (size_t)k * sizeof(int);
 }
 
+// a + b with one rounding a component (never fused with the product that made a or b).
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ cdouble add_rn(cdouble a, cdouble b) { return cdouble{__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y)}; }
+// acc + conj(a) b.
+__device__ __forceinline__ double dot_acc(double a, double b, double acc) { return fma(a, b, acc); }
+__device__ __forceinline__ cdouble dot_acc(cdouble a, cdouble b, cdouble acc) { return acc + conjg(a) * b; }
+// |a|^2 added to acc.
+__device__ __forceinline__ double sq_acc(double a, double acc) { return fma(a, a, acc); }
+__device__ __forceinline__ double sq_acc(cdouble a, double acc) { return fma(a.y, a.y, fma(a.x, a.x, acc)); }
+// (cs x - sn y, sn x + cs y), for real scalars with the roundings of jacobi_svd's rotation.
+__device__ __forceinline__ void rotate(double cs, double sn, double& x, double& y) {
+  const double p = fma(cs, x, -__dmul_rn(sn, y)), q = fma(sn, x, __dmul_rn(cs, y));
+  x = p;
+  y = q;
+}
+__device__ __forceinline__ void rotate(double cs, double sn, cdouble& x, cdouble& y) {
+  rotate(cs, sn, x.x, y.x);
+  rotate(cs, sn, x.y, y.y);
+}
+__device__ __forceinline__ double phase_mul(double a, double ph) { return __dmul_rn(a, ph); }
+__device__ __forceinline__ cdouble phase_mul(cdouble a, cdouble ph) { return a * ph; }
+
 // Sum over the virtual lanes of a pair's lanes (v[c]: virtual lane l + L c), as warp_sum adds 32
 // lanes.
-template <int L>
-__device__ __forceinline__ double lanes_sum(const double (&v)[32 / L]) {
-  double t[32 / L];
+template <int L, typename V>
+__device__ __forceinline__ V lanes_sum(const V (&v)[32 / L]) {
+  V t[32 / L];
 #pragma unroll
   for (int c = 0; c < 32 / L; ++c) t[c] = v[c];
 #pragma unroll
   for (int n = 16 / L; n > 0; n >>= 1)
 #pragma unroll
-    for (int c = 0; c < n; ++c) t[c] = __dadd_rn(t[c], t[c + n]);
-  double s = t[0];
+    for (int c = 0; c < n; ++c) t[c] = add_rn(t[c], t[c + n]);
+  V s = t[0];
 #pragma unroll
-  for (int off = L / 2; off > 0; off >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, off));
+  for (int off = L / 2; off > 0; off >>= 1) s = add_rn(s, ts_xor(s, off));
   return s;
 }
 
-// jacobi_svd with L lanes a pair; Wm and V in shared memory.
-template <int L>
-__device__ bool jacobi_svd_lanes(double* Wm, double* V, int k, int* s_rot) {
-  constexpr int C = 32 / L, H = kDenseJacobiChain;
+// jacobi_svd with L lanes a pair, columns of at most 32 H; Wm and V in shared memory.
+template <int L, int H, typename W>
+__device__ bool jacobi_svd_lanes(W* Wm, W* V, int k, int* s_rot) {
+  constexpr int C = 32 / L;
   const int l = threadIdx.x % L, grp = threadIdx.x / L, ngrp = blockDim.x / L;
   const int kk = (k + 1) & ~1;
   const int max_sweeps = g_jacobi_max_sweeps;
@@ -1064,49 +1124,50 @@ __device__ bool jacobi_svd_lanes(double* Wm, double* V, int k, int* s_rot) {
         const int b = 1 + (kk - 2 - pr + round) % (kk - 1);
         const int p = min(a, b), q = max(a, b);
         const bool live = pr < kk / 2 && q < k;
-        double* wp = Wm + (size_t)(live ? p : 0) * k;
-        double* wq = Wm + (size_t)(live ? q : 0) * k;
-        double x[C][H], y[C][H], alc[C], bec[C], gc[C];
+        W* wp = Wm + (size_t)(live ? p : 0) * k;
+        W* wq = Wm + (size_t)(live ? q : 0) * k;
+        W x[C][H], y[C][H], gc[C];
+        double alc[C], bec[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-          double al = 0.0, be = 0.0, g = 0.0;
+          alc[c] = bec[c] = 0.0;
+          gc[c] = zero<W>();
 #pragma unroll
           for (int h = 0; h < H; ++h) {
             const int i = l + L * c + 32 * h;
             const bool in = live && i < k;
-            x[c][h] = in ? wp[i] : 0.0;
-            y[c][h] = in ? wq[i] : 0.0;
-            al = fma(x[c][h], x[c][h], al);
-            be = fma(y[c][h], y[c][h], be);
-            g = fma(x[c][h], y[c][h], g);
+            x[c][h] = in ? wp[i] : zero<W>();
+            y[c][h] = in ? wq[i] : zero<W>();
+            alc[c] = sq_acc(x[c][h], alc[c]);
+            bec[c] = sq_acc(y[c][h], bec[c]);
+            gc[c] = dot_acc(x[c][h], y[c][h], gc[c]);
           }
-          alc[c] = al;
-          bec[c] = be;
-          gc[c] = g;
         }
-        const double al = lanes_sum<L>(alc), be = lanes_sum<L>(bec), g = lanes_sum<L>(gc);
+        const double al = lanes_sum<L>(alc), be = lanes_sum<L>(bec);
+        const W g = lanes_sum<L>(gc);
         const double ag = sqrt(abs2(g));
         if (!live || ag == 0.0 || ag <= 1e-15 * sqrt(al * be)) continue;
         if (l == 0) *s_rot = 1;
-        const double phc = __dmul_rn(1.0 / ag, g);
+        const W phc = conjg(scal(1.0 / ag, g));
         const double zeta = __dsub_rn(be, al) / __dmul_rn(2.0, ag);
         const double t = (zeta >= 0.0 ? 1.0 : -1.0) / __dadd_rn(fabs(zeta), sqrt(fma(zeta, zeta, 1.0)));
         const double cs = 1.0 / sqrt(fma(t, t, 1.0)), sn = __dmul_rn(cs, t);
-        double* vp = V + (size_t)p * k;
-        double* vq = V + (size_t)q * k;
+        W* vp = V + (size_t)p * k;
+        W* vq = V + (size_t)q * k;
 #pragma unroll
         for (int c = 0; c < C; ++c)
 #pragma unroll
           for (int h = 0; h < H; ++h) {
             const int i = l + L * c + 32 * h;
             if (i < k) {
-              // the roundings of the slab kernel's rotation, pinned
-              const double wx = x[c][h], wy = __dmul_rn(y[c][h], phc);
-              wp[i] = fma(cs, wx, -__dmul_rn(sn, wy));
-              wq[i] = fma(sn, wx, __dmul_rn(cs, wy));
-              const double vx = vp[i], vy = __dmul_rn(vq[i], phc);
-              vp[i] = fma(cs, vx, -__dmul_rn(sn, vy));
-              vq[i] = fma(sn, vx, __dmul_rn(cs, vy));
+              W wx = x[c][h], wy = phase_mul(y[c][h], phc);
+              rotate(cs, sn, wx, wy);
+              wp[i] = wx;
+              wq[i] = wy;
+              W vx = vp[i], vy = phase_mul(vq[i], phc);
+              rotate(cs, sn, vx, vy);
+              vp[i] = vx;
+              vq[i] = vy;
             }
           }
       }
@@ -1159,7 +1220,7 @@ __global__ void __launch_bounds__(kDenseJacobiThreads, 2) dense_jacobi_kernel(co
     __syncthreads();
     for (int e = tid; e < k * k; e += blockDim.x) Vm[e] = e % (k + 1) == 0 ? 1.0 : 0.0;
     __syncthreads();
-    const bool conv = jacobi_svd_lanes<kDenseJacobiLanes>(Rm, Vm, k, &s_rot);
+    const bool conv = jacobi_svd_lanes<kDenseJacobiLanes, kDenseJacobiChain>(Rm, Vm, k, &s_rot);
     for (int j = tid; j < k; j += blockDim.x) {
       double s2 = 0.0;
       for (int i = 0; i < k; ++i) s2 += abs2(Rm[i + (size_t)j * k]);
@@ -1252,14 +1313,19 @@ __global__ void __launch_bounds__(kTruncThreads) tsqr_cta_kernel(const TsItem* _
 
 // Core of one leaf: Ra Rb^T, Jacobi, sigma order, k', and the maps (k x k, ld k, columns at
 // or past k' zero), as tscore_kernel.
-template <typename W>
-__global__ void __launch_bounds__(kTruncThreads) tscore_cta_kernel(const TsCore* __restrict__ items, int nitems,
-                                                                    const W* __restrict__ tri, W* maps, int* ranks,
-                                                                    int* status, double eps, W* scratch,
-                                                                    long long slab_elems, int* counter) {
+// With H > 0 the core's matrix and V sit in shared memory and a Jacobi pair takes 16 lanes
+// (jacobi_svd_lanes: the arithmetic of jacobi_svd), for cores of at most 32 H columns and as many
+// threads as all pairs take up to 64 columns; with H = 0, on the slab with a warp a pair
+// (30,000-point Helmholtz cylinder, ranks 17 to 63: 9.9 ms, 4.9 ms in shared memory).
+__host__ __device__ constexpr int tscore_cta_threads(int H) { return H == 0 ? kTruncThreads : (H == 1 ? 256 : 512); }
+template <typename W, int H>
+__global__ void __launch_bounds__(tscore_cta_threads(H))
+    tscore_cta_kernel(const TsCore* __restrict__ items, int nitems, const W* __restrict__ tri, W* maps, int* ranks,
+                      int* status, double eps, W* scratch, long long slab_elems, int* counter) {
+  extern __shared__ __align__(16) unsigned char tscore_smem[];
   __shared__ RedScratch rs;
-  __shared__ int s_item, s_newk;
-  W* slab = scratch + (size_t)blockIdx.x * slab_elems;
+  __shared__ int s_item, s_newk, s_rot;
+  W* slab = H > 0 ? reinterpret_cast<W*>(tscore_smem) : scratch + (size_t)blockIdx.x * slab_elems;
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
@@ -1281,7 +1347,14 @@ __global__ void __launch_bounds__(kTruncThreads) tscore_cta_kernel(const TsCore*
       Rm[e] = s;
     }
     __syncthreads();
-    const bool conv = jacobi_svd(Rm, Vm, k, rs);
+    bool conv;
+    if constexpr (H > 0) {
+      for (int e = threadIdx.x; e < k * k; e += blockDim.x) Vm[e] = e % (k + 1) == 0 ? one<W>() : zero<W>();
+      __syncthreads();
+      conv = jacobi_svd_lanes<kDenseJacobiLanes, H>(Rm, Vm, k, &s_rot);
+    } else {
+      conv = jacobi_svd(Rm, Vm, k, rs);
+    }
     for (int j = threadIdx.x; j < k; j += blockDim.x) {
       double s2 = 0.0;
       for (int i = 0; i < k; ++i) s2 += abs2(Rm[i + (size_t)j * k]);
@@ -1597,19 +1670,43 @@ void launch_tsqr_cta(const TsItem* items, int nitems, const T* ws, typename Trai
     tsqr_cta_kernel<W, T><<<g, kTruncThreads, 0, s>>>(items, nitems, ws, tri, scratch, slab, counter);
 }
 template <typename T>
-void launch_tscore_cta(const TsCore* items, int nitems, const typename Traits<T>::wide* tri,
+void launch_tscore_cta(const TsCore* items, int nitems, int kmax, const typename Traits<T>::wide* tri,
                        typename Traits<T>::wide* maps, int* ranks, int* status, double eps,
                        typename Traits<T>::wide* scratch, long long slab, int grid, int* counter, cudaStream_t s) {
   typedef typename Traits<T>::wide W;
-  if (nitems <= 0) {
-    cudaFuncAttributes a;
-    cudaFuncGetAttributes(&a, tscore_cta_kernel<W>);
-    return;
+  const size_t smem = (2 * (size_t)kmax * kmax) * sizeof(W) + (size_t)kmax * (sizeof(double) + sizeof(int));
+  auto run = [&](auto kern, int threads, size_t bytes) {
+    if (nitems <= 0) {
+      cudaFuncAttributes a;
+      cudaFuncGetAttributes(&a, kern);
+      return;
+    }
+    cudaMemsetAsync(counter, 0, sizeof(int), s);
+    int g = grid;
+    if (bytes > 0) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseJacobiSmem);
+      int per_sm = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, bytes) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+      g = persistent_grid(per_sm);
+    }
+    kern<<<g < nitems ? g : nitems, threads, bytes, s>>>(items, nitems, tri, maps, ranks, status, eps, scratch, slab,
+                                                         counter);
+  };
+  if (nitems <= 0) {  // loads every variant
+    run(tscore_cta_kernel<W, 0>, 0, 0);
+    run(tscore_cta_kernel<W, 1>, 0, 0);
+    run(tscore_cta_kernel<W, 2>, 0, 0);
+    run(tscore_cta_kernel<W, 3>, 0, 0);
+  } else if (kmax > 96 || smem > kDenseJacobiSmem) {
+    run(tscore_cta_kernel<W, 0>, tscore_cta_threads(0), 0);
+  } else if (kmax > 64) {
+    run(tscore_cta_kernel<W, 3>, tscore_cta_threads(3), smem);
+  } else if (kmax > 32) {
+    run(tscore_cta_kernel<W, 2>, tscore_cta_threads(2), smem);
+  } else {
+    run(tscore_cta_kernel<W, 1>, tscore_cta_threads(1), smem);
   }
-  cudaMemsetAsync(counter, 0, sizeof(int), s);
-  const int g = grid < nitems ? grid : nitems;
-  tscore_cta_kernel<W><<<g, kTruncThreads, 0, s>>>(items, nitems, tri, maps, ranks, status, eps, scratch, slab,
-                                                   counter);
 }
 template <typename T>
 void launch_tsapply_cta(const TsItem* items, int nitems, T* ws, const typename Traits<T>::wide* maps,
@@ -1650,7 +1747,7 @@ void preload_truncate_kernels() {
     launch_tsapply<T>(K, nullptr, 0, nullptr, nullptr, nullptr, 0);
   }
   launch_tsqr_cta<T>(nullptr, 0, nullptr, nullptr, false, nullptr, 0, 0, nullptr, 0);
-  launch_tscore_cta<T>(nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0.0, nullptr, 0, 0, nullptr, 0);
+  launch_tscore_cta<T>(nullptr, 0, 0, nullptr, nullptr, nullptr, nullptr, 0.0, nullptr, 0, 0, nullptr, 0);
   launch_tsapply_cta<T>(nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0, 0, nullptr, 0);
 }
 
@@ -1668,7 +1765,7 @@ void preload_truncate_kernels() {
   template void preload_truncate_kernels<T>();                                                            \
   template void launch_tsqr_cta<T>(const TsItem*, int, const T*, typename Traits<T>::wide*, bool,            \
                                    typename Traits<T>::wide*, long long, int, int*, cudaStream_t);         \
-  template void launch_tscore_cta<T>(const TsCore*, int, const typename Traits<T>::wide*,                    \
+  template void launch_tscore_cta<T>(const TsCore*, int, int, const typename Traits<T>::wide*,                    \
                                      typename Traits<T>::wide*, int*, int*, double, typename Traits<T>::wide*, \
                                      long long, int, int*, cudaStream_t);                                  \
   template void launch_tsapply_cta<T>(const TsItem*, int, T*, const typename Traits<T>::wide*, const int*,   \

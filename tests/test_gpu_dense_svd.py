@@ -64,3 +64,38 @@ def test_dense_svd_blocks(hb, vt, n, leaf, leaf_cols, min_leaf):
                 assert np.linalg.norm(got - M, 2) <= (eps + 1e-5) * s[0]
     finally:
         h.close()
+
+
+@pytest.mark.parametrize("vt,eps", [(1, 1e-5), (1, 1e-7), (1, 1e-9), (3, 1e-4), (3, 1e-6)])
+def test_high_rank_cores(hb, vt, eps):
+    """Ranks above the register buckets, whose cores are diagonalised in shared memory (up to 32, 64
+    and 96 columns) or on the slab: the factors come out as U sqrt(S), V sqrt(S) with the singular
+    values in order, and the block is within the tolerance of the kernel's."""
+    pts = np.random.default_rng(5).random((2500, 3))
+    k = hb.kernel(hb.HELMHOLTZ_REG, delta=0.01, wavenumber=5.0) if vt >= 2 else hb.kernel(hb.EXP_COV, ell=0.3,
+                                                                                        nugget=1e-6)
+    hb.set_parameters(compressionMinLeafSize=0)
+    h = hb.HMatrix(pts, k, value_type=vt, leaf_size=110, eta=4.0, epsilon=eps)
+    try:
+        T = h.leaf_table()
+        pr = h.perm()
+        rk = [i for i in range(len(T)) if T[i, 4] == 1 and T[i, 5] > 0]
+        rk.sort(key=lambda i: -T[i, 5])
+        assert T[rk[0], 5] > (16 if vt >= 2 else 32)
+        for i in rk[:: max(1, len(rk) // 25)]:
+            r0, m, c0, nn, _, r = T[i]
+            p = h.leaf_payload(i)
+            A, B = p[:r * m].reshape(r, m).T, p[r * m:].reshape(r, nn).T
+            # U sqrt(S): orthogonal columns of norm sqrt(sigma_j), the same for A and B.  A column
+            # is formed as A M with errors of order k u sigma_0 / sqrt(sigma_j), sigma_j > eps sigma_0
+            ga, gb = A.conj().T @ A, B.conj().T @ B
+            s = np.real(np.diag(ga))
+            tol = 64.0 * 2.0 ** -53 / eps * s[0] + 1e-12 * s[0]
+            assert np.all(np.diff(s) <= tol) and np.all(s > 0.5 * eps * s[0])
+            assert np.abs(ga - np.diag(s)).max() <= tol and np.abs(gb - np.diag(s)).max() <= tol
+            rows, cols = pr[r0:r0 + m], pr[c0:c0 + nn]
+            M = kernel_matrix(vt, pts[rows], pts[cols], rows, cols)
+            # ACA's own stopping estimate and the truncation, each at eps
+            assert np.linalg.norm(A @ B.T - M) <= 50.0 * eps * np.linalg.norm(M)
+    finally:
+        h.close()
