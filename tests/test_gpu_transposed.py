@@ -1,4 +1,4 @@
-"""Transposed and adjoint products ('T', 'C') against the stored leaves multiplied out in FP64:
+"""Products ('N', 'T', 'C') against the stored leaves multiplied out in FP64:
 block heights at the edges of the kernels' tiles (one row, odd, 64, 128, leaves cut into several
 blocks), row and column trees of different leaf sizes, ranks above the first height class, every
 right-hand-side tile and more than one, every type."""
@@ -33,8 +33,8 @@ def test_transposed_products(hb, vt, n, leaf, leaf_cols, eta, eps):
         for i, (r0, m, c0, nn, _, _) in enumerate(T):
             H[np.ix_(pr[r0:r0 + m], pc[c0:c0 + nn])] = h.leaf_block(i)
         rng = np.random.default_rng(1)
-        for trans in "TC" if vt >= 2 else "T":
-            op = H.T if trans == "T" else H.conj().T
+        for trans in "NTC" if vt >= 2 else "NT":
+            op = {"N": H, "T": H.T, "C": H.conj().T}[trans]
             for nrhs in (1, 2, 4, 5, 8, 11, 16, 21):
                 x = rng.standard_normal((n, nrhs)) + (1j * rng.standard_normal((n, nrhs)) if vt >= 2 else 0.0)
                 x = x.astype(h.dtype)
