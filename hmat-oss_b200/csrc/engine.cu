@@ -1931,7 +1931,7 @@ class Engine : public EngineBase {
     const int RS16 = gemv_rhs_stride((int)sizeof(T), Rmax);
     const int wpc = warp_stream_warps_per_cta();
     const int nt = (int)tasks.size();
-    const int cta = std::max(1, std::min((nt + wpc - 1) / wpc, launch_ctas(omax, map)));
+    const int cta = std::max(1, std::min(nt, launch_ctas(omax, map)));  // few tasks: one a CTA, over all SMs
     *ncta = cta;
     const int G = cta * wpc;
     std::vector<double> cost(tasks.size());
@@ -1953,6 +1953,28 @@ class Engine : public EngineBase {
     }
     for (; g < G; ++g) begin[g] = (int)tasks.size();
     begin[G] = (int)tasks.size();
+    return begin;
+  }
+
+  // Warps that share the n units of the 'N' y-phase: all of the grid's `most`, unless that leaves a
+  // warp fewer than kTaskUnits units.  A warp's pieces come in one after the other, but every task
+  // writes its rows and the final pass adds a block's one after the other (3,000-point cylinder,
+  // FP64, 8 right-hand sides: 73 us with a task a warp, 59, 57, 53 and 57 us with at least 2, 3, 4
+  // and 9 units).  The transposed products' group pass, with several times the outputs, is fastest
+  // with every warp at work.
+  static constexpr int kTaskUnits = 4;
+  static int task_warps(int n, int most) { return std::max(1, std::min(most, n / kTaskUnits)); }
+
+  // Ranges of tasks (their starts and the end), one a warp, laid out over as many CTAs of wpc warps as
+  // there are ranges, at most max_cta: few ranges go to different SMs.
+  static std::vector<int> spread_ranges(const std::vector<int>& starts, int max_cta, int wpc, int* ncta) {
+    const int n = (int)starts.size() - 1;
+    *ncta = std::min(n, max_cta);
+    std::vector<int> begin((size_t)*ncta * wpc + 1, starts[n]);
+    for (int b = 0; b < *ncta; ++b) {
+      const int r0 = (int)((long long)n * b / *ncta), r1 = (int)((long long)n * (b + 1) / *ncta);
+      for (int w = 0; w < wpc; ++w) begin[(size_t)b * wpc + w] = starts[std::min(r0 + w, r1)];
+    }
     return begin;
   }
 
@@ -1986,8 +2008,8 @@ class Engine : public EngineBase {
     std::vector<int2> yrows;
   };
 
-  // With `begin` given (one range of tasks per warp, or per CTA for map 4, of the full persistent
-  // grid), the ranges are taken as they are instead of being cut by cost here.
+  // With `begin` given (one range of tasks per warp, or per CTA for map 4), the ranges are taken as
+  // they are instead of being cut by cost here.
   static void finish_launch(GemvLaunch& L, SidePlan& sp, int slot, std::vector<GemvTask>& tasks,
                             std::vector<int>* begin_given = nullptr) {
     const std::vector<GemvUnit>& units = sp.units;
@@ -2038,9 +2060,10 @@ class Engine : public EngineBase {
     std::vector<int> begin;
     if (begin_given) {
       const int wpc = L.map != 4 ? warp_stream_warps_per_cta() : 1;
-      L.ncta = launch_ctas(omax, L.map);
       begin.swap(*begin_given);
-      if ((int)begin.size() != L.ncta * wpc + 1 || begin.front() != 0 || begin.back() != (int)tasks.size())
+      L.ncta = ((int)begin.size() - 1) / wpc;
+      if (L.ncta < 1 || L.ncta > launch_ctas(omax, L.map) || (int)begin.size() != L.ncta * wpc + 1 || begin.front() != 0 ||
+          begin.back() != (int)tasks.size())
         throw Error("gemv plan: task ranges do not match the launch grid");
     } else {
       begin = partition(tasks, units, omax, L.map, &L.ncta);
@@ -2050,8 +2073,9 @@ class Engine : public EngineBase {
   }
 
   // The 'N' side (host work only: it may run beside build_trans_side).
+  // bound_rows: see noalloc_trans_rows.
   void build_side(const std::vector<GemvRkLeaf>& K, const std::vector<int>& rk_leaf, long long& next_row,
-                  GemvSide& side, SidePlan& sp) const {
+                  long long& bound_rows, GemvSide& side, SidePlan& sp) const {
     const auto& L = bt_->leaves;
     const std::vector<Block>& oblocks = rblocks_;
     std::vector<GemvUnit>& units = sp.units;
@@ -2066,6 +2090,8 @@ class Engine : public EngineBase {
     std::vector<GemvTask> zt[4];
     std::vector<GemvZred>& zred = sp.zred;
     const auto& G = layout_.zgroups;
+    bound_rows = next_row;
+    const int bound_units = gemv_tuned ? kMaxUnits : 16;
     // one launch takes every height up to 32; the tensor-core kernel takes every height up to 64
     // in one (its tile count is a per-task constant), so one wave covers them
     auto z_class = [](int O) { return kTensorN && O <= 64 ? 2 : std::max(1, rank_class(O)); };
@@ -2091,6 +2117,7 @@ class Engine : public EngineBase {
         const int O = g.h, zrow = zgroup_row_[0][t], first = (int)units.size();
         px_units(units, g.base, g.h, g.n, g.col_off, zc, xoff);
         const int nu = (int)units.size() - first;
+        if (nu > bound_units) bound_rows += (long long)((nu + bound_units - 1) / bound_units) * O;
         if (nu <= kMaxUnits) {
           zt[cls].push_back(GemvTask{O, first, nu, zrow});
           continue;
@@ -2203,31 +2230,44 @@ class Engine : public EngineBase {
       if (tc_y) probe.map = 4;
       else warp_shape(probe, maxlen);
       const int wpc = probe.map == 4 ? 1 : warp_stream_warps_per_cta();
-      const int G = launch_ctas(probe.map == 3 ? 8 * probe.rpt : maxlen, probe.map) * wpc;
+      const int max_cta = launch_ctas(probe.map == 3 ? 8 * probe.rpt : maxlen, probe.map);
       const int nyu = (int)units.size() - first_y;
       std::vector<double> cum(nyu + 1, 0.0);
       for (int v = 0; v < nyu; ++v) {
         const GemvUnit& u = units[first_y + v];
         cum[v + 1] = cum[v] + (double)u.pel + (double)u.c * RS16 + 64;
       }
-      const double tot = std::max(cum[nyu], 1.0);
-      ybegin.assign(G + 1, 0);
-      int w = 0;
-      std::vector<int> task_block;
-      for (int v = 0; v < nyu;) {
-        // the warp of unit v: the last w with cum[v] >= tot * w / G
-        while (w + 1 < G && cum[v] >= tot * (w + 1) / G) {
-          ++w;
-          ybegin[w] = (int)yt.size();
+      std::vector<int> task_block, starts;
+      // the tasks of G ranges of equal cost, split at block boundaries: task(v, v1) for each, and
+      // the first task of every range
+      auto cut = [&](int G, std::vector<int>& at, auto task) {
+        const double tot = std::max(cum[nyu], 1.0);
+        at.assign(G + 1, 0);
+        int w = 0, nt = 0;
+        for (int v = 0; v < nyu;) {
+          // the range of unit v: the last w with cum[v] >= tot * w / G
+          while (w + 1 < G && cum[v] >= tot * (w + 1) / G) at[++w] = nt;
+          const double wend = w + 1 < G ? tot * (w + 1) / G : 1e300;
+          int v1 = v + 1;
+          while (v1 < nyu && ublock[v1] == ublock[v] && cum[v1] < wend) ++v1;
+          task(v, v1);
+          ++nt;
+          v = v1;
         }
-        const double wend = w + 1 < G ? tot * (w + 1) / G : 1e300;
-        int v1 = v + 1;
-        while (v1 < nyu && ublock[v1] == ublock[v] && cum[v1] < wend) ++v1;
+        for (++w; w <= G; ++w) at[w] = nt;
+      };
+      const int G = tc_y ? max_cta : task_warps(nyu, max_cta * wpc);
+      cut(G, starts, [&](int v, int v1) {
         yt.push_back(GemvTask{oblocks[ublock[v]].len, first_y + v, v1 - v, 0});
         task_block.push_back(ublock[v]);
-        v = v1;
-      }
-      for (++w; w <= G; ++w) ybegin[w] = (int)yt.size();
+      });
+      int ncta = 0;
+      ybegin = spread_ranges(starts, max_cta, wpc, &ncta);
+      // rows the allocation-free products are bounded by: a task a warp of the full grid
+      if (G == max_cta * wpc)
+        for (const GemvTask& t : yt) bound_rows += t.O;
+      else
+        cut(max_cta * wpc, starts, [&](int v, int) { bound_rows += oblocks[ublock[v]].len; });
       // partial-row slots: the tasks of a block (consecutive) take consecutive slots
       std::vector<int> nparts(oblocks.size(), 0), part_row(oblocks.size(), 0);
       for (size_t t = 0; t < yt.size(); ++t) {
@@ -2392,10 +2432,10 @@ class Engine : public EngineBase {
       l = GemvLaunch();
       l.piece_bytes = piece;
       l.xrows = hmax;
-      l.ncta = trans_ctas(trans_groups_smem(piece, hmax, RS16 * s));
-      const int wpc = trans_warps_per_cta();
-      l.ncta = std::max(1, std::min(l.ncta, ((int)owner.size() + wpc - 1) / wpc));
-      cut_tasks(units, first, owner, l.ncta * wpc, gt[side.ng], gstrip[side.ng], gbegin[side.ng]);
+      const int max_cta = trans_ctas(trans_groups_smem(piece, hmax, RS16 * s)), wpc = trans_warps_per_cta();
+      std::vector<int> starts;
+      cut_tasks(units, first, owner, std::min((int)owner.size(), max_cta * wpc), gt[side.ng], gstrip[side.ng], starts);
+      gbegin[side.ng] = spread_ranges(starts, max_cta, wpc, &l.ncta);
       for (int st : gstrip[side.ng]) nparts[st]++;
       side.ng++;
     }
@@ -2499,9 +2539,7 @@ class Engine : public EngineBase {
       l.piece_bytes = stage;
       l.xrows = omax;
       // x rows padded by 16 bytes where the kernel pads them
-      l.ncta = trans_ctas(trans_columns_smem(stage, omax, RS16 * s + 16));
-      const int wpc = trans_warps_per_cta();
-      l.ncta = std::max(1, std::min(l.ncta, ((int)owner.size() + wpc - 1) / wpc));
+      l.ncta = std::min((int)owner.size(), trans_ctas(trans_columns_smem(stage, omax, RS16 * s + 16)));
       std::vector<GemvTask> ct;
       std::vector<int> cblock, cbegin;
       cut_tasks(units, first, owner, l.ncta, ct, cblock, cbegin);
@@ -2588,13 +2626,14 @@ class Engine : public EngineBase {
     plan_.rk = g_rk_.p;
     plan_.nfull = (int)F.size();
     plan_.nrk = (int)K.size();
+    long long bound_rows = 0;
     {
       SidePlan sp[2];
       std::future<void> trans;
       if (!only_n)
         trans = std::async(std::launch::async,
                            [&] { build_trans_side(K, rk_leaf, next_row[1], plan_.side[1], sp[1]); });
-      build_side(K, rk_leaf, next_row[0], plan_.side[0], sp[0]);
+      build_side(K, rk_leaf, next_row[0], bound_rows, plan_.side[0], sp[0]);
       if (!only_n) trans.get();
       upload_side(sp[0], plan_.side[0], side_buf_[0]);
       if (!only_n) upload_side(sp[1], plan_.side[1], side_buf_[1]);
@@ -2608,13 +2647,14 @@ class Engine : public EngineBase {
     }
     for (int side = 0; side < 2; ++side)
       if (plan_.xz_rows[side] >= (1LL << 31)) throw Error("gemv plan: z buffer too large");
-    noalloc_rows_ = next_row[0] + noalloc_trans_rows(K);
+    noalloc_rows_ = bound_rows + noalloc_trans_rows(K);
   }
 
   // The bound of the allocation-free products is stated in rows of one buffer for both
-  // directions, with the partial rows of transposed products that took a slot per 16 units of 32
-  // columns: callers know which matrices it takes, so it stays, although a transposed product now
-  // uses its scratch differently (gemv_device_with_scratch).
+  // directions, with z chunks of 16 units (the tuner's, of a tuned matrix), a part of y per warp of
+  // the full grid, and the partial rows of transposed products that took a slot per 16 units of 32
+  // columns: callers know which matrices it takes, so it stays, although the products now use
+  // their scratch differently (gemv_device_with_scratch).
   long long noalloc_trans_rows(const std::vector<GemvRkLeaf>& K) const {
     const auto& L = bt_->leaves;
     const long long kUnits = 16;
@@ -2684,6 +2724,25 @@ class Engine : public EngineBase {
     *yms = b;
   }
 
+  // Chunk size of the z tasks of a matrix too small to tune: as many units as give every warp of
+  // the z launch about one chunk, 16 at most (one right-hand side, 8,000-point cylinder, FP64: 43 us
+  // with chunks of 16 units, 35 with the 2 this gives; 15,000 points, FP32, 16 right-hand sides: 66
+  // -> 53 us; 5,000-point Helmholtz cylinder, complex FP32, four: 53 -> 42 us).
+  int small_zparts() const {
+    long long units = 0;
+    int omax = 1;
+    for (const ZGroup& g : layout_.zgroups) {
+      int xoff = 0;
+      const int zc = kTensorN ? mma_unit_cols(g.h, &xoff) : warp_unit_cols_wide(g.h, &xoff);
+      units += (g.n + zc - 1) / zc;
+      omax = std::max(omax, g.h);
+    }
+    GemvLaunch l;
+    warp_shape(l, omax);
+    const long long warps = (long long)launch_ctas(l.map == 3 ? 8 * l.rpt : omax, l.map) * warp_stream_warps_per_cta();
+    return (int)std::max(1LL, std::min(16LL, (units + warps - 1) / warps));
+  }
+
   // Builds the products' schedules, with the tuner's choice for the matrix's class.
   void plan_products() {
     gemv_tuned = 0;
@@ -2694,6 +2753,7 @@ class Engine : public EngineBase {
     const int mode = gemv_tuning_mode();
     const long long bytes = layout_.total * (long long)sizeof(T);
     if (mode == 0 || (mode == 1 && bytes < (64LL << 20))) {
+      if (mode == 1) gemv_choice[0] = tune_zparts_ = small_zparts();
       build_plan();
       return;
     }
@@ -2714,6 +2774,7 @@ class Engine : public EngineBase {
         return;
       }
     }
+    gemv_tuned = 1;
     static const int kZparts[3] = {8, 16, 32};
     double best_z = 1e300;
     int zp = 16;
