@@ -1931,7 +1931,7 @@ class Engine : public EngineBase {
     const int RS16 = gemv_rhs_stride((int)sizeof(T), Rmax);
     const int wpc = warp_stream_warps_per_cta();
     const int nt = (int)tasks.size();
-    const int cta = std::max(1, std::min(nt, launch_ctas(omax, map)));  // few tasks: one a CTA, over all SMs
+    const int cta = spread_ctas(nt, launch_ctas(omax, map), wpc);
     *ncta = cta;
     const int G = cta * wpc;
     std::vector<double> cost(tasks.size());
@@ -1965,11 +1965,18 @@ class Engine : public EngineBase {
   static constexpr int kTaskUnits = 4;
   static int task_warps(int n, int most) { return std::max(1, std::min(most, n / kTaskUnits)); }
 
-  // Ranges of tasks (their starts and the end), one a warp, laid out over as many CTAs of wpc warps as
-  // there are ranges, at most max_cta: few ranges go to different SMs.
+  // CTAs of wpc warps for n ranges of work: full ones, but one per SM at least while there are
+  // ranges for them, and max_cta at most.  (A CTA a range up to max_cta leaves less room to the
+  // products of other streams: 50,000-point Helmholtz cylinder, three matrices in turn, 260 us a
+  // product against 254.)
+  static int spread_ctas(int n, int max_cta, int wpc) {
+    return std::max(1, std::min(max_cta, std::max((n + wpc - 1) / wpc, std::min(n, persistent_grid(1)))));
+  }
+
+  // Ranges of tasks (their starts and the end), one a warp, laid out over a grid's warps.
   static std::vector<int> spread_ranges(const std::vector<int>& starts, int max_cta, int wpc, int* ncta) {
     const int n = (int)starts.size() - 1;
-    *ncta = std::min(n, max_cta);
+    *ncta = spread_ctas(n, max_cta, wpc);
     std::vector<int> begin((size_t)*ncta * wpc + 1, starts[n]);
     for (int b = 0; b < *ncta; ++b) {
       const int r0 = (int)((long long)n * b / *ncta), r1 = (int)((long long)n * (b + 1) / *ncta);
