@@ -1337,15 +1337,18 @@ class Engine : public EngineBase {
                       const std::vector<int>& h_status, std::vector<int>& h_ranks, double eps,
                       const RkLeafDesc* d_desc, T* d_ws, int* d_ranks, int* d_status, int* d_counter) {
     typedef typename Traits<T>::wide W;
-    std::vector<int> small, large;
-    int sm = 1, sn = 1, lm = 1, ln = 1, lk = 1;
+    // the shared-memory kernel's blocks by their columns (at most 32, 64, more): a launch holds as
+    // many CTAs an SM as its largest block leaves room for
+    std::vector<int> small[3], large;
+    int sm[3] = {1, 1, 1}, sn[3] = {1, 1, 1}, lm = 1, ln = 1, lk = 1;
     for (int b = 0; b < (int)jobs.size(); ++b) {
       if (!jobs[b].svd || jobs[b].pass || h_status[b] != kLeafOk || h_ranks[b] <= 0) continue;
       const int m = desc[b].m, n = desc[b].n;
       if (dense_svd_fits<T>(m, n)) {
-        small.push_back(b);
-        sm = std::max(sm, std::min(m, n));
-        sn = std::max(sn, std::max(m, n));
+        const int k = std::min(m, n), c = k <= 32 ? 0 : (k <= 64 ? 1 : 2);
+        small[c].push_back(b);
+        sm[c] = std::max(sm[c], k);
+        sn[c] = std::max(sn[c], std::max(m, n));
       } else {
         large.push_back(b);
         lm = std::max(lm, m);
@@ -1353,21 +1356,22 @@ class Engine : public EngineBase {
         lk = std::max(lk, h_ranks[b]);
       }
     }
-    if (small.empty() && large.empty()) return;
+    if (small[0].empty() && small[1].empty() && small[2].empty() && large.empty()) return;
     auto cost = [&](int b) { return (double)(desc[b].m + desc[b].n) * h_ranks[b] * h_ranks[b]; };
-    by_decreasing(small, cost);
+    for (auto& v : small) by_decreasing(v, cost);
     by_decreasing(large, cost);
-    DevArray<int> d_small, d_large;
+    DevArray<int> d_small[3], d_large;
     DevArray<W> d_scratch;
-    d_small.upload(small, stream_);
+    for (int c = 0; c < 3; ++c) d_small[c].upload(small[c], stream_);
     d_large.upload(large, stream_);
     long long slab = 0, grid = 0;
     if (!large.empty()) grid = alloc_slabs(d_scratch, lm, ln, lk, large.size(), &slab);
     HB_CUDA(cudaStreamSynchronize(stream_));
     HB_CUDA(cudaEventRecord(ev_[4], stream_));
-    if (!small.empty())
-      HB_CUDA(launch_dense_svd<T>(d_desc, d_small.p, (int)small.size(), sm, sn, eps, d_ws, d_ranks, d_status, d_counter,
-                                  stream_));
+    for (int c = 2; c >= 0; --c)  // the longest blocks first
+      if (!small[c].empty())
+        HB_CUDA(launch_dense_svd<T>(d_desc, d_small[c].p, (int)small[c].size(), sm[c], sn[c], eps, d_ws, d_ranks, d_status,
+                                    d_counter, stream_));
     if (!large.empty()) {
       HB_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(int), stream_));
       launch_truncate<T>(d_desc, d_large.p, (int)large.size(), eps, d_ws, d_ranks, d_status, d_counter, d_scratch.p,

@@ -1050,17 +1050,25 @@ __global__ void __launch_bounds__(kDenseSvdThreads) dense_svd_kernel(const RkLea
 //
 // The block, the rotated matrix and V sit in shared memory, and what the identity factor adds is
 // known: its QR is R = -I and its Q negates.  A Jacobi pair takes 16 lanes, two pairs a warp, all
-// pairs of 64 columns in one pass of 512 threads: the scalar chain of a rotation (square roots and
-// divides, about 170 dependent FP64 operations) bounds a round, a warp runs it for two pairs at
-// once, and the other warps' loads and sums hide behind it.  The lanes add their elements in the
+// pairs of 64 columns in one pass of 512 threads, in a kernel for columns of up to 32, 64 and 96:
+// bound by the instructions of its rounds (dozens of sweeps: pairs of columns near rounding level
+// keep passing the 1e-15 test) and the barrier between them.  The lanes add their elements in the
 // order of a warp's sum over lanes 0 .. 31: chains over v, v + 32, ... for the virtual lanes
 // v = l + 16 c, then (v, v + 16), (v, v + 8), ... .
 //
 // 8,000-point cylinder (leaf 64, epsilon 1e-4, FP64), default compressionMinLeafSize, 1,048 blocks
-// of up to 63 x 63: truncation 37.8 ms with every block on the slab kernel, 15.7 ms here (4 lanes
-// a pair 22.1 ms, 8 lanes 17.6 ms).
-constexpr int kDenseJacobiLanes = 16;                        // lanes a pair
-constexpr int kDenseJacobiThreads = 32 * kDenseJacobiLanes;  // all pairs of 64 columns at once
+// of up to 63 x 63: truncation 37.8 ms with every block on the slab kernel, 13.7 ms here (4 lanes
+// a pair 22 ms, 8 lanes 14.7 ms; 15.7 ms with one kernel for all widths and a modulo per pair).
+// Lanes a pair (complex: half, whose elements and products are twice the work of a lane).
+template <typename W>
+__host__ __device__ constexpr int jacobi_lanes() {
+  return std::is_same<W, double>::value ? 16 : 8;
+}
+// Threads for columns of at most 32 H: all pairs of 32 columns at once, or of 64 columns.
+template <typename W>
+__host__ __device__ constexpr int jacobi_threads(int H) {
+  return (H == 1 ? 16 : 32) * jacobi_lanes<W>();
+}
 constexpr int kDenseJacobiChain = 3;  // elements of a chain: columns of at most 96
 constexpr size_t kDenseJacobiSmem = 216 * 1024;
 
@@ -1107,6 +1115,22 @@ __device__ __forceinline__ V lanes_sum(const V (&v)[32 / L]) {
   return s;
 }
 
+// jacobi_svd's test of a pair, !(ag == 0 || ag <= 1e-15 sqrt(al be)) with ag = sqrt(g2), decided on
+// the squares unless they are within a billionth of the threshold or out of the normal range:
+// most pairs of the later sweeps do not rotate, and two square roots are most of their time.
+__device__ __forceinline__ bool jacobi_rotates(double g2, double albe) {
+  const double lim = 1e-30 * albe;
+  if (lim > 1e-280) {
+    if (g2 < lim * (1.0 - 1e-9)) return false;
+    if (g2 > lim * (1.0 + 1e-9) && g2 < 1e300) return true;
+  }
+  const double ag = sqrt(g2);
+  return !(ag == 0.0 || ag <= 1e-15 * sqrt(albe));
+}
+// sqrt(|g|^2); for a real g it is |g| itself, exactly, unless the square left the normal range.
+__device__ __forceinline__ double abs_of(double g, double g2) { return g2 > 1e-290 && g2 < 1e300 ? fabs(g) : sqrt(g2); }
+__device__ __forceinline__ double abs_of(cdouble, double g2) { return sqrt(g2); }
+
 // jacobi_svd with L lanes a pair, columns of at most 32 H; Wm and V in shared memory.
 template <int L, int H, typename W>
 __device__ bool jacobi_svd_lanes(W* Wm, W* V, int k, int* s_rot) {
@@ -1120,8 +1144,11 @@ __device__ bool jacobi_svd_lanes(W* Wm, W* V, int k, int* s_rot) {
     for (int round = 0; round < kk - 1; ++round) {
       for (int pr0 = 0; pr0 < kk / 2; pr0 += ngrp) {  // block-uniform: every lane joins the shuffles
         const int pr = pr0 + grp;
-        const int a = pr == 0 ? 0 : 1 + (pr - 1 + round) % (kk - 1);
-        const int b = 1 + (kk - 2 - pr + round) % (kk - 1);
+        // 1 + (pr - 1 + round) mod (kk - 1) and 1 + (kk - 2 - pr + round) mod (kk - 1): both sums
+        // are below 2 (kk - 1) for the live pairs
+        const int ra = pr - 1 + round, rb = kk - 2 - pr + round;
+        const int a = pr == 0 ? 0 : 1 + (ra >= kk - 1 ? ra - (kk - 1) : ra);
+        const int b = 1 + (rb >= kk - 1 ? rb - (kk - 1) : rb);
         const int p = min(a, b), q = max(a, b);
         const bool live = pr < kk / 2 && q < k;
         W* wp = Wm + (size_t)(live ? p : 0) * k;
@@ -1145,9 +1172,10 @@ __device__ bool jacobi_svd_lanes(W* Wm, W* V, int k, int* s_rot) {
         }
         const double al = lanes_sum<L>(alc), be = lanes_sum<L>(bec);
         const W g = lanes_sum<L>(gc);
-        const double ag = sqrt(abs2(g));
-        if (!live || ag == 0.0 || ag <= 1e-15 * sqrt(al * be)) continue;
+        const double g2 = abs2(g);
+        if (!live || !jacobi_rotates(g2, al * be)) continue;
         if (l == 0) *s_rot = 1;
+        const double ag = abs_of(g, g2);
         const W phc = conjg(scal(1.0 / ag, g));
         const double zeta = __dsub_rn(be, al) / __dmul_rn(2.0, ag);
         const double t = (zeta >= 0.0 ? 1.0 : -1.0) / __dadd_rn(fabs(zeta), sqrt(fma(zeta, zeta, 1.0)));
@@ -1179,8 +1207,8 @@ __device__ bool jacobi_svd_lanes(W* Wm, W* V, int k, int* s_rot) {
   return false;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kDenseJacobiThreads, 2) dense_jacobi_kernel(const RkLeafDesc* __restrict__ leaves,
+template <typename T, int H>
+__global__ void __launch_bounds__(jacobi_threads<double>(H), 2) dense_jacobi_kernel(const RkLeafDesc* __restrict__ leaves,
                                                                             const int* __restrict__ order,
                                                                             int nleaves, double eps, T* ws,
                                                                             int* ranks, int* status, int* counter) {
@@ -1220,7 +1248,7 @@ __global__ void __launch_bounds__(kDenseJacobiThreads, 2) dense_jacobi_kernel(co
     __syncthreads();
     for (int e = tid; e < k * k; e += blockDim.x) Vm[e] = e % (k + 1) == 0 ? 1.0 : 0.0;
     __syncthreads();
-    const bool conv = jacobi_svd_lanes<kDenseJacobiLanes, kDenseJacobiChain>(Rm, Vm, k, &s_rot);
+    const bool conv = jacobi_svd_lanes<jacobi_lanes<double>(), H>(Rm, Vm, k, &s_rot);
     for (int j = tid; j < k; j += blockDim.x) {
       double s2 = 0.0;
       for (int i = 0; i < k; ++i) s2 += abs2(Rm[i + (size_t)j * k]);
@@ -1314,12 +1342,15 @@ __global__ void __launch_bounds__(kTruncThreads) tsqr_cta_kernel(const TsItem* _
 // Core of one leaf: Ra Rb^T, Jacobi, sigma order, k', and the maps (k x k, ld k, columns at
 // or past k' zero), as tscore_kernel.
 // With H > 0 the core's matrix and V sit in shared memory and a Jacobi pair takes 16 lanes
-// (jacobi_svd_lanes: the arithmetic of jacobi_svd), for cores of at most 32 H columns and as many
-// threads as all pairs take up to 64 columns; with H = 0, on the slab with a warp a pair
+// (8 of them complex; jacobi_svd_lanes: the arithmetic of jacobi_svd), for cores of at most 32 H
+// columns and as many threads as all pairs take up to 64 columns; with H = 0, on the slab with a warp a pair
 // (30,000-point Helmholtz cylinder, ranks 17 to 63: 9.9 ms, 4.9 ms in shared memory).
-__host__ __device__ constexpr int tscore_cta_threads(int H) { return H == 0 ? kTruncThreads : (H == 1 ? 256 : 512); }
+template <typename W>
+__host__ __device__ constexpr int tscore_cta_threads(int H) {
+  return H == 0 ? kTruncThreads : jacobi_threads<W>(H);
+}
 template <typename W, int H>
-__global__ void __launch_bounds__(tscore_cta_threads(H))
+__global__ void __launch_bounds__(tscore_cta_threads<W>(H))
     tscore_cta_kernel(const TsCore* __restrict__ items, int nitems, const W* __restrict__ tri, W* maps, int* ranks,
                       int* status, double eps, W* scratch, long long slab_elems, int* counter) {
   extern __shared__ __align__(16) unsigned char tscore_smem[];
@@ -1351,7 +1382,7 @@ __global__ void __launch_bounds__(tscore_cta_threads(H))
     if constexpr (H > 0) {
       for (int e = threadIdx.x; e < k * k; e += blockDim.x) Vm[e] = e % (k + 1) == 0 ? one<W>() : zero<W>();
       __syncthreads();
-      conv = jacobi_svd_lanes<kDenseJacobiLanes, H>(Rm, Vm, k, &s_rot);
+      conv = jacobi_svd_lanes<jacobi_lanes<W>(), H>(Rm, Vm, k, &s_rot);
     } else {
       conv = jacobi_svd(Rm, Vm, k, rs);
     }
@@ -1491,10 +1522,19 @@ cudaError_t launch_dense_svd(const RkLeafDesc* d_leaves, const int* d_order, int
                                                           counter);
     return cudaGetLastError();
   };
-  if constexpr (Traits<T>::is_complex)
+  if constexpr (Traits<T>::is_complex) {
     return run(dense_svd_kernel<T>, kDenseSvdThreads, (size_t)dense_svd_ld(len) * k * sizeof(cdouble), kDenseSvdSmem);
-  else
-    return run(dense_jacobi_kernel<T>, kDenseJacobiThreads, dense_jacobi_smem(len, k), kDenseJacobiSmem);
+  } else {
+    const size_t smem = dense_jacobi_smem(len, k);
+    if (nleaves <= 0) {  // loads every variant
+      run(dense_jacobi_kernel<T, 1>, 0, 0, 0);
+      run(dense_jacobi_kernel<T, 2>, 0, 0, 0);
+      return run(dense_jacobi_kernel<T, 3>, 0, 0, 0);
+    }
+    if (k <= 32) return run(dense_jacobi_kernel<T, 1>, jacobi_threads<double>(1), smem, kDenseJacobiSmem);
+    if (k <= 64) return run(dense_jacobi_kernel<T, 2>, jacobi_threads<double>(2), smem, kDenseJacobiSmem);
+    return run(dense_jacobi_kernel<T, 3>, jacobi_threads<double>(3), smem, kDenseJacobiSmem);
+  }
 }
 
 template <typename T>
@@ -1699,13 +1739,13 @@ void launch_tscore_cta(const TsCore* items, int nitems, int kmax, const typename
     run(tscore_cta_kernel<W, 2>, 0, 0);
     run(tscore_cta_kernel<W, 3>, 0, 0);
   } else if (kmax > 96 || smem > kDenseJacobiSmem) {
-    run(tscore_cta_kernel<W, 0>, tscore_cta_threads(0), 0);
+    run(tscore_cta_kernel<W, 0>, tscore_cta_threads<W>(0), 0);
   } else if (kmax > 64) {
-    run(tscore_cta_kernel<W, 3>, tscore_cta_threads(3), smem);
+    run(tscore_cta_kernel<W, 3>, tscore_cta_threads<W>(3), smem);
   } else if (kmax > 32) {
-    run(tscore_cta_kernel<W, 2>, tscore_cta_threads(2), smem);
+    run(tscore_cta_kernel<W, 2>, tscore_cta_threads<W>(2), smem);
   } else {
-    run(tscore_cta_kernel<W, 1>, tscore_cta_threads(1), smem);
+    run(tscore_cta_kernel<W, 1>, tscore_cta_threads<W>(1), smem);
   }
 }
 template <typename T>
