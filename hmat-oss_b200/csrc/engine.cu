@@ -1816,17 +1816,9 @@ class Engine : public EngineBase {
     DevArray<GemvTask> tasks[GemvSide::kMaxLaunch + 2];
     DevArray<int> begin[GemvSide::kMaxLaunch + 2];
     DevArray<GemvZred> zred;
-    DevArray<int> zcnt;
     DevArray<int> colmap;
     DevArray<int2> yrows;
   };
-
-  // Whether the z kernels sum the chunks of long groups themselves (the warp finishing a sum's
-  // last chunk adds the parts) instead of a separate pass: the 'N' products in FP64 and complex
-  // (cylinder 100,000, 16 RHS, FP64: z-phase 0.385 -> 0.352 ms).  Not the FP32 tensor-core
-  // z-phase, whose short kernel ends later by the chunks' fences and the last warps' sums than
-  // the separate pass takes (0.134 -> 0.141 ms).
-  static constexpr bool kZsumInKernel = !std::is_same<T, float>::value;
 
   static int rank_class(int k) { return k <= 16 ? 0 : (k <= 32 ? 1 : (k <= 64 ? 2 : 3)); }
   // Columns per unit of a warp-level launch: the piece (O x cols) and its X rows fit one
@@ -2008,6 +2000,16 @@ class Engine : public EngineBase {
     L.rpt = omax <= 32 ? 2 : 4;
   }
 
+  // Sums sorted by decreasing parts; returns how many of them take a CTA of eight warps instead of
+  // one warp (more than kZredWideParts parts).
+  static constexpr int kZredWideParts = 16;
+  static int wide_sums_first(std::vector<GemvZred>& zred) {
+    std::stable_sort(zred.begin(), zred.end(), [](const GemvZred& x, const GemvZred& y) { return x.nparts > y.nparts; });
+    int n = 0;
+    while (n < (int)zred.size() && zred[n].nparts > kZredWideParts) n++;
+    return n;
+  }
+
   // A side's schedule as built on the host, before its upload.
   struct SidePlan {
     std::vector<GemvUnit> units;
@@ -2138,9 +2140,7 @@ class Engine : public EngineBase {
         next_row += (long long)nparts * O;
         for (int pidx = 0; pidx < nparts; ++pidx) {
           const int u0 = pidx * kMaxUnits, u1 = std::min(nu, u0 + kMaxUnits);
-          GemvTask task{O, first + u0, u1 - u0, part_row + pidx * O};
-          if (kZsumInKernel) task.red = (int)zred.size();
-          zt[cls].push_back(task);
+          zt[cls].push_back(GemvTask{O, first + u0, u1 - u0, part_row + pidx * O});
         }
         zred.push_back(GemvZred{zrow, O, part_row, nparts});
       }
@@ -2315,7 +2315,7 @@ class Engine : public EngineBase {
     else
       warp_shape(side.y, maxlen);
     finish_launch(side.y, sp, GemvSide::kMaxLaunch, yt, &ybegin);
-    side.zfused = kZsumInKernel;
+    side.nzwide = wide_sums_first(zred);
   }
 
   // Uploads a side's schedule and points its launches at it.
@@ -2341,9 +2341,6 @@ class Engine : public EngineBase {
     sb.zred.upload(sp.zred, stream_);
     side.nzred = (int)sp.zred.size();
     side.zred = sb.zred.p;
-    sb.zcnt.alloc(std::max<size_t>(sp.zred.size(), 1));
-    HB_CUDA(cudaMemsetAsync(sb.zcnt.p, 0, sb.zcnt.n * sizeof(int), stream_));
-    side.zcnt = sb.zcnt.p;
     sb.yrows.upload(sp.yrows, stream_);
     side.nyrows = (int)sp.yrows.size();
     side.yrows = sb.yrows.p;
@@ -2517,10 +2514,7 @@ class Engine : public EngineBase {
         }
       }
     }
-    // the longest sums first: they take a CTA each
-    std::stable_sort(zred.begin(), zred.end(), [](const GemvZred& x, const GemvZred& y) { return x.nparts > y.nparts; });
-    side.nzwide = 0;
-    while (side.nzwide < (int)zred.size() && zred[side.nzwide].nparts > kZredWideParts) side.nzwide++;
+    side.nzwide = wide_sums_first(zred);
     const int first = (int)units.size();
     std::vector<int> owner;
     int stage = 32, omax = 1;
@@ -2570,10 +2564,7 @@ class Engine : public EngineBase {
     }
     for (int m : colmap)
       if (m < 0 || m >= next_row) throw Error("gemv plan: column map out of range");
-    side.zfused = false;
   }
-  // Sums of z' parts above this many take a CTA of eight warps instead of one warp.
-  static constexpr int kZredWideParts = 16;
 
   // The products' schedules.  The two sides are built on two threads (host work of about the same
   // length), then uploaded.  With `only_n` (the tuner's candidates) the 'T' side stays as it is.

@@ -158,18 +158,15 @@ constexpr int rs_of(int R) {
 // kGatherRows client rows: it reads each column of x along the rows (coalesced), transposes
 // through shared memory, and writes each client row's RS values as one contiguous xz row at
 // its cluster position iperm[j].  One more CTA clears the kZeroRows zero rows from row `zrow0`
-// (the X rows of the y matrices' padding columns) and the ncnt chunk counters of the fused z
-// sums, so that every product starts from zero (also after one that stopped early).
+// (the X rows of the y matrices' padding columns).
 constexpr int kGatherRows = 64;
 template <typename T, int R, int RS>
 __global__ void __launch_bounds__(256) gather_kernel(const T* __restrict__ x, int N, int ldx, int q0, int r,
-                                                     const int* __restrict__ iperm, T* __restrict__ xz, int zrow0,
-                                                     int* zcnt, int ncnt) {
+                                                     const int* __restrict__ iperm, T* __restrict__ xz, int zrow0) {
   __shared__ T tile[RS][kGatherRows + 1];
   const int nblk = (N + kGatherRows - 1) / kGatherRows;
   if ((int)blockIdx.x >= nblk) {
     for (int e = threadIdx.x; e < kZeroRows * RS; e += blockDim.x) xz[(size_t)zrow0 * RS + e] = zero<T>();
-    for (int e = threadIdx.x; e < ncnt; e += blockDim.x) zcnt[e] = 0;  // the z sums' chunk counters
     return;
   }
   const int j0 = blockIdx.x * kGatherRows;
@@ -186,42 +183,6 @@ __global__ void __launch_bounds__(256) gather_kernel(const T* __restrict__ x, in
   }
 }
 inline unsigned gather_grid(int N) { return (unsigned)((N + kGatherRows - 1) / kGatherRows + 1); }
-
-// Loads through L2 only (another SM's writes, made visible by its fence, are not in this
-// SM's L1).
-__device__ inline float ld_l2(const float* p) { return __ldcg(p); }
-__device__ inline double ld_l2(const double* p) { return __ldcg(p); }
-__device__ inline cfloat ld_l2(const cfloat* p) {
-  const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
-  return cfloat{v.x, v.y};
-}
-__device__ inline cdouble ld_l2(const cdouble* p) {
-  const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
-  return cdouble{v.x, v.y};
-}
-
-// End of a z task that is a chunk of a long group (task.red >= 0), after its partial slot is
-// written: the warp's writes are fenced, the sum's counter taken, and the warp that finishes
-// the sum's last chunk adds the partial slots in part order into the final slot (the order of
-// zred_kernel, so the result does not depend on which chunk finishes last).  No warp waits.
-template <typename T, int RS>
-__device__ inline void z_chunk_done(const GemvTask& task, const GemvZred* __restrict__ zred, int* zcnt, T* xz,
-                                    int lane) {
-  if (task.red < 0 || !zcnt) return;
-  __threadfence();
-  __syncwarp();
-  int last = 0;
-  if (lane == 0) last = atomicAdd(&zcnt[task.red], 1) == zred[task.red].nparts - 1;
-  last = __shfl_sync(0xffffffffu, last, 0);
-  if (!last) return;
-  __threadfence();
-  const GemvZred d = zred[task.red];
-  for (int e = lane; e < d.k * RS; e += 32) {
-    T v = zero<T>();
-    for (int p = 0; p < d.nparts; ++p) v = v + ld_l2(xz + ((size_t)d.part_row + (size_t)p * d.k) * RS + e);
-    xz[(size_t)d.final_row * RS + e] = v;
-  }
-}
 
 // Checks a unit's copies into a warp-level stage before they are issued: 16-byte sizes and
 // addresses (the bulk-copy rule), the piece below the X rows, the X rows inside the stage, and
@@ -422,8 +383,7 @@ constexpr int warp_min_blocks() {
 template <typename T, int R, int RS, int MODE, int A2>
 __global__ void __launch_bounds__(kWarpCTA * 32, (warp_min_blocks<T, R, A2>()))
     warp_stream_kernel(const GemvTask* __restrict__ tasks, const int* __restrict__ warp_begin,
-                       const GemvUnit* __restrict__ units, const T* __restrict__ arena, T* xz, GemvStatus* err,
-                       const GemvZred* __restrict__ zred, int* zcnt) {
+                       const GemvUnit* __restrict__ units, const T* __restrict__ arena, T* xz, GemvStatus* err) {
   using Ops = RowOps<T, R>;
   constexpr int OL = MODE == 0 ? 32 : 16;
   // MODE 2: right-hand sides per round of the slice sums (a power of two)
@@ -594,7 +554,6 @@ __global__ void __launch_bounds__(kWarpCTA * 32, (warp_min_blocks<T, R, A2>()))
       if (lane == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       issue_next(u - 1 + kWarpStages);
     }
-    z_chunk_done<T, RS>(task, zred, zcnt, xz, lane);
   }
 }
 
@@ -698,8 +657,7 @@ __host__ __device__ constexpr int mma_min_blocks(int /*ntile*/, int /*elem_bytes
 template <typename T, int R, int RS, int NTILE>
 __global__ void __launch_bounds__(kWarpCTA * 32, mma_min_blocks(NTILE, sizeof(T)))
     mma_stream_kernel(const GemvTask* __restrict__ tasks, const int* __restrict__ warp_begin,
-                      const GemvUnit* __restrict__ units, const T* __restrict__ arena, T* xz, GemvStatus* err,
-                      const GemvZred* __restrict__ zred, int* zcnt) {
+                      const GemvUnit* __restrict__ units, const T* __restrict__ arena, T* xz, GemvStatus* err) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -797,7 +755,6 @@ __global__ void __launch_bounds__(kWarpCTA * 32, mma_min_blocks(NTILE, sizeof(T)
         }
       }
     }
-    z_chunk_done<T, RS>(task, zred, zcnt, xz, lane);
   }
 }
 
@@ -1406,8 +1363,11 @@ __global__ void __launch_bounds__(256) yfinal_kernel(const int2* __restrict__ ro
 // Sums partial slots: xz[final + l] = sum_p xz[part + p k + l].  A warp per sum (kZredWarps sums
 // a CTA), lanes over 16-byte chunks of the k x RS slot (a row of RS scalars is a multiple of 16
 // bytes), the parts added in part order; the first `nwide` sums take a CTA each, its warps an
-// eighth of the parts, joined in warp order (the z' of long leaves in the transposed products:
-// hundreds of parts, one warp's loads being a chain).
+// eighth of the parts, joined in warp order (long groups and leaves have hundreds of parts, and
+// one warp's loads are a chain).  FP64 and complex z kernels that summed their chunks themselves,
+// the last chunk's warp adding all parts, took 331 us for the 50,000-point Helmholtz cylinder
+// (complex FP32, four right-hand sides; 280 us with this pass) and 35 us for the 8,000-point
+// cylinder (FP64, one; 31 us).
 constexpr int kZredWarps = 8;
 constexpr int kZredBatch = 8;  // parts loaded before they are added (loads in flight together)
 template <typename T, int RS>
@@ -1496,8 +1456,7 @@ void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cuda
 
 // ---------------------------------------------------------------------------------
 template <typename T, int R, int RS, int MODE, int A2>
-void launch_warp_t(const GemvLaunch& L, const GemvUnit* units, const T* arena, T* xz, GemvStatus* err, cudaStream_t s,
-                   const GemvZred* zred, int* zcnt) {
+void launch_warp_t(const GemvLaunch& L, const GemvUnit* units, const T* arena, T* xz, GemvStatus* err, cudaStream_t s) {
   auto kern = warp_stream_kernel<T, R, RS, MODE, A2>;
   const size_t smem = warp_stream_smem_bytes((int)sizeof(T));
   static bool attr = false;
@@ -1505,13 +1464,12 @@ void launch_warp_t(const GemvLaunch& L, const GemvUnit* units, const T* arena, T
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     attr = true;
   }
-  launch_pdl(kern, dim3(L.ncta), dim3(kWarpCTA * 32), smem, s, L.tasks, L.cta_begin, units, arena, xz, err, zred,
-             zcnt);
+  launch_pdl(kern, dim3(L.ncta), dim3(kWarpCTA * 32), smem, s, L.tasks, L.cta_begin, units, arena, xz, err);
 }
 
 template <typename T, int R, int RS, int NTILE>
 void launch_mma_t(const GemvLaunch& L, const GemvUnit* units, const T* arena, T* xz, GemvStatus* err,
-                  cudaStream_t s, const GemvZred* zred, int* zcnt) {
+                  cudaStream_t s) {
   auto kern = mma_stream_kernel<T, R, RS, NTILE>;
   const size_t smem = warp_stream_smem_bytes((int)sizeof(T));
   static bool attr = false;
@@ -1519,15 +1477,12 @@ void launch_mma_t(const GemvLaunch& L, const GemvUnit* units, const T* arena, T*
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     attr = true;
   }
-  launch_pdl(kern, dim3(L.ncta), dim3(kWarpCTA * 32), smem, s, L.tasks, L.cta_begin, units, arena, xz, err, zred,
-             zcnt);
+  launch_pdl(kern, dim3(L.ncta), dim3(kWarpCTA * 32), smem, s, L.tasks, L.cta_begin, units, arena, xz, err);
 }
 
-// The 'N' launches.  zred / zcnt: the sums of the z chunks, done by the warp-level z kernels
-// themselves (z_chunk_done); null for the y launches.
+// The 'N' launches.
 template <typename T, int R, int RS>
-void launch_stream(const GemvLaunch& L, const GemvUnit* units, const T* arena, T* xz, GemvStatus* err, cudaStream_t s,
-                   const GemvZred* zred = nullptr, int* zcnt = nullptr) {
+void launch_stream(const GemvLaunch& L, const GemvUnit* units, const T* arena, T* xz, GemvStatus* err, cudaStream_t s) {
   if (L.ntasks <= 0) return;
   if constexpr (std::is_same<T, float>::value) {
     if (L.map == 4) {
@@ -1540,33 +1495,33 @@ void launch_stream(const GemvLaunch& L, const GemvUnit* units, const T* arena, T
     // the same leaves 3.1e-7 -> 1.6e-7).  At four the tiles are still faster (95 against 101 us).
     if constexpr (R == 1) {
       if (L.rpt <= 4)
-        launch_warp_t<T, R, RS, 2, 2>(L, units, arena, xz, err, s, zred, zcnt);
+        launch_warp_t<T, R, RS, 2, 2>(L, units, arena, xz, err, s);
       else if (L.rpt <= 8)
-        launch_warp_t<T, R, RS, 0, 2>(L, units, arena, xz, err, s, zred, zcnt);
+        launch_warp_t<T, R, RS, 0, 2>(L, units, arena, xz, err, s);
       else
-        launch_warp_t<T, R, RS, 0, 4>(L, units, arena, xz, err, s, zred, zcnt);
+        launch_warp_t<T, R, RS, 0, 4>(L, units, arena, xz, err, s);
       return;
     }
     switch (L.rpt) {  // map 3: rpt = 8-row tiles of the launch's tallest task (exact up to 8)
-      case 1: launch_mma_t<T, R, RS, 1>(L, units, arena, xz, err, s, zred, zcnt); break;
-      case 2: launch_mma_t<T, R, RS, 2>(L, units, arena, xz, err, s, zred, zcnt); break;
-      case 3: launch_mma_t<T, R, RS, 3>(L, units, arena, xz, err, s, zred, zcnt); break;
-      case 4: launch_mma_t<T, R, RS, 4>(L, units, arena, xz, err, s, zred, zcnt); break;
-      case 5: launch_mma_t<T, R, RS, 5>(L, units, arena, xz, err, s, zred, zcnt); break;
-      case 6: launch_mma_t<T, R, RS, 6>(L, units, arena, xz, err, s, zred, zcnt); break;
-      case 7: launch_mma_t<T, R, RS, 7>(L, units, arena, xz, err, s, zred, zcnt); break;
-      case 8: launch_mma_t<T, R, RS, 8>(L, units, arena, xz, err, s, zred, zcnt); break;
-      default: launch_mma_t<T, R, RS, 16>(L, units, arena, xz, err, s, zred, zcnt); break;
+      case 1: launch_mma_t<T, R, RS, 1>(L, units, arena, xz, err, s); break;
+      case 2: launch_mma_t<T, R, RS, 2>(L, units, arena, xz, err, s); break;
+      case 3: launch_mma_t<T, R, RS, 3>(L, units, arena, xz, err, s); break;
+      case 4: launch_mma_t<T, R, RS, 4>(L, units, arena, xz, err, s); break;
+      case 5: launch_mma_t<T, R, RS, 5>(L, units, arena, xz, err, s); break;
+      case 6: launch_mma_t<T, R, RS, 6>(L, units, arena, xz, err, s); break;
+      case 7: launch_mma_t<T, R, RS, 7>(L, units, arena, xz, err, s); break;
+      case 8: launch_mma_t<T, R, RS, 8>(L, units, arena, xz, err, s); break;
+      default: launch_mma_t<T, R, RS, 16>(L, units, arena, xz, err, s); break;
     }
   } else {
     if (L.map == 2)
-      launch_warp_t<T, R, RS, 2, 2>(L, units, arena, xz, err, s, zred, zcnt);
+      launch_warp_t<T, R, RS, 2, 2>(L, units, arena, xz, err, s);
     else if (L.map == 5)
-      launch_warp_t<T, R, RS, 0, 2>(L, units, arena, xz, err, s, zred, zcnt);
+      launch_warp_t<T, R, RS, 0, 2>(L, units, arena, xz, err, s);
     else if (L.map == 1)
-      launch_warp_t<T, R, RS, 1, 4>(L, units, arena, xz, err, s, zred, zcnt);
+      launch_warp_t<T, R, RS, 1, 4>(L, units, arena, xz, err, s);
     else
-      launch_warp_t<T, R, RS, 0, 4>(L, units, arena, xz, err, s, zred, zcnt);
+      launch_warp_t<T, R, RS, 0, 4>(L, units, arena, xz, err, s);
   }
 }
 
@@ -1579,7 +1534,7 @@ void allow_smem(F kern, bool& done) {
 
 template <typename T, int RS>
 void launch_zred(const GemvSide& side, T* xz, cudaStream_t s) {
-  if (side.nzred > 0 && !side.zfused)
+  if (side.nzred > 0)
     launch_pdl(zred_kernel<T, RS>, dim3(zred_grid(side.nzred, side.nzwide)), dim3(kZredWarps * 32), 0, s, side.zred,
                side.nzred, side.nzwide, xz);
 }
@@ -1624,14 +1579,13 @@ void run_tile(const GemvPlan& p, int nrhs, int q0, T alpha, T beta, const T* x, 
   const int ld_in = n_in, ld_out = TRANSP ? p.n_cols : p.n_rows;
   const T* arena = (const T*)p.arena;
   if (tm) cudaEventRecord(tm->ev[0], s);
-  gather_kernel<T, R, RS><<<gather_grid(n_in), 256, 0, s>>>(x, n_in, ld_in, q0, nrhs, iperm_in, xz, p.n_in_max,
-                                                            side.zcnt, side.zfused ? side.nzred : 0);
+  gather_kernel<T, R, RS><<<gather_grid(n_in), 256, 0, s>>>(x, n_in, ld_in, q0, nrhs, iperm_in, xz, p.n_in_max);
   if (tm) cudaEventRecord(tm->ev[1], s);
   if constexpr (TRANSP) {
     run_trans_columns<T, R, RS>(side, arena, xz, conj, err, s);
   } else {
     for (int c = 0; c < side.nz; ++c)
-      launch_stream<T, R, RS>(side.z[c], side.units, arena, xz, err, s, side.zfused ? side.zred : nullptr, side.zcnt);
+      launch_stream<T, R, RS>(side.z[c], side.units, arena, xz, err, s);
     launch_zred<T, RS>(side, xz, s);
   }
   if (tm) cudaEventRecord(tm->ev[2], s);
@@ -1758,9 +1712,9 @@ void forward_z(const GemvPlan& p, int nrhs, const T* x, T* xz, GemvStatus* err, 
   constexpr int RS = rs_of<T>(R);
   const GemvSide& sn = p.side[0];
   gather_kernel<T, R, RS><<<gather_grid(p.n_cols), 256, 0, s>>>(x, p.n_cols, p.n_cols, 0, nrhs, p.iperm_cols, xz,
-                                                                p.n_in_max, sn.zcnt, sn.zfused ? sn.nzred : 0);
+                                                                p.n_in_max);
   for (int c = 0; c < sn.nz; ++c)
-    launch_stream<T, R, RS>(sn.z[c], sn.units, (const T*)p.arena, xz, err, s, sn.zfused ? sn.zred : nullptr, sn.zcnt);
+    launch_stream<T, R, RS>(sn.z[c], sn.units, (const T*)p.arena, xz, err, s);
   launch_zred<T, RS>(sn, xz, s);
 }
 template <typename T, int R>
@@ -1780,7 +1734,7 @@ void grads_tile(const GemvPlan& p, int nrhs, const T* x, const T* r, T* xz, T* r
   forward_z<T, R>(p, nrhs, x, xz, err, s);
   // r in cluster order (rows) and w = A^T r
   gather_kernel<T, R, RS><<<gather_grid(p.n_rows), 256, 0, s>>>(r, p.n_rows, p.n_rows, 0, nrhs, p.iperm_rows, rz,
-                                                                p.n_in_max, nullptr, 0);
+                                                                p.n_in_max);
   run_trans_columns<T, R, RS>(p.side[1], (const T*)p.arena, rz, 0, err, s);
   grads_outer<T, R>(p, xz, rz, gfull, grk, accumulate, s);
 }
@@ -1824,7 +1778,7 @@ int gemv_launch_count(const GemvPlan& p, char trans, int nrhs, int elem_bytes) {
   const GemvSide& side = p.side[(trans == 'N' || trans == 'n') ? 0 : 1];
   int per_tile = 1;  // gather
   for (int c = 0; c < side.nz; ++c) per_tile += side.z[c].ntasks > 0;
-  per_tile += side.nzred > 0 && !side.zfused;
+  per_tile += side.nzred > 0;
   per_tile += side.y.ntasks > 0;
   for (int c = 0; c < side.ng; ++c) per_tile += side.g[c].ntasks > 0;
   per_tile += side.nyrows > 0;  // final pass

@@ -50,8 +50,6 @@ struct GemvTask {
   int first_unit;  // units [first_unit, first_unit + nunits) in order
   int nunits;
   int out_row;     // first xz row of the output slot; column pass: first xz row of the x rows
-  int red = -1;    // 'N' z chunk of a long group: its z sum (GemvZred index); the last chunk of
-                   // the sum to finish adds the partial slots in part order
 };
 
 // One launch: tasks of one shape class; each CTA (column pass) or warp of a persistent grid takes
@@ -139,10 +137,6 @@ struct GemvSide {
   const int* colmap = nullptr;  // 'T': destination rows of the column pass
   int ng = 0;                   // 'T': group-pass launches (one per group height class)
   GemvLaunch g[2];
-  // zfused: the z kernels sum the parts themselves ('N', FP64 and complex); zcnt[i]: chunks of sum i
-  // finished in the current product (cleared by the gather that opens every product)
-  bool zfused = false;
-  int* zcnt = nullptr;
   GemvLaunch y;  // 'N'
   const GemvUnit* units = nullptr;         // 'N'
   const GemvTransUnit* tunits = nullptr;   // 'T'
