@@ -26,26 +26,32 @@
 namespace hmatb200 {
 namespace {
 
+// A device array.  alloc() and upload() keep the memory of an array that is large enough and not
+// twice too large, so that assembling a matrix again does not free and map all of it (the callers
+// that rewrite a live matrix wait for its products first: quiesce()).
 template <typename X>
 struct DevArray {
   X* p = nullptr;
-  size_t n = 0;
+  size_t n = 0, cap = 0;
   DevArray() = default;
   DevArray(const DevArray&) = delete;
   DevArray& operator=(const DevArray&) = delete;
-  DevArray(DevArray&& o) noexcept : p(o.p), n(o.n) {
+  DevArray(DevArray&& o) noexcept : p(o.p), n(o.n), cap(o.cap) {
     o.p = nullptr;
-    o.n = 0;
+    o.n = o.cap = 0;
   }
   ~DevArray() { release(); }
   void release() {
     if (p) cudaFree(p);
     p = nullptr;
-    n = 0;
+    n = cap = 0;
   }
   void alloc(size_t count) {
-    release();
-    if (count) HB_CUDA(cudaMalloc(&p, count * sizeof(X)));
+    if (count == 0 || count > cap || cap > 2 * count + 4096) {
+      release();
+      if (count) HB_CUDA(cudaMalloc(&p, count * sizeof(X)));
+      cap = count;
+    }
     n = count;
   }
   void ensure(size_t count) {
@@ -58,6 +64,7 @@ struct DevArray {
   void swap(DevArray& o) {
     std::swap(p, o.p);
     std::swap(n, o.n);
+    std::swap(cap, o.cap);
   }
 };
 
@@ -263,10 +270,7 @@ class Engine : public EngineBase {
       throw Error("the Helmholtz kernel requires a complex value type and the real kernels a real one");
     if (method != 0 && method != 1) throw Error("only ACA+ and partial ACA compression run on the device");
     assembled = false;
-    if (gexec_) {
-      cudaGraphExecDestroy(gexec_);
-      gexec_ = nullptr;
-    }
+    quiesce();
     kp_ = a.kp;
     // a multi-strata kernel: a_0 .. a_{S-1}, w_0 .. w_{S-1}
     if (a.strata.size() % 2 || a.strata.size() > 2 * (size_t)kMaxStrata)
@@ -454,10 +458,7 @@ class Engine : public EngineBase {
         throw Error("stored data: rank out of range");
     }
     assembled = false;
-    if (gexec_) {
-      cudaGraphExecDestroy(gexec_);
-      gexec_ = nullptr;
-    }
+    quiesce();
     ranks.assign(rk_in, rk_in + nleaves);
     // the permutations the gemv gathers and scatters with (assemble uploads them with the
     // points; a loaded matrix has no points)
@@ -527,6 +528,7 @@ class Engine : public EngineBase {
   void retruncate(double eps) override {
     if (!assembled) throw Error("matrix not assembled");
     check_device();
+    quiesce();
     HB_CUDA(set_jacobi_max_sweeps(jacobi_sweeps()));
     const auto& L = bt_->leaves;
     const int nleaves = (int)L.size();
@@ -560,10 +562,6 @@ class Engine : public EngineBase {
       if (!retry.empty()) throw Error("re-truncation: unexpected capacity retry");
     }
     rebuild_arena();
-    if (gexec_) {
-      cudaGraphExecDestroy(gexec_);
-      gexec_ = nullptr;
-    }
     plan_products();
     HB_CUDA(cudaStreamSynchronize(stream_));
     for (int i = 0; i < 4; ++i) times_ms[i] = saved[i];
@@ -683,6 +681,16 @@ class Engine : public EngineBase {
     if (d != device)
       throw Error("the current CUDA device (" + std::to_string(d) + ") is not the matrix's device (" +
                   std::to_string(device) + ")");
+  }
+
+  // Before the matrix's arrays are rewritten: its products on every stream have ended, and the
+  // graph that holds the arrays' addresses goes.
+  void quiesce() {
+    HB_CUDA(cudaDeviceSynchronize());
+    if (gexec_) {
+      cudaGraphExecDestroy(gexec_);
+      gexec_ = nullptr;
+    }
   }
 
   void clear_status(cudaStream_t s) {
@@ -2566,8 +2574,8 @@ class Engine : public EngineBase {
       if (m < 0 || m >= next_row) throw Error("gemv plan: column map out of range");
   }
 
-  // The products' schedules.  The two sides are built on two threads (host work of about the same
-  // length), then uploaded.  With `only_n` (the tuner's candidates) the 'T' side stays as it is.
+  // The products' schedules.  The two sides of a large matrix are built on two threads (host work of
+  // about the same length), then uploaded.  With `only_n` (the tuner's candidates) the 'T' side stays as it is.
   void build_plan(bool only_n = false) {
     const auto& L = bt_->leaves;
     std::vector<GemvFullLeaf> F;
@@ -2632,11 +2640,15 @@ class Engine : public EngineBase {
     {
       SidePlan sp[2];
       std::future<void> trans;
-      if (!only_n)
-        trans = std::async(std::launch::async,
-                           [&] { build_trans_side(K, rk_leaf, next_row[1], plan_.side[1], sp[1]); });
+      auto build_trans = [&] { build_trans_side(K, rk_leaf, next_row[1], plan_.side[1], sp[1]); };
+      // a thread costs about as much to start as the side of a matrix of four million scalars
+      const bool beside = !only_n && layout_.total > (4LL << 20);
+      if (beside)
+        trans = std::async(std::launch::async, build_trans);
+      else if (!only_n)
+        build_trans();
       build_side(K, rk_leaf, next_row[0], bound_rows, plan_.side[0], sp[0]);
-      if (!only_n) trans.get();
+      if (beside) trans.get();
       upload_side(sp[0], plan_.side[0], side_buf_[0]);
       if (!only_n) upload_side(sp[1], plan_.side[1], side_buf_[1]);
       HB_CUDA(cudaStreamSynchronize(stream_));  // the host vectors go out of scope
