@@ -2740,8 +2740,9 @@ class Engine : public EngineBase {
 
   // Chunk size of the z tasks of a matrix too small to tune: as many units as give every warp of
   // the z launch about one chunk, 16 at most (one right-hand side, 8,000-point cylinder, FP64: 43 us
-  // with chunks of 16 units, 35 with the 2 this gives; 15,000 points, FP32, 16 right-hand sides: 66
-  // -> 53 us; 5,000-point Helmholtz cylinder, complex FP32, four: 53 -> 42 us).
+  // with chunks of 16 units, 35 with the 2 this gives, both before the parts were summed by
+  // zred_kernel, 31 since; 15,000 points, FP32, 16 right-hand sides: 66 -> 53 us; 5,000-point
+  // Helmholtz cylinder, complex FP32, four: 53 -> 42 us).
   int small_zparts() const {
     long long units = 0;
     int omax = 1;

@@ -1,17 +1,15 @@
 // Device-resident schedule of the batched H-matrix-vector product (built on the host by
 // the engine from the leaf list, consumed by gemv.cu).
 //
-// Leaf storage is panelised so that every product term is one contiguous chunk:
-//  * a full leaf F (m x n) is stored as row panels, one per output block of its rows,
-//    each panel column-major (len x n);
-//  * an Rk leaf stores A as row panels (len x k, column-major) and B transposed,
-//    B^T column-major (k x n), i.e. each row of B contiguous.
-// An output block is a leaf of the output cluster tree, cut into pieces of at most 128 rows.
+// The leaf arena has two regions (layout in engine.cu): per output block (a leaf of the output
+// cluster tree, cut into pieces of at most 128 rows) one column-major matrix holding the block's
+// rows of every full leaf F and of every Rk leaf's A over those rows; then the B^T of the Rk
+// leaves, those of one column range stacked into column-major groups.
 //
-// A product is a list of tasks; a task is one output (an output block of y, or the z = B^T x
-// slot of an Rk leaf) accumulated from a list of units; a unit is out += op(P) X for one
-// contiguous piece P of the leaf arena and one contiguous piece X of the xz buffer (x in
-// cluster order, row-major, followed by the z rows).
+// A product is a list of tasks; a task is one output ('N': an output block of y or the z = B^T x
+// slots of a group; 'T': the columns of an output block, or a strip of columns of a column block)
+// accumulated from a list of units, each one contiguous piece P of the arena times rows X of the
+// xz buffer (x in cluster order, row-major, followed by the z rows).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
