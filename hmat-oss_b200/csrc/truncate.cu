@@ -14,6 +14,7 @@
 
 #include "block_reduce.cuh"
 #include "kernels.h"
+#include "sigma_order.h"
 
 namespace hmatb200 {
 namespace {
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(kTruncThreads) truncate_kernel(const RkLeafDes
     // descending order, ties by index (stable)
     for (int j = threadIdx.x; j < k; j += blockDim.x) {
       int r = 0;
-      for (int i = 0; i < k; ++i) r += (sig[i] > sig[j]) || (sig[i] == sig[j] && i < j);
+      for (int i = 0; i < k; ++i) r += sigma_before(sig[i], i, sig[j], j);
       ord[r] = j;
     }
     __syncthreads();
@@ -667,7 +668,7 @@ __global__ void __launch_bounds__(NW * 32) tscore_kernel(const TsCore* __restric
 #pragma unroll
     for (int i = 0; i < K; ++i) {
       const double si = __shfl_sync(0xffffffffu, sg, i, SW);
-      if (i < k) rnk += (si > sg) || (si == sg && i < j);
+      if (i < k) rnk += sigma_before(si, i, sg, j);
     }
     if (j < k) ord[rnk] = j;
     __syncwarp();
@@ -990,7 +991,7 @@ __global__ void __launch_bounds__(kDenseSvdThreads) dense_svd_kernel(const RkLea
     __syncthreads();
     for (int p = tid; p < r; p += blockDim.x) {
       int at = 0;
-      for (int i = 0; i < r; ++i) at += (s_nrm[i] > s_nrm[p]) || (s_nrm[i] == s_nrm[p] && i < p);
+      for (int i = 0; i < r; ++i) at += sigma_before(s_nrm[i], i, s_nrm[p], p);
       s_ord[at] = p;
     }
     __syncthreads();
@@ -1258,7 +1259,7 @@ __global__ void __launch_bounds__(jacobi_threads<double>(H), 2) dense_jacobi_ker
     // descending order, ties by index (stable)
     for (int j = tid; j < k; j += blockDim.x) {
       int r = 0;
-      for (int i = 0; i < k; ++i) r += (sig[i] > sig[j]) || (sig[i] == sig[j] && i < j);
+      for (int i = 0; i < k; ++i) r += sigma_before(sig[i], i, sig[j], j);
       ord[r] = j;
     }
     __syncthreads();
@@ -1394,7 +1395,7 @@ __global__ void __launch_bounds__(tscore_cta_threads<W>(H))
     __syncthreads();
     for (int j = threadIdx.x; j < k; j += blockDim.x) {
       int r = 0;
-      for (int i = 0; i < k; ++i) r += (sig[i] > sig[j]) || (sig[i] == sig[j] && i < j);
+      for (int i = 0; i < k; ++i) r += sigma_before(sig[i], i, sig[j], j);
       ord[r] = j;
     }
     __syncthreads();
