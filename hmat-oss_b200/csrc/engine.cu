@@ -684,9 +684,19 @@ class Engine : public EngineBase {
   }
 
   // Before the matrix's arrays are rewritten: its products on every stream have ended, and the
-  // graph that holds the arrays' addresses goes.
+  // graph that holds the arrays' addresses goes.  cudaFree waits for them, as freeing the arrays
+  // themselves would; cudaDeviceSynchronize is an error while any thread captures a stream (the
+  // products of another matrix, say), and a matrix that was never multiplied waits for nobody.
   void quiesce() {
-    HB_CUDA(cudaDeviceSynchronize());
+    check_device();
+    if (fence_.p) {
+      DevArray<int> old;
+      old.swap(fence_);
+      int* p = old.p;
+      old.p = nullptr;
+      HB_CUDA(cudaFree(p));
+      fence_.alloc(1);
+    }
     if (gexec_) {
       cudaGraphExecDestroy(gexec_);
       gexec_ = nullptr;
@@ -2758,8 +2768,14 @@ class Engine : public EngineBase {
     return (int)std::max(1LL, std::min(16LL, (units + warps - 1) / warps));
   }
 
-  // Builds the products' schedules, with the tuner's choice for the matrix's class.
+  // The products' schedules; products can run afterwards.
   void plan_products() {
+    choose_plan();
+    if (!fence_.p) fence_.alloc(1);
+  }
+
+  // Builds the schedules with the tuner's choice for the matrix's class.
+  void choose_plan() {
     gemv_tuned = 0;
     gemv_choice[0] = tune_zparts_ = 16;
     gemv_choice[1] = 0;
@@ -2857,6 +2873,7 @@ class Engine : public EngineBase {
   GemvPlan plan_;
   long long noalloc_rows_ = 0;
   DevArray<T> xz_, rz_, stage_x_, stage_y_;  // scratch of 'N' and of 'T' products, host staging
+  DevArray<int> fence_;            // held once products can run; freed and taken again by quiesce()
   DevArray<GemvStatus> err_;       // status block of this matrix's products (flag, wait bound)
   GemvStatus* h_err_ = nullptr;    // pinned host copy
   cudaGraphExec_t gexec_ = nullptr;
