@@ -331,8 +331,6 @@ class Engine : public EngineBase {
     check_gemv_args(trans, nrhs);
     if (nrhs == 0) return;
     const T a = *(const T*)alpha, b = *(const T*)beta;
-    DevArray<T>& scratch = trans == 'N' ? xz_ : rz_;
-    scratch.ensure(xz_elems(trans == 'N' ? 0 : 1));
     GraphKey key(trans, nrhs, x, y);
     memcpy(key.ab, &a, sizeof(T));
     memcpy(key.ab + sizeof(T), &b, sizeof(T));
@@ -343,7 +341,7 @@ class Engine : public EngineBase {
       }
       cudaGraph_t g;
       HB_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-      launch_gemv<T>(plan_, trans, nrhs, a, b, (const T*)x, (T*)y, scratch.p, err_.p, stream_);
+      launch_gemv<T>(plan_, trans, nrhs, a, b, (const T*)x, (T*)y, xz_.p, err_.p, stream_);
       cudaError_t launch_err = cudaGetLastError();
       HB_CUDA(cudaStreamEndCapture(stream_, &g));
       HB_CUDA(launch_err);
@@ -427,7 +425,6 @@ class Engine : public EngineBase {
     if (Traits<T>::is_complex) throw Error("leaf gradients are implemented for real value types");
     if (nrhs < 1 || nrhs > 16) throw Error("leaf gradients take 1 to 16 right-hand sides");
     check_device();
-    xz_.ensure(xz_elems(0));
     rz_.ensure(xz_elems(1));
     cudaStream_t s = user_stream ? user_stream : stream_;
     launch_leaf_gradients<T>(plan_, nrhs, (const T*)x, (const T*)r, xz_.p, rz_.p, (T*)grad, (T*)grad, accumulate,
@@ -441,7 +438,6 @@ class Engine : public EngineBase {
     if (Traits<T>::is_complex) throw Error("the adjoint is implemented for real value types");
     if (nrhs < 1 || nrhs > 16) throw Error("the adjoint takes 1 to 16 right-hand sides");
     check_device();
-    xz_.ensure(xz_elems(0));
     rz_.ensure(xz_elems(1));
     cudaStream_t s = user_stream ? user_stream : stream_;
     launch_gemv_adjoint<T>(plan_, nrhs, (const T*)x, (const T*)r, (T*)dx, xz_.p, rz_.p, (T*)grad, (T*)grad, accumulate,
@@ -570,11 +566,9 @@ class Engine : public EngineBase {
   void profile_gemv(char trans, const void* x, void* y, int nrhs, double* ms3, double* bytes3) override {
     check_gemv_args(trans, nrhs);
     if (nrhs < 1 || nrhs > 16) throw Error("profile_gemv takes 1 to 16 right-hand sides");
-    DevArray<T>& scratch = trans == 'N' ? xz_ : rz_;
-    scratch.ensure(xz_elems(trans == 'N' ? 0 : 1));
     GemvTiming tm;
     for (int i = 0; i < 4; ++i) HB_CUDA(cudaEventCreate(&tm.ev[i]));
-    launch_gemv<T>(plan_, trans, nrhs, one<T>(), zero<T>(), (const T*)x, (T*)y, scratch.p, err_.p, stream_, &tm);
+    launch_gemv<T>(plan_, trans, nrhs, one<T>(), zero<T>(), (const T*)x, (T*)y, xz_.p, err_.p, stream_, &tm);
     cudaError_t le = cudaGetLastError();
     cudaError_t se = cudaStreamSynchronize(stream_);
     float a = 0, b = 0, c = 0;
@@ -664,7 +658,9 @@ class Engine : public EngineBase {
   };
 
   // Elements of the scratch of an 'N' (side 0) or 'T' / 'C' product in its widest tiles of
-  // right-hand sides (16; complex double 4).  Products in the two directions use a buffer each (xz_, rz_).
+  // right-hand sides (16; complex double 4).  Products of both directions use xz_, which holds the
+  // larger of the two from the assembly on, so that no product allocates (the first one in a new
+  // direction may be under capture); the adjoint's pass over r has rz_, taken at its first call.
   size_t xz_elems(int side) const {
     return (size_t)std::max(plan_.xz_rows[side], 1LL) * gemv_rhs_stride((int)sizeof(T), sizeof(T) >= 16 ? 4 : 16);
   }
@@ -2771,6 +2767,7 @@ class Engine : public EngineBase {
   // The products' schedules; products can run afterwards.
   void plan_products() {
     choose_plan();
+    xz_.ensure(std::max(xz_elems(0), xz_elems(1)));
     if (!fence_.p) fence_.alloc(1);
   }
 
@@ -2872,7 +2869,7 @@ class Engine : public EngineBase {
   std::vector<int> zgroup_row_[2];  // first z row of each B^T group, 'N' and 'T' 
   GemvPlan plan_;
   long long noalloc_rows_ = 0;
-  DevArray<T> xz_, rz_, stage_x_, stage_y_;  // scratch of 'N' and of 'T' products, host staging
+  DevArray<T> xz_, rz_, stage_x_, stage_y_;  // scratch of products and of the adjoint's second vector, host staging
   DevArray<int> fence_;            // held once products can run; freed and taken again by quiesce()
   DevArray<GemvStatus> err_;       // status block of this matrix's products (flag, wait bound)
   GemvStatus* h_err_ = nullptr;    // pinned host copy

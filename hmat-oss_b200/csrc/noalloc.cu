@@ -4,11 +4,10 @@
 // runs under a memory pool or allocator it does not own (a framework's caching allocator,
 // a solver that has reserved all device memory up front), code inside a callback where
 // cudaMalloc / cudaFree would synchronise the device or deadlock, or hard real-time loops
-// that forbid allocation after start-up.  hmat_b200_gemv_device allocates its scratch
-// lazily (the cluster-ordered copy of x and the per-leaf z = B^T x values) and builds a CUDA
-// graph on first use; this variant does neither.  Its scratch is one file-scope device
-// array of fixed size, reserved by every GPU that loads this library's device code and
-// held until the process exits.
+// that forbid allocation after start-up.  hmat_b200_gemv_device builds a CUDA graph for new
+// arguments, which allocates; this variant does not.  Its scratch (the cluster-ordered copy of
+// x, the per-leaf z = B^T x values, partial sums) is one file-scope device array of fixed size,
+// reserved by every GPU that loads this library's device code and held until the process exits.
 #include <cuda_runtime.h>
 
 #include <mutex>
