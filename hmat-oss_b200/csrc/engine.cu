@@ -613,18 +613,12 @@ class Engine : public EngineBase {
                                 cudaStream_t stream, void* scratch, size_t scratch_bytes) override {
     check_gemv_args(trans, nrhs);
     if (nrhs == 0) return;
-    // the widest tile of right-hand sides whose rows fit (the partial rows of a transposed product
-    // of a large matrix may not fit at 16)
-    int tile = 16;
-    auto need = [&]() {
-      return (size_t)plan_.xz_rows[trans == 'N' ? 0 : 1] * gemv_rhs_stride((int)sizeof(T), tile) * sizeof(T);
-    };
-    while (tile > 1 && need() > scratch_bytes) tile = tile > 4 ? tile / 2 : 1;
-    if (need() > scratch_bytes) throw Error("scratch buffer too small for this matrix");
+    if (xz_elems(trans == 'N' ? 0 : 1) * sizeof(T) > scratch_bytes)
+      throw Error("scratch buffer too small for this matrix");
     cudaStream_t s = stream ? stream : stream_;
     // the status flag is the matrix's own (allocated with the engine), read by gemv_status
     launch_gemv<T>(plan_, trans, nrhs, *(const T*)alpha, *(const T*)beta, (const T*)x, (T*)y, (T*)scratch, err_.p,
-                   s, nullptr, tile);
+                   s);
     HB_CUDA(cudaGetLastError());
   }
 
@@ -2014,14 +2008,15 @@ class Engine : public EngineBase {
     L.rpt = omax <= 32 ? 2 : 4;
   }
 
-  // Sums sorted by decreasing parts; returns how many of them take a CTA of eight warps instead of
+  // Sums (from the given one on) sorted by decreasing parts; returns how many of them take a CTA of eight warps instead of
   // one warp (more than kZredWideParts parts).
   static constexpr int kZredWideParts = 16;
-  static int wide_sums_first(std::vector<GemvZred>& zred) {
-    std::stable_sort(zred.begin(), zred.end(), [](const GemvZred& x, const GemvZred& y) { return x.nparts > y.nparts; });
-    int n = 0;
+  static int wide_sums_first(std::vector<GemvZred>& zred, int first = 0) {
+    std::stable_sort(zred.begin() + first, zred.end(),
+                     [](const GemvZred& x, const GemvZred& y) { return x.nparts > y.nparts; });
+    int n = first;
     while (n < (int)zred.size() && zred[n].nparts > kZredWideParts) n++;
-    return n;
+    return n - first;
   }
 
   // A side's schedule as built on the host, before its upload.
@@ -2033,6 +2028,7 @@ class Engine : public EngineBase {
     std::vector<GemvZred> zred;
     std::vector<int> colmap;
     std::vector<int2> yrows;
+    std::vector<int> round_begin;  // 'T': where each round's ranges start in begin[0]
   };
 
   // With `begin` given (one range of tasks per warp, or per CTA for map 4), the ranges are taken as
@@ -2156,7 +2152,7 @@ class Engine : public EngineBase {
           const int u0 = pidx * kMaxUnits, u1 = std::min(nu, u0 + kMaxUnits);
           zt[cls].push_back(GemvTask{O, first + u0, u1 - u0, part_row + pidx * O});
         }
-        zred.push_back(GemvZred{zrow, O, part_row, nparts});
+        zred.push_back(GemvZred{zrow, (unsigned short)O, 0, part_row, nparts});
       }
     }
     // ---- y-phase ----
@@ -2346,6 +2342,10 @@ class Engine : public EngineBase {
     for (int c = 0; c < side.nz; ++c) point(side.z[c], c);
     for (int c = 0; c < side.ng; ++c) point(side.g[c], GemvSide::kMaxLaunch + c);
     if (side.y.ntasks > 0) point(side.y, GemvSide::kMaxLaunch);
+    for (size_t r = 0; r < side.rounds.size(); ++r) {
+      side.rounds[r].columns.tasks = sb.tasks[0].p;
+      side.rounds[r].columns.cta_begin = sb.begin[0].p + sp.round_begin[r];
+    }
     sb.units.upload(sp.units, stream_);
     side.units = sb.units.p;
     sb.tunits.upload(sp.tunits, stream_);
@@ -2353,7 +2353,7 @@ class Engine : public EngineBase {
     sb.colmap.upload(sp.colmap, stream_);
     side.colmap = sb.colmap.p;
     sb.zred.upload(sp.zred, stream_);
-    side.nzred = (int)sp.zred.size();
+    side.nzred = side.rounds.empty() ? (int)sp.zred.size() : 0;
     side.zred = sb.zred.p;
     sb.yrows.upload(sp.yrows, stream_);
     side.nyrows = (int)sp.yrows.size();
@@ -2369,7 +2369,7 @@ class Engine : public EngineBase {
     std::vector<double> cum(n + 1, 0.0);
     for (int v = 0; v < n; ++v) cum[v + 1] = cum[v] + (double)units[first + v].rows * units[first + v].cols + 256;
     const double tot = std::max(cum[n], 1.0);
-    begin.assign(G + 1, 0);
+    begin.assign(G + 1, (int)tasks.size());
     int w = 0;
     for (int v = 0; v < n;) {
       while (w + 1 < G && cum[v] >= tot * (w + 1) / G) begin[++w] = (int)tasks.size();
@@ -2422,6 +2422,7 @@ class Engine : public EngineBase {
     std::vector<GemvTask> gt[2];
     std::vector<int> gstrip[2], gbegin[2];
     side.ng = 0;
+    side.rounds.clear();
     for (int cls = 0; cls < 2; ++cls) {
       const int first = (int)units.size();
       std::vector<int> owner;
@@ -2462,18 +2463,34 @@ class Engine : public EngineBase {
       side.ng++;
     }
 
-    // ---- the parts of y: a full leaf gives a strip one part per row block it covers ----
-    std::vector<int> fullparts(strips.size(), 0);
+    // ---- the parts of y: a full leaf gives a strip one part per row block it covers; the columns
+    // of a block that take a slot of their own (full leaves, Rk leaves over several blocks) ----
+    std::vector<int> fullparts(strips.size(), 0), used(rblocks_.size(), 0), slots(rblocks_.size(), 0);
     for (int i = 0; i < (int)L.size(); ++i) {
-      if (layout_.first[i] < 0 || L[i].type != 0) continue;
+      if (layout_.first[i] < 0) continue;
       auto br = row_blocks(L[i].row_off, L[i].m);
+      const int nb = br.second - br.first, w = L[i].type == 0 ? L[i].n : ranks[i];
+      for (int b = br.first; b < br.second; ++b) {
+        used[b] += w;
+        if (L[i].type == 0 || nb > 1) slots[b] += w;
+      }
+      if (L[i].type != 0) continue;
       const int last = strip_of[L[i].col_off + L[i].n - 1];
-      for (int st = strip_of[L[i].col_off]; st <= last; ++st) fullparts[st] += br.second - br.first;
+      for (int st = strip_of[L[i].col_off]; st <= last; ++st) fullparts[st] += nb;
     }
+    // In one round every column keeps its slot to the end, the full leaves' as parts of y.  Where
+    // those rows are too many, consecutive blocks take turns on the same slots: each round's parts
+    // are summed before the next, the full leaves' into one part of y a strip.
+    const long long budget = trans_row_budget(K);
+    long long all_slots = 0, grouped = 0;
+    for (int n : slots) all_slots += n;
+    for (size_t st = 0; st < strips.size(); ++st) grouped += (long long)nparts[st] * strips[st].len;
+    const bool many = next_row + grouped + all_slots > budget;
     std::vector<int> part_row(strips.size(), 0), taken(strips.size(), 0);
     std::vector<int2>& yrows = sp.yrows;
     yrows.assign(C_->n, int2{0, 0});
     for (size_t st = 0; st < strips.size(); ++st) {
+      if (many) fullparts[st] = std::min(fullparts[st], 1);
       const int np = fullparts[st] + nparts[st];
       part_row[st] = (int)next_row;
       next_row += (long long)np * strips[st].len;
@@ -2486,7 +2503,23 @@ class Engine : public EngineBase {
         gt[c][t].O = strips[st].len;
         gt[c][t].out_row = part_row[st] + (fullparts[st] + taken[st]++) * strips[st].len;
       }
-    std::fill(taken.begin(), taken.end(), 0);
+    std::vector<std::pair<int, int>> cuts;  // the rounds' blocks
+    const int nblocks = (int)rblocks_.size();
+    if (many) {
+      long long most = 0;
+      for (int n : slots) most = std::max<long long>(most, n);
+      // a block a round at least; beyond the allocation-free products' bound also an eighth of the
+      // columns, as the rows that are not slots may fill the budget by themselves
+      const bool bounded = budget * RS16 * s <= kNoAllocArrayBytes;
+      const long long room = std::max({budget - next_row, most, bounded ? 0LL : all_slots / 8});
+      for (int b0 = 0, b1; b0 < nblocks; b0 = b1) {
+        long long n = 0;
+        for (b1 = b0; b1 < nblocks && n + slots[b1] <= room; ++b1) n += slots[b1];
+        cuts.push_back({b0, b1});
+      }
+    } else {
+      cuts.push_back({0, nblocks});
+    }
 
     // ---- column pass: the destination row of every column of every output block's matrix (the
     // block's columns at colbase, a multiple of 8), then its units of whole columns ----
@@ -2495,82 +2528,116 @@ class Engine : public EngineBase {
     if (colbase.back() >= (1LL << 31)) throw Error("gemv plan: too many columns");
     std::vector<int>& colmap = sp.colmap;
     colmap.assign((size_t)colbase.back() + 4, 0);
-    std::vector<int> used(rblocks_.size(), 0);
     std::vector<GemvZred>& zred = sp.zred;
     std::vector<int> rk_index(L.size(), -1);
     for (size_t t = 0; t < rk_leaf.size(); ++t) rk_index[rk_leaf[t]] = (int)t;
-    for (int i = 0; i < (int)L.size(); ++i) {
-      if (layout_.first[i] < 0) continue;
-      auto br = row_blocks(L[i].row_off, L[i].m);
-      const int nb = br.second - br.first, w = L[i].type == 0 ? L[i].n : ranks[i];
-      int zrow = 0;
-      if (L[i].type != 0) {
-        const GemvRkLeaf& k = K[rk_index[i]];
-        zrow = k.zrow_t;
-        if (nb > 1) {  // parts, one per row block, summed into the leaf's z' rows
-          zred.push_back(GemvZred{zrow, w, (int)next_row, nb});
-          zrow = (int)next_row;
-          next_row += (long long)nb * w;
+    const long long slot0 = next_row;
+    std::vector<int> first_slot(part_row), round_parts(strips.size(), 0);
+    std::vector<char> summed(strips.size(), 0);  // strips with a sum of earlier rounds
+    std::vector<GemvTask> ct;
+    for (const auto& cut : cuts) {
+      GemvTransRound round;
+      round.zred0 = (int)zred.size();
+      long long slot = slot0;
+      auto blocks_of = [&](int i) {
+        auto br = row_blocks(L[i].row_off, L[i].m);
+        return std::make_pair(std::max(br.first, cut.first), std::min(br.second, cut.second));
+      };
+      if (many) {
+        std::fill(round_parts.begin(), round_parts.end(), 0);
+        for (int i = 0; i < (int)L.size(); ++i) {
+          if (layout_.first[i] < 0 || L[i].type != 0) continue;
+          const auto br = blocks_of(i);
+          if (br.first >= br.second) continue;
+          const int last = strip_of[L[i].col_off + L[i].n - 1];
+          for (int st = strip_of[L[i].col_off]; st <= last; ++st) round_parts[st] += br.second - br.first;
+        }
+        for (size_t st = 0; st < strips.size(); ++st) {
+          if (!round_parts[st]) continue;
+          const int len = strips[st].len;
+          zred.push_back(GemvZred{part_row[st], (unsigned short)len, (unsigned short)summed[st], (int)slot, round_parts[st]});
+          summed[st] = 1;
+          first_slot[st] = (int)slot;
+          slot += (long long)round_parts[st] * len;
         }
       }
-      for (int b = br.first; b < br.second; ++b) {
-        int* m = &colmap[(size_t)colbase[b] + layout_.pcol[layout_.first[i] + (b - br.first)]];
-        used[b] += w;
+      std::fill(taken.begin(), taken.end(), 0);
+      for (int i = 0; i < (int)L.size(); ++i) {
+        if (layout_.first[i] < 0) continue;
+        const auto all = row_blocks(L[i].row_off, L[i].m), br = blocks_of(i);
+        if (br.first >= br.second) continue;
+        const int nb = br.second - br.first, w = L[i].type == 0 ? L[i].n : ranks[i];
+        int zrow = 0;
         if (L[i].type != 0) {
-          for (int j = 0; j < w; ++j) m[j] = zrow + (b - br.first) * w + j;
-          continue;
+          const GemvRkLeaf& k = K[rk_index[i]];
+          zrow = k.zrow_t;
+          if (all.second - all.first > 1) {  // parts, one per row block, summed into the leaf's z' rows
+            zred.push_back(GemvZred{zrow, (unsigned short)w, (unsigned short)(all.first < cut.first), (int)slot, nb});
+            zrow = (int)slot;
+            slot += (long long)nb * w;
+          }
         }
-        for (int j = 0; j < w;) {
-          const int c = L[i].col_off + j, st = strip_of[c], e = std::min(w - j, strips[st].off + strips[st].len - c);
-          const int row = part_row[st] + taken[st]++ * strips[st].len + (c - strips[st].off);
-          for (int q = 0; q < e; ++q) m[j + q] = row + q;
-          j += e;
+        for (int b = br.first; b < br.second; ++b) {
+          int* m = &colmap[(size_t)colbase[b] + layout_.pcol[layout_.first[i] + (b - all.first)]];
+          if (L[i].type != 0) {
+            for (int j = 0; j < w; ++j) m[j] = zrow + (b - br.first) * w + j;
+            continue;
+          }
+          for (int j = 0; j < w;) {
+            const int c = L[i].col_off + j, st = strip_of[c], e = std::min(w - j, strips[st].off + strips[st].len - c);
+            const int row = first_slot[st] + taken[st]++ * strips[st].len + (c - strips[st].off);
+            for (int q = 0; q < e; ++q) m[j + q] = row + q;
+            j += e;
+          }
         }
       }
-    }
-    side.nzwide = wide_sums_first(zred);
-    const int first = (int)units.size();
-    std::vector<int> owner;
-    int stage = 32, omax = 1;
-    for (size_t b = 0; b < rblocks_.size(); ++b) {
-      const int O = rblocks_[b].len;
-      // CW columns where the piece stays small, twice that for short blocks, else as many CL-wide
-      // groups as fit
-      int cols = std::max(1, kTransPieceBytes / (O * s * CL)) * CL;
-      cols = cols >= 2 * CW && O * s * 2 * CW <= kTransPieceBytes / 2 ? 2 * CW : std::min(cols, CW);
-      for (int j0 = 0; j0 < used[b]; j0 += cols) {
-        GemvTransUnit u{};
-        u.poff = layout_.yblock[b] + (long long)j0 * O;
-        u.x = (int)(colbase[b] + j0);
-        u.rows = (unsigned char)O;
-        u.cols = (unsigned char)std::min(cols, used[b] - j0);
-        if (u.poff % kPad) throw Error("gemv plan: misaligned block piece");
-        units.push_back(u);
-        owner.push_back((int)b);
-        stage = std::max(stage, (O * u.cols * s + 15) / 16 * 16 + (u.cols * 4 + 15) / 16 * 16);
-        omax = std::max(omax, O);
+      next_row = std::max(next_row, slot);
+      round.nzwide = wide_sums_first(zred, round.zred0);
+      round.nzred = (int)zred.size() - round.zred0;
+      const int first = (int)units.size();
+      std::vector<int> owner;
+      int stage = 32, omax = 1;
+      for (int b = cut.first; b < cut.second; ++b) {
+        const int O = rblocks_[b].len;
+        // CW columns where the piece stays small, twice that for short blocks, else as many CL-wide
+        // groups as fit
+        int cols = std::max(1, kTransPieceBytes / (O * s * CL)) * CL;
+        cols = cols >= 2 * CW && O * s * 2 * CW <= kTransPieceBytes / 2 ? 2 * CW : std::min(cols, CW);
+        for (int j0 = 0; j0 < used[b]; j0 += cols) {
+          GemvTransUnit u{};
+          u.poff = layout_.yblock[b] + (long long)j0 * O;
+          u.x = (int)(colbase[b] + j0);
+          u.rows = (unsigned char)O;
+          u.cols = (unsigned char)std::min(cols, used[b] - j0);
+          if (u.poff % kPad) throw Error("gemv plan: misaligned block piece");
+          units.push_back(u);
+          owner.push_back(b);
+          stage = std::max(stage, (O * u.cols * s + 15) / 16 * 16 + (u.cols * 4 + 15) / 16 * 16);
+          omax = std::max(omax, O);
+        }
       }
-    }
-    side.nz = 0;
-    if (!owner.empty()) {
-      GemvLaunch& l = side.z[0];
-      l = GemvLaunch();
-      l.piece_bytes = stage;
-      l.xrows = omax;
-      // x rows padded by 16 bytes where the kernel pads them
-      l.ncta = std::min((int)owner.size(), trans_ctas(trans_columns_smem(stage, omax, RS16 * s + 16)));
-      std::vector<GemvTask> ct;
-      std::vector<int> cblock, cbegin;
-      cut_tasks(units, first, owner, l.ncta, ct, cblock, cbegin);
-      for (size_t t = 0; t < ct.size(); ++t) {
-        ct[t].O = rblocks_[cblock[t]].len;
-        ct[t].out_row = rblocks_[cblock[t]].off;  // the block's x rows
+      if (!owner.empty()) {
+        GemvLaunch& l = round.columns;
+        l.piece_bytes = stage;
+        l.xrows = omax;
+        // x rows padded by 16 bytes where the kernel pads them
+        l.ncta = std::min((int)owner.size(), trans_ctas(trans_columns_smem(stage, omax, RS16 * s + 16)));
+        std::vector<int> cblock, cbegin;
+        const size_t t0 = ct.size();
+        cut_tasks(units, first, owner, l.ncta, ct, cblock, cbegin);
+        for (size_t t = t0; t < ct.size(); ++t) {
+          ct[t].O = rblocks_[cblock[t - t0]].len;
+          ct[t].out_row = rblocks_[cblock[t - t0]].off;  // the block's x rows
+        }
+        l.ntasks = (int)(ct.size() - t0);
+        sp.round_begin.push_back((int)sp.begin[0].size());
+        sp.begin[0].insert(sp.begin[0].end(), cbegin.begin(), cbegin.end());
+      } else {
+        sp.round_begin.push_back(0);
       }
-      l.ntasks = (int)ct.size();
-      sp.tasks[0].swap(ct);
-      sp.begin[0].swap(cbegin);
-      side.nz = 1;
+      side.rounds.push_back(round);
     }
+    sp.tasks[0].swap(ct);
     for (int c = 0; c < side.ng; ++c) {
       side.g[c].ntasks = (int)gt[c].size();
       sp.tasks[GemvSide::kMaxLaunch + c].swap(gt[c]);
@@ -2670,11 +2737,26 @@ class Engine : public EngineBase {
     noalloc_rows_ = bound_rows + noalloc_trans_rows(K);
   }
 
+  // Rows a transposed product may take, at the widest tile of right-hand sides: the array of the
+  // allocation-free products for every matrix that may be within their bound (a column of a block
+  // took a sixteenth of a slot when the bound was set); for larger ones a GiB, or half the leaves'
+  // bytes (only blocks of fewer than 32 rows need more).  A round costs a product with one
+  // right-hand side two launches, 5 us, and one with 16 nothing, the sums then reading the parts
+  // from L2: 20,000-point cube, FP64, leaves of 32, one round against two 164 and 170 us, 494 and
+  // 418 us; FP32, leaves of 16, one round against four 107 and 122 us, 243 and 235 us.
+  static constexpr long long kTransBudgetBytes = 1LL << 30;
+  long long trans_row_budget(const std::vector<GemvRkLeaf>& K) const {
+    const long long s = (long long)sizeof(T), row = gemv_rhs_stride((int)s, s >= 16 ? 4 : 16) * s;
+    const long long bound = (plan_.n_in_max + kZeroRows + noalloc_trans_rows(K)) * gemv_rhs_stride((int)s, 16) * s;
+    if (bound <= kNoAllocBoundBytes) return kNoAllocArrayBytes / row;
+    return std::max(kTransBudgetBytes, layout_.total * s / 2) / row;
+  }
+
   // The bound of the allocation-free products is stated in rows of one buffer for both
   // directions, with z chunks of 16 units (the tuner's, of a tuned matrix), a part of y per warp of
   // the full grid, and the partial rows of transposed products that took a slot per 16 units of 32
   // columns: callers know which matrices it takes, so it stays, although the products now use
-  // their scratch differently (gemv_device_with_scratch).
+  // their scratch differently (trans_row_budget, small_zparts).
   long long noalloc_trans_rows(const std::vector<GemvRkLeaf>& K) const {
     const auto& L = bt_->leaves;
     const long long kUnits = 16;
@@ -2761,7 +2843,21 @@ class Engine : public EngineBase {
     GemvLaunch l;
     warp_shape(l, omax);
     const long long warps = (long long)launch_ctas(l.map == 3 ? 8 * l.rpt : omax, l.map) * warp_stream_warps_per_cta();
-    return (int)std::max(1LL, std::min(16LL, (units + warps - 1) / warps));
+    long long chunk = std::max(1LL, std::min(16LL, (units + warps - 1) / warps));
+    // the parts' rows stay within what the array of the allocation-free products has beyond their bound
+    const long long row = gemv_rhs_stride((int)sizeof(T), 16) * (long long)sizeof(T);
+    auto part_rows = [&]() {
+      long long rows = 0;
+      for (const ZGroup& g : layout_.zgroups) {
+        int xoff = 0;
+        const int zc = kTensorN ? mma_unit_cols(g.h, &xoff) : warp_unit_cols_wide(g.h, &xoff);
+        const long long nu = (g.n + zc - 1) / zc;
+        if (nu > chunk) rows += (nu + chunk - 1) / chunk * g.h;
+      }
+      return rows;
+    };
+    while (chunk < 16 && part_rows() * row > kNoAllocArrayBytes - kNoAllocBoundBytes) chunk = std::min(16LL, 2 * chunk);
+    return (int)chunk;
   }
 
   // The products' schedules; products can run afterwards.

@@ -1389,6 +1389,14 @@ __device__ __forceinline__ void zred_parts(const T* part, int k, int c, int p0, 
       }
   }
 }
+// The sum so far, of the rounds before this one.
+template <typename T, int V>
+__device__ __forceinline__ void zred_add(const T* fin, T (&s)[V]) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(fin);
+  const T* v = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+  for (int e = 0; e < V; ++e) s[e] = v[e] + s[e];
+}
 template <typename T, int RS>
 __global__ void __launch_bounds__(kZredWarps * 32) zred_kernel(const GemvZred* __restrict__ zr, int n, int nwide, T* xz) {
   constexpr int V = sizeof(T) >= 16 ? 1 : 16 / (int)sizeof(T);
@@ -1417,6 +1425,7 @@ __global__ void __launch_bounds__(kZredWarps * 32) zred_kernel(const GemvZred* _
 #pragma unroll
           for (int e = 0; e < V; ++e) s[e] = s[e] + v[e];
         }
+        if (d.add) zred_add<T, V>(fin + (size_t)c * V, s);
         *reinterpret_cast<uint4*>(fin + (size_t)c * V) = *reinterpret_cast<const uint4*>(s);
       }
       __syncthreads();
@@ -1432,6 +1441,7 @@ __global__ void __launch_bounds__(kZredWarps * 32) zred_kernel(const GemvZred* _
   for (int c = lane; c < nchunk; c += 32) {
     T s[V];
     zred_parts<T, RS>(part, d.k, c, 0, d.nparts, s);
+    if (d.add) zred_add<T, V>(fin + (size_t)c * V, s);
     *reinterpret_cast<uint4*>(fin + (size_t)c * V) = *reinterpret_cast<const uint4*>(s);
   }
 }
@@ -1533,26 +1543,27 @@ void allow_smem(F kern, bool& done) {
 }
 
 template <typename T, int RS>
-void launch_zred(const GemvSide& side, T* xz, cudaStream_t s) {
-  if (side.nzred > 0)
-    launch_pdl(zred_kernel<T, RS>, dim3(zred_grid(side.nzred, side.nzwide)), dim3(kZredWarps * 32), 0, s, side.zred,
-               side.nzred, side.nzwide, xz);
+void launch_zred(const GemvZred* zred, int n, int nwide, T* xz, cudaStream_t s) {
+  if (n > 0)
+    launch_pdl(zred_kernel<T, RS>, dim3(zred_grid(n, nwide)), dim3(kZredWarps * 32), 0, s, zred, n, nwide, xz);
 }
 
-// The column pass of the transposed products and its z' sums: afterwards xz holds the z' rows of
-// every Rk leaf and the full leaves' partial rows of y.
+// The column pass of the transposed products and its sums, round by round: afterwards xz holds the
+// z' rows of every Rk leaf and the full leaves' partial rows of y.
 template <typename T, int R, int RS>
 void run_trans_columns(const GemvSide& side, const T* arena, T* xz, int conj, GemvStatus* err, cudaStream_t s) {
-  const GemvLaunch& L = side.z[0];
-  if (side.nz > 0 && L.ntasks > 0) {
-    auto kern = trans_columns_kernel<T, R, RS>;
-    static bool attr = false;
-    allow_smem(kern, attr);
-    launch_pdl(kern, dim3(L.ncta), dim3(kTransWarps * 32),
-               trans_columns_smem(L.piece_bytes, L.xrows, trans_xstride<T, RS>() * (int)sizeof(T)), s, L.tasks,
-               L.cta_begin, side.tunits, side.colmap, arena, xz, conj, L.piece_bytes, L.xrows, err);
+  for (const GemvTransRound& round : side.rounds) {
+    const GemvLaunch& L = round.columns;
+    if (L.ntasks > 0) {
+      auto kern = trans_columns_kernel<T, R, RS>;
+      static bool attr = false;
+      allow_smem(kern, attr);
+      launch_pdl(kern, dim3(L.ncta), dim3(kTransWarps * 32),
+                 trans_columns_smem(L.piece_bytes, L.xrows, trans_xstride<T, RS>() * (int)sizeof(T)), s, L.tasks,
+                 L.cta_begin, side.tunits, side.colmap, arena, xz, conj, L.piece_bytes, L.xrows, err);
+    }
+    launch_zred<T, RS>(side.zred + round.zred0, round.nzred, round.nzwide, xz, s);
   }
-  launch_zred<T, RS>(side, xz, s);
 }
 
 template <typename T, int R, int RS>
@@ -1586,7 +1597,7 @@ void run_tile(const GemvPlan& p, int nrhs, int q0, T alpha, T beta, const T* x, 
   } else {
     for (int c = 0; c < side.nz; ++c)
       launch_stream<T, R, RS>(side.z[c], side.units, arena, xz, err, s);
-    launch_zred<T, RS>(side, xz, s);
+    launch_zred<T, RS>(side.zred, side.nzred, side.nzwide, xz, s);
   }
   if (tm) cudaEventRecord(tm->ev[2], s);
   if constexpr (TRANSP)
@@ -1601,13 +1612,12 @@ void run_tile(const GemvPlan& p, int nrhs, int q0, T alpha, T beta, const T* x, 
   if (tm) cudaEventRecord(tm->ev[3], s);
 }
 
-// Right-hand sides are taken in tiles of at most max_tile (16, 12, 8, 4 or 1; complex double never
-// more than 4: its accumulators).
+// Right-hand sides are taken in tiles of 16, 12, 8, 4 or 1 (complex double 4 or 1: its
+// accumulators).
 template <typename T, bool TRANSP>
 void run_all(const GemvPlan& p, int nrhs, T alpha, T beta, const T* x, T* y, T* xz, int conj, GemvStatus* err,
-             cudaStream_t s, const GemvTiming* tm, int max_tile) {
+             cudaStream_t s, const GemvTiming* tm) {
   constexpr int maxR = sizeof(T) >= 16 ? 4 : 16;
-  const int most = max_tile < maxR ? max_tile : maxR;
   int tile;
   for (int q0 = 0; q0 < nrhs; q0 += tile) {
     const int rem = nrhs - q0;
@@ -1616,16 +1626,16 @@ void run_all(const GemvPlan& p, int nrhs, T alpha, T beta, const T* x, T* y, T* 
     // whose tensor-core tiles hold 16 anyway): 60,000-point cylinder, FP64, 11 right-hand sides
     // 387 -> 292 us
     constexpr bool has12 = sizeof(T) == 8 || (sizeof(T) == 4 && TRANSP);
-    if (has12 && most >= 16 && rem > 8 && rem <= 12) {
+    if (has12 && rem > 8 && rem <= 12) {
       tile = 12;
       run_tile<T, (has12 ? 12 : 4), TRANSP>(p, nrhs, q0, alpha, beta, x, y, xz, conj, err, s, tm);
-    } else if (most >= 16 && rem > 8) {
+    } else if (maxR == 16 && rem > 8) {
       tile = 16;
       run_tile<T, (maxR >= 16 ? 16 : 4), TRANSP>(p, nrhs, q0, alpha, beta, x, y, xz, conj, err, s, tm);
-    } else if (most >= 8 && rem > 4) {
+    } else if (maxR == 16 && rem > 4) {
       tile = 8;
       run_tile<T, (maxR >= 16 ? 8 : 4), TRANSP>(p, nrhs, q0, alpha, beta, x, y, xz, conj, err, s, tm);
-    } else if (most >= 4 && rem > 1) {
+    } else if (rem > 1) {
       tile = 4;
       run_tile<T, 4, TRANSP>(p, nrhs, q0, alpha, beta, x, y, xz, conj, err, s, tm);
     } else {
@@ -1725,7 +1735,7 @@ void forward_z(const GemvPlan& p, int nrhs, const T* x, T* xz, GemvStatus* err, 
                                                                 p.n_in_max);
   for (int c = 0; c < sn.nz; ++c)
     launch_stream<T, R, RS>(sn.z[c], sn.units, (const T*)p.arena, xz, err, s);
-  launch_zred<T, RS>(sn, xz, s);
+  launch_zred<T, RS>(sn.zred, sn.nzred, sn.nzwide, xz, s);
 }
 template <typename T, int R>
 void grads_outer(const GemvPlan& p, const T* xz, const T* rz, T* gfull, T* grk, bool accumulate, cudaStream_t s) {
@@ -1789,6 +1799,7 @@ int gemv_launch_count(const GemvPlan& p, char trans, int nrhs, int elem_bytes) {
   int per_tile = 1;  // gather
   for (int c = 0; c < side.nz; ++c) per_tile += side.z[c].ntasks > 0;
   per_tile += side.nzred > 0;
+  for (const GemvTransRound& r : side.rounds) per_tile += (r.columns.ntasks > 0) + (r.nzred > 0);
   per_tile += side.y.ntasks > 0;
   for (int c = 0; c < side.ng; ++c) per_tile += side.g[c].ntasks > 0;
   per_tile += side.nyrows > 0;  // final pass
@@ -1818,16 +1829,16 @@ void launch_gemv_adjoint(const GemvPlan& p, int nrhs, const T* x, const T* r, T*
 
 template <typename T>
 void launch_gemv(const GemvPlan& p, char trans, int nrhs, T alpha, T beta, const T* x_client, T* y_client, T* xz,
-                 GemvStatus* err, cudaStream_t s, const GemvTiming* tm, int max_tile) {
-  if (trans == 'N') run_all<T, false>(p, nrhs, alpha, beta, x_client, y_client, xz, 0, err, s, tm, max_tile);
+                 GemvStatus* err, cudaStream_t s, const GemvTiming* tm) {
+  if (trans == 'N') run_all<T, false>(p, nrhs, alpha, beta, x_client, y_client, xz, 0, err, s, tm);
   else
     run_all<T, true>(p, nrhs, alpha, beta, x_client, y_client, xz, (trans == 'C' && Traits<T>::is_complex) ? 1 : 0,
-                     err, s, tm, max_tile);
+                     err, s, tm);
 }
 
 #define HB_INST(T)                                                                                            \
   template void launch_gemv<T>(const GemvPlan&, char, int, T, T, const T*, T*, T*, GemvStatus*, cudaStream_t,         \
-                               const GemvTiming*, int);                                                             \
+                               const GemvTiming*);                                                             \
   template void launch_leaf_gradients<T>(const GemvPlan&, int, const T*, const T*, T*, T*, T*, T*, bool, GemvStatus*, \
                                          cudaStream_t);                                                                  \
   template void launch_gemv_adjoint<T>(const GemvPlan&, int, const T*, const T*, T*, T*, T*, T*, T*, bool, GemvStatus*, \

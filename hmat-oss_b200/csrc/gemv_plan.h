@@ -14,6 +14,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 namespace hmatb200 {
 
 // X rows of a unit come from at most kUnitRuns runs of consecutive xz rows (the columns of a
@@ -119,27 +121,44 @@ constexpr int kWarpXBytes = 2048;
 // other way, kWarpXBytesWide bytes of X rows after a piece of the rest.
 constexpr int kWarpXBytesWide = 3584;
 
-// A long group or leaf whose z is computed in several parts: the parts' slots
-// (nparts consecutive slots of k rows from part_row) are summed into final_row.
+// A sum of partial slots (a long group's or leaf's z, a strip's y): nparts consecutive slots of k
+// rows from part_row are summed into final_row, with add != 0 on top of what stands there.
 struct GemvZred {
-  int final_row, k, part_row, nparts;
+  int final_row;
+  unsigned short k, add;
+  int part_row, nparts;
+};
+
+// The allocation-free products (noalloc.cu) take a matrix by a bound on its rows; every matrix
+// within the bound is planned so that its rows, at the widest tile of right-hand sides, fit the
+// array those products use.
+constexpr long long kNoAllocBoundBytes = 16LL << 20;
+constexpr long long kNoAllocArrayBytes = 40LL << 20;
+
+// A round of the 'T' column pass: consecutive output blocks, then the sums [zred0, zred0 + nzred) of
+// its partial slots, the first nzwide of them on a CTA each.  The rounds use the same slots.
+struct GemvTransRound {
+  GemvLaunch columns;
+  int zred0 = 0, nzred = 0, nzwide = 0;
 };
 
 struct GemvSide {
   static const int kMaxLaunch = 4;
-  int nz = 0;  // 'N': z-phase launches (one per rank class); 'T': the column pass
+  int nz = 0;  // 'N': z-phase launches (one per rank class)
   GemvLaunch z[kMaxLaunch];
-  int nzred = 0;
-  int nzwide = 0;  // sums at the front of zred that take a CTA each
+  int nzred = 0;   // 'N'
+  int nzwide = 0;  // 'N': sums at the front of zred that take a CTA each
   const GemvZred* zred = nullptr;
+  std::vector<GemvTransRound> rounds;  // 'T'
   const int* colmap = nullptr;  // 'T': destination rows of the column pass
   int ng = 0;                   // 'T': group-pass launches (one per group height class)
   GemvLaunch g[2];
   GemvLaunch y;  // 'N'
   const GemvUnit* units = nullptr;         // 'N'
   const GemvTransUnit* tunits = nullptr;   // 'T'
-  // The y launches, the group pass and the column pass (full leaves) write partial rows of the
-  // output blocks into xz; the final pass reads, per client row i, yrows[i] = {xz row of part 0, nparts << 8 | O}.
+  // The y launches, the group pass and the column pass (full leaves; with several rounds, the sum of
+  // their parts) write partial rows of the output blocks into xz; the final pass reads, per client
+  // row i, yrows[i] = {xz row of part 0, nparts << 8 | O}.
   int nyrows = 0;
   const int2* yrows = nullptr;
 };

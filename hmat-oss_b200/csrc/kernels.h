@@ -190,12 +190,13 @@ void launch_tsapply_cta(const TsItem* items, int nitems, T* ws, const typename T
 }  // namespace hmatb200
 #include "gemv_plan.h"
 namespace hmatb200 {
-// y = alpha op(H) x + beta y on device buffers (client numbering), right-hand sides in tiles of at
-// most max_tile (16, 8, 4 or 1); `xz` is the scratch buffer of the side's rows (plan.xz_rows) of
-// gemv_rhs_stride(sizeof(T), max_tile) scalars; `err` is set when a pipeline wait gives up.
+// y = alpha op(H) x + beta y on device buffers (client numbering), right-hand sides in tiles of 16,
+// 12, 8, 4 or 1 (complex double: 4 or 1); `xz` is the scratch buffer of the side's rows
+// (plan.xz_rows) of gemv_rhs_stride(sizeof(T), 16 or 4) scalars; `err` is set when a pipeline wait
+// gives up.
 template <typename T>
 void launch_gemv(const GemvPlan& p, char trans, int nrhs, T alpha, T beta, const T* x_client, T* y_client, T* xz,
-                 GemvStatus* err, cudaStream_t s, const GemvTiming* timing = nullptr, int max_tile = 16);
+                 GemvStatus* err, cudaStream_t s, const GemvTiming* timing = nullptr);
 // Row stride (scalars) of the xz buffer for R right-hand sides.
 int gemv_rhs_stride(int elem_bytes, int R);
 // Kernel launches of one product with nrhs right-hand sides.

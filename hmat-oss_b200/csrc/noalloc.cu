@@ -14,6 +14,7 @@
 #include <string>
 
 #include "engine.h"
+#include "gemv_plan.h"
 #include "hmat_b200.h"
 
 namespace hmatb200 {
@@ -26,13 +27,10 @@ using namespace hmatb200;
 namespace {
 
 // A matrix is taken when its gemv_scratch_bytes (the cluster-ordered x, N x 16 scalars, plus the
-// z buffer) are at most 16 MiB.  The array is larger: a transposed product of such a matrix runs
-// in the widest tile of right-hand sides whose partial rows fit it, and at one right-hand side
-// the rows of an FP32 matrix of mostly full leaves take up to about 18 MB.
+// z buffer) are at most kNoAllocBoundBytes.  The array is larger: the products' partial rows are
+// planned to fit it (a transposed product in rounds where they would not at once).
 // The address looked up for a device stays valid for the life of the process's context on
 // that device; a cudaDeviceReset (which destroys that context) is not supported.
-constexpr size_t kNoAllocScratchBytes = 16u << 20;
-constexpr size_t kNoAllocArrayBytes = 24u << 20;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocArrayBytes];
 
 constexpr int kMaxDevices = 64;
@@ -62,9 +60,9 @@ extern "C" int hmat_b200_gemv_device_noalloc(hmat_matrix_t* m, char trans, const
     EngineBase* e = existing_engine(m);
     if (!e || !e->assembled) throw Error("matrix is not assembled");
     const size_t need = e->gemv_scratch_bytes();
-    if (need > kNoAllocScratchBytes)
+    if (need > (size_t)kNoAllocBoundBytes)
       throw Error("matrix needs " + std::to_string(need) + " bytes of gemv scratch, more than the " +
-                  std::to_string(kNoAllocScratchBytes) + " bytes this entry point holds; use hmat_b200_gemv_device");
+                  std::to_string(kNoAllocBoundBytes) + " bytes this entry point holds; use hmat_b200_gemv_device");
     // the scratch address is looked up on the matrix's own device, which must be current
     int dev = 0;
     cudaError_t ce = cudaGetDevice(&dev);

@@ -408,10 +408,10 @@ int hmat_b200_gemv_status(hmat_matrix_t* hmatrix, void* stream, int* failed);
  * cudaFree would synchronise or deadlock, or in loops that forbid allocation after
  * start-up can use it: it calls no cudaMalloc, cudaFree or other allocating routine.
  * Its scratch (x in cluster order and the per-leaf B^T x values) is
- * one fixed 24 MiB device array compiled into the library: every GPU on which the
+ * one fixed 40 MiB device array compiled into the library: every GPU on which the
  * library's device code is loaded holds it until the process exits.  Matrices whose
- * vectors and B^T x values (the two directions in one buffer, at 16 right-hand sides, 4 for
- * complex FP64) take more than 16 MiB are rejected with a non-zero return and an error
+ * vectors and B^T x values (the two directions in one buffer, at 16 scalars a row for every
+ * type) take more than 16 MiB are rejected with a non-zero return and an error
  * message (use hmat_b200_gemv_device for them).  The first call on each device
  * looks up the array's device address (with that device current); make that first call
  * before any stream capture.  Every call shares the one array, so calls that can overlap
