@@ -177,6 +177,10 @@ void launch_tsapply(int K, const TsItem* items, int nitems, T* ws, const typenam
 template <typename T>
 void launch_tsqr_cta(const TsItem* items, int nitems, const T* ws, typename Traits<T>::wide* tri, bool from_tri,
                      typename Traits<T>::wide* scratch, long long slab, int grid, int* counter, cudaStream_t s);
+// Variant of the core kernel for a leaf of rank k: shared memory up to 32, 64 or 96 columns (0 to 2),
+// or the slab (3).  A launch takes the leaves of one class, kmax their largest rank.
+template <typename T>
+int tscore_cta_class(int k);
 template <typename T>
 void launch_tscore_cta(const TsCore* items, int nitems, int kmax, const typename Traits<T>::wide* tri,
                        typename Traits<T>::wide* maps, int* ranks, int* status, double eps,

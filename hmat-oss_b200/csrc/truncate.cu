@@ -1345,7 +1345,9 @@ __global__ void __launch_bounds__(kTruncThreads) tsqr_cta_kernel(const TsItem* _
 // With H > 0 the core's matrix and V sit in shared memory and a Jacobi pair takes 16 lanes
 // (8 of them complex; jacobi_svd_lanes: the arithmetic of jacobi_svd), for cores of at most 32 H
 // columns and as many threads as all pairs take up to 64 columns; with H = 0, on the slab with a warp a pair
-// (30,000-point Helmholtz cylinder, ranks 17 to 63: 9.9 ms, 4.9 ms in shared memory).
+// (30,000-point Helmholtz cylinder, ranks 17 to 63: 9.9 ms, 4.9 ms in shared memory).  A core's
+// variant is that of its own rank (tscore_cta_class: at most 96 columns, complex 82, whose two
+// matrices fill the shared memory), so that its factors do not depend on the leaves beside it.
 template <typename W>
 __host__ __device__ constexpr int tscore_cta_threads(int H) {
   return H == 0 ? kTruncThreads : jacobi_threads<W>(H);
@@ -1710,12 +1712,21 @@ void launch_tsqr_cta(const TsItem* items, int nitems, const T* ws, typename Trai
   else
     tsqr_cta_kernel<W, T><<<g, kTruncThreads, 0, s>>>(items, nitems, ws, tri, scratch, slab, counter);
 }
+template <typename W>
+constexpr size_t tscore_cta_smem(int k) {
+  return (2 * (size_t)k * k) * sizeof(W) + (size_t)k * (sizeof(double) + sizeof(int));
+}
+template <typename T>
+int tscore_cta_class(int k) {
+  if (k > 96 || tscore_cta_smem<typename Traits<T>::wide>(k) > kDenseJacobiSmem) return 3;
+  return k > 64 ? 2 : (k > 32 ? 1 : 0);
+}
 template <typename T>
 void launch_tscore_cta(const TsCore* items, int nitems, int kmax, const typename Traits<T>::wide* tri,
                        typename Traits<T>::wide* maps, int* ranks, int* status, double eps,
                        typename Traits<T>::wide* scratch, long long slab, int grid, int* counter, cudaStream_t s) {
   typedef typename Traits<T>::wide W;
-  const size_t smem = (2 * (size_t)kmax * kmax) * sizeof(W) + (size_t)kmax * (sizeof(double) + sizeof(int));
+  const size_t smem = tscore_cta_smem<W>(kmax);
   auto run = [&](auto kern, int threads, size_t bytes) {
     if (nitems <= 0) {
       cudaFuncAttributes a;
@@ -1739,14 +1750,13 @@ void launch_tscore_cta(const TsCore* items, int nitems, int kmax, const typename
     run(tscore_cta_kernel<W, 1>, 0, 0);
     run(tscore_cta_kernel<W, 2>, 0, 0);
     run(tscore_cta_kernel<W, 3>, 0, 0);
-  } else if (kmax > 96 || smem > kDenseJacobiSmem) {
-    run(tscore_cta_kernel<W, 0>, tscore_cta_threads<W>(0), 0);
-  } else if (kmax > 64) {
-    run(tscore_cta_kernel<W, 3>, tscore_cta_threads<W>(3), smem);
-  } else if (kmax > 32) {
-    run(tscore_cta_kernel<W, 2>, tscore_cta_threads<W>(2), smem);
   } else {
-    run(tscore_cta_kernel<W, 1>, tscore_cta_threads<W>(1), smem);
+    switch (tscore_cta_class<T>(kmax)) {
+      case 0: run(tscore_cta_kernel<W, 1>, tscore_cta_threads<W>(1), smem); break;
+      case 1: run(tscore_cta_kernel<W, 2>, tscore_cta_threads<W>(2), smem); break;
+      case 2: run(tscore_cta_kernel<W, 3>, tscore_cta_threads<W>(3), smem); break;
+      default: run(tscore_cta_kernel<W, 0>, tscore_cta_threads<W>(0), 0); break;
+    }
   }
 }
 template <typename T>
@@ -1806,6 +1816,7 @@ void preload_truncate_kernels() {
   template void preload_truncate_kernels<T>();                                                            \
   template void launch_tsqr_cta<T>(const TsItem*, int, const T*, typename Traits<T>::wide*, bool,            \
                                    typename Traits<T>::wide*, long long, int, int*, cudaStream_t);         \
+  template int tscore_cta_class<T>(int);                                                                   \
   template void launch_tscore_cta<T>(const TsCore*, int, int, const typename Traits<T>::wide*,                    \
                                      typename Traits<T>::wide*, int*, int*, double, typename Traits<T>::wide*, \
                                      long long, int, int*, cudaStream_t);                                  \
