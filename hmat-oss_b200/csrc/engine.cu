@@ -9,6 +9,7 @@
 #include <mutex>
 #include <numeric>
 #include <string>
+#include <system_error>
 #include <tuple>
 #include <type_traits>
 #include <unordered_map>
@@ -2735,13 +2736,15 @@ class Engine : public EngineBase {
       std::future<void> trans;
       auto build_trans = [&] { build_trans_side(K, rk_leaf, next_row[1], plan_.side[1], sp[1]); };
       // a thread costs about as much to start as the side of a matrix of four million scalars
-      const bool beside = !only_n && layout_.total > (4LL << 20);
-      if (beside)
-        trans = std::async(std::launch::async, build_trans);
-      else if (!only_n)
-        build_trans();
+      if (!only_n && layout_.total > (4LL << 20)) {
+        try {
+          trans = std::async(std::launch::async, build_trans);
+        } catch (const std::system_error&) {  // no thread to be had: one side after the other
+        }
+      }
+      if (!only_n && !trans.valid()) build_trans();
       build_side(K, rk_leaf, next_row[0], bound_rows, plan_.side[0], sp[0]);
-      if (beside) trans.get();
+      if (trans.valid()) trans.get();
       upload_side(sp[0], plan_.side[0], side_buf_[0]);
       if (!only_n) upload_side(sp[1], plan_.side[1], side_buf_[1]);
       HB_CUDA(cudaStreamSynchronize(stream_));  // the host vectors go out of scope

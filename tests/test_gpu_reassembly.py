@@ -96,3 +96,37 @@ def test_other_ranks_with_products_in_flight(hb, vt):
                 fresh.close()
     finally:
         h.close()
+
+
+NO_THREADS = r"""
+import ctypes, sys
+sys.path.insert(0, "tests")
+import conftest
+import numpy as np
+hb = conftest.load_engine_package()
+hb.set_parameters(compressionMinLeafSize=0)
+pts = np.random.default_rng(0).random((8000, 3))
+h = hb.HMatrix(pts, hb.kernel(hb.EXP_COV, ell=0.3, nugget=1e-6), leaf_size=64, eta=2.0, epsilon=1e-4)
+assert h.payload_layout()[1] > 4 << 20  # large enough to be planned on two threads
+x = np.random.default_rng(1).standard_normal((8000, 2))
+want = h.gemv(x), h.gemv(x, trans="T")
+libc = ctypes.CDLL(None)
+attr = ctypes.create_string_buffer(256)
+assert libc.pthread_attr_init(attr) == 0
+assert libc.pthread_attr_setstacksize(attr, ctypes.c_size_t(1 << 47)) == 0
+assert libc.pthread_setattr_default_np(attr) == 0  # no further thread can be started: its stack cannot be mapped
+h.assemble()
+got = h.gemv(x), h.gemv(x, trans="T")
+assert all(np.array_equal(a, b) for a, b in zip(got, want))
+h.close()
+print("assembled")
+"""
+
+
+def test_assembly_where_no_thread_can_be_started():
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+    r = subprocess.run([sys.executable, "-c", NO_THREADS], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "assembled" in r.stdout, r.stderr[-2000:]
