@@ -1894,15 +1894,13 @@ class Engine : public EngineBase {
     return wide;
   }
 
-  // Tensor-core units (FP32, FP64): the widest multiple of the kernel's column step (8 for the
-  // TF32 MMA, 4 for the FP64 one) whose piece (O x c) and X rows (c rows of 16 scalars) fit
-  // one pipeline stage, the X rows right after the piece (16-byte aligned); *xoff is their
-  // offset in the stage.
+  // Tensor-core units (FP32): the widest multiple of the TF32 MMA's 8 columns whose piece (O x c)
+  // and X rows (c rows of 16 scalars) fit one pipeline stage, the X rows right after the piece
+  // (16-byte aligned); *xoff is their offset in the stage.
   static int mma_unit_cols(int O, int* xoff) {
-    const int s = (int)sizeof(T);
+    const int s = 4, step = 8;
     const int stage = warp_piece_bytes(s) + kWarpXBytes;
     const int xrow = gemv_rhs_stride(s, 16) * s;
-    const int step = s == 4 ? 8 : 4;
     auto need = [&](int c) { return (((long long)O * c * s + 15) / 16) * 16 + (long long)c * xrow; };
     int c = step;
     while (need(c + step) <= stage) c += step;
@@ -1936,7 +1934,7 @@ class Engine : public EngineBase {
     // kernels' launch bounds guarantee the registers for that many CTAs)
     const size_t alloc = (smem + 127) / 128 * 128;
     int per_sm = (int)std::min<size_t>(8, (228 * 1024) / (alloc + 1024));
-    if (map == 3) per_sm = std::min(per_sm, mma_stream_blocks_per_sm(omax / 8, (int)sizeof(T)));  // registers
+    if (map == 3) per_sm = std::min(per_sm, mma_stream_blocks_per_sm());  // registers
     per_sm = std::max(per_sm, 1);
     return persistent_grid(per_sm);
   }
@@ -2712,8 +2710,6 @@ class Engine : public EngineBase {
       }
     }
     if (!d_perm_rows_.p || !d_perm_cols_.p) throw Error("gemv plan: cluster permutations are not on the device");
-    plan_.perm_rows = d_perm_rows_.p;
-    plan_.perm_cols = d_perm_cols_.p;
     std::vector<int> inv(R_->n);
     for (int i = 0; i < R_->n; ++i) inv[R_->perm[i]] = i;
     d_iperm_rows_.upload(inv, stream_);

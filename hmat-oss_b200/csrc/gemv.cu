@@ -652,10 +652,10 @@ __device__ __forceinline__ void mma_unit_dispatch(int ntn, const T* P, const T* 
 // CTAs an SM the tensor-core kernel is compiled for: four, the number its shared memory allows
 // (two stages of warp_stage_bytes(4) for each of its four warps), so every tile count gets the
 // registers of four CTAs.
-__host__ __device__ constexpr int mma_min_blocks(int /*ntile*/, int /*elem_bytes*/) { return 4; }
+constexpr int kMmaMinBlocks = 4;
 
 template <typename T, int R, int RS, int NTILE>
-__global__ void __launch_bounds__(kWarpCTA * 32, mma_min_blocks(NTILE, sizeof(T)))
+__global__ void __launch_bounds__(kWarpCTA * 32, kMmaMinBlocks)
     mma_stream_kernel(const GemvTask* __restrict__ tasks, const int* __restrict__ warp_begin,
                       const GemvUnit* __restrict__ units, const T* __restrict__ arena, T* xz, GemvStatus* err) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1787,7 +1787,7 @@ size_t warp_stream_smem_bytes(int elem_bytes) {
   return (size_t)kWarpCTA * kWarpStages * (warp_stage_bytes(elem_bytes) + sizeof(int2) + sizeof(uint64_t));
 }
 int warp_stream_warps_per_cta() { return kWarpCTA; }
-int mma_stream_blocks_per_sm(int ntile, int elem_bytes) { return mma_min_blocks(ntile, elem_bytes); }
+int mma_stream_blocks_per_sm() { return kMmaMinBlocks; }
 
 size_t umma_smem_bytes() {
   return (size_t)kTcStages * kTcStage + 2 * kTcSteps * (kTcTileA + kTcTileB) + (kTcStages + 1) * 8 + 16 +

@@ -195,8 +195,6 @@ struct GemvPlan {
   // rows of the xz buffer of an 'N' and of a 'T' / 'C' product (x part, zero rows, z slots,
   // partial slots); the two numberings are independent (rows past the zero rows overlap)
   long long xz_rows[2] = {0, 0};
-  const int* perm_rows = nullptr;  // internal -> client
-  const int* perm_cols = nullptr;
   const int* iperm_rows = nullptr;  // client -> internal
   const int* iperm_cols = nullptr;
   const void* arena = nullptr;
