@@ -111,3 +111,31 @@ def test_adjoint(hb, vt, n, leaf, eta, nrhs):
                 assert np.all(np.abs(got - a @ b.T) <= bound + 1e-300), i
     finally:
         h.close()
+
+
+def test_large_matrix(hb):
+    """Beyond the allocation-free products' bound: 3 GB of leaves, many of them Rk leaves over several
+    blocks, in rounds of at most half the leaves' bytes.  <H x, r> = <x, H^T r>: each side's error is below
+    n u ||K|| ||x|| ||r||, and the norm below n (entries of at most 1, nugget aside)."""
+    import torch
+    n = 60000
+    pts = np.random.default_rng(1).random((n, 3))
+    hb.set_parameters(compressionMinLeafSize=0)
+    torch.manual_seed(0)
+    h = hb.HMatrix(pts, hb.kernel(hb.EXP_COV, ell=0.3, nugget=1e-6), leaf_size=12, eta=1.5, epsilon=1e-5)
+    try:
+        T = h.leaf_table()
+        assert np.sum((T[:, 4] == 1) & (T[:, 1] > 12)) > 1000
+        assert h.gemv_launches(1, trans="T") >= 1 + 3 * 2 + 1
+        for nrhs in (1, 5, 16):
+            x, r = (torch.randn((nrhs, n), dtype=torch.float64, device="cuda") for _ in range(2))
+            y, z = torch.zeros_like(x), torch.zeros_like(x)
+            torch.cuda.synchronize()
+            h.gemv_device(x.data_ptr(), y.data_ptr(), nrhs)
+            h.gemv_device(r.data_ptr(), z.data_ptr(), nrhs, trans="T")
+            torch.cuda.synchronize()
+            lhs, rhs = (y * r).sum(1), (x * z).sum(1)
+            assert torch.all((lhs - rhs).abs() <= 2.0 * n * n * 2.0 ** -53 * x.norm(dim=1) * r.norm(dim=1))
+            assert torch.all(lhs.abs() > 1e4 * (lhs - rhs).abs())
+    finally:
+        h.close()
