@@ -762,9 +762,10 @@ __global__ void __launch_bounds__(kWarpCTA * 32, kMmaMinBlocks)
 // Transposed products ('T' / 'C'), every type: out[col] += sum_i op(P[i, col]) X[i] for
 // column-major pieces P.  A warp holds CL x CP columns, lane = slice * CL + cl: column cl + CL a
 // (a < CP) in its registers for all R right-hand sides, rows slice, slice + SL, ... of the piece.
-// Each X row it loads serves CP columns, and each P scalar R multiply-adds, so at 16 right-hand
-// sides the FMAs bound it (FP32: 32 paired FMAs per 4 scalars of P and 4 loads of X a lane); the
-// slices are joined by a shuffle exchange that leaves each lane a share of the sums.
+// Each X row it loads serves CP columns, and each P scalar R multiply-adds (FP32, 16 right-hand
+// sides: 32 paired FMAs per 4 scalars of P and 4 loads of X a lane); the slices are joined by a
+// shuffle exchange that leaves each lane a share of the sums.  At 16 right-hand sides latency bounds
+// it: 122 to 128 registers leave 13 warps an SM, issue slots half and the FMA pipe a quarter busy.
 //
 // Products that ran a CTA per task, with a block barrier per unit and one column a lane, took
 // (device time, before -> now): cylinder of 50,001 points, FP32, 16 right-hand sides 753 -> 192 us
@@ -1367,7 +1368,8 @@ __global__ void __launch_bounds__(256) yfinal_kernel(const int2* __restrict__ ro
 // one warp's loads are a chain).  FP64 and complex z kernels that summed their chunks themselves,
 // the last chunk's warp adding all parts, took 331 us for the 50,000-point Helmholtz cylinder
 // (complex FP32, four right-hand sides; 280 us with this pass) and 35 us for the 8,000-point
-// cylinder (FP64, one; 31 us).
+// cylinder (FP64, one; 31 us), one product alone; products queued one after the other 22.3 -> 20.4 us
+// for the small one and nothing beyond noise for the large one.
 constexpr int kZredWarps = 8;
 constexpr int kZredBatch = 8;  // parts loaded before they are added (loads in flight together)
 template <typename T, int RS>
